@@ -1347,8 +1347,6 @@ template <int L, int R, class LoadOp, class StoreOp>
 __global__ void __launch_bounds__(512, MinBlocks<R>::value) axis_pass_kernel(const AxisParams p) {
   static_assert(R <= L || L < 2, "radix at most the length");
   constexpr int TPT = L / R;
-  pdl_release();
-  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int64_t* offs = reinterpret_cast<int64_t*>(smem_raw);
   const int64_t left = p.nbatch - int64_t(blockIdx.x) * p.cpb;
@@ -1380,8 +1378,12 @@ __global__ void __launch_bounds__(512, MinBlocks<R>::value) axis_pass_kernel(con
   x.oout = to.out_off[x.c];
   x.b0 = umod(x.b, p.d0);
 
+  // everything above reads kernel parameters only, so it runs while the
+  // previous kernel drains
   cpx v[R];
+  pdl_wait();
   LoadOp::template run<L, R>(p, x, t, v);
+  pdl_release();
   run_passes<L, R, 1>(v, x.j, x.c, t, p.tw);
   StoreOp::template run<L, R>(p, x, t, to, v);
 }

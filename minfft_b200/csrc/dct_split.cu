@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(8 * (L / R), 1) dctq_row_fwd(const DctqParams 
   constexpr int TPT = L / R;
   constexpr int NT = 8 * TPT;
   constexpr int N = 2 * L;
-  pdl_release();
   pdl_wait();
+  pdl_release();
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   const int c = tid / TPT, jt = tid % TPT;
@@ -153,8 +153,8 @@ __global__ void __launch_bounds__(8 * (L / R), 1) dctq_row_fwd(const DctqParams 
 template <int QL, int R>
 __global__ void __launch_bounds__(512, 1) dctq_col_fwd(const DctqParams q) {
   constexpr int TPT = QL / R;
-  pdl_release();
   pdl_wait();
+  pdl_release();
   extern __shared__ __align__(16) unsigned char smem[];
   const int W = q.W, cpb = 2 * W;
   const int tid = threadIdx.x;
@@ -232,8 +232,8 @@ __global__ void __launch_bounds__(512, 1) dctq_col_fwd(const DctqParams q) {
 template <int QL, int R>
 __global__ void __launch_bounds__(512, 1) dctq_col_inv(const DctqParams q) {
   constexpr int TPT = QL / R;
-  pdl_release();
   pdl_wait();
+  pdl_release();
   extern __shared__ __align__(16) unsigned char smem[];
   const int W = q.W, cpb = 2 * W;
   const int tid = threadIdx.x;
@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(8 * (L / R), 1) dctq_row_inv(const DctqParams 
   constexpr int TPT = L / R;
   constexpr int NT = 8 * TPT;
   constexpr int N = 2 * L;
-  pdl_release();
   pdl_wait();
+  pdl_release();
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   const int64_t j = blockIdx.x % q.Q, h = blockIdx.x / q.Q;

@@ -19,8 +19,8 @@ struct HasItem32<Op, std::void_t<decltype(&Op::item32)>> : std::true_type {};
 // take it when Op::fast(p) holds for the whole launch.
 template <class Op>
 __global__ void k_line(const LineParams p) {
-  pdl_release();
   pdl_wait();
+  pdl_release();
   if constexpr (HasItem32<Op>::value) {
     if (Op::fast(p)) {
       const uint32_t total = Op::count32(p), stride = gridDim.x * blockDim.x;

@@ -478,6 +478,41 @@ struct Planner {
     return cpb;
   }
 
+  // Radix and transforms per CTA of a launch without a tuned entry or an
+  // override (ap.cpb comes in as choose_cpb's).
+  //
+  // Radix 8 doubles the threads and halves the registers of each: it wins
+  // where the passes are as many either way (32 and 64 points: a batch of
+  // 32768 DCT-4 of 64 points in f32 takes 6.3 us against 10.8), and for the
+  // kinds with a load or store stage of their own up to about 2048 points
+  // per SM, where one wave of CTAs covers the batch and its latency is the
+  // time (2048 DCT-2 + DCT-3 of 256 points in f64: 9.4 us a pair against
+  // 10.8; from 2^20 points on radix 16 is ahead, 20.7 against 23.3).
+  //
+  // Row tiles are CTAs of about 64 threads, on which barriers and the wait
+  // for the slowest load are short: 2048 DFTs of 1024 points in f64 take
+  // 13.7 us with one transform per CTA, 17.0 with four; 8192 DCT-4 of 64
+  // points in f32 2.9 us with eight, 6.6 with 128.  Column tiles stay wide
+  // enough for their runs of adjacent columns: 32 bytes while few points
+  // share the chip, 64 bytes in double (DFT columns of 256 points x 8192 in
+  // f64: 64.3 us for a round trip with 128-thread CTAs, 69.6 with 256),
+  // choose_cpb's 128 bytes in single.
+  void choose_shape(int combo, int L, int64_t nbatch, AxisParams& ap, int* R) {
+    if (four_rows(combo) || mirror_pairs(combo) || ap.st_ns > 1 || (ap.flags & mb::F_STAGE_ROWS)) return;
+    const bool col = ap.colmode != 0, few = nbatch * L <= int64_t(sms) * 2048;
+    const bool r8 = L == 32 || L == 64 || (few && combo != mb::K_CPLX && L > 16);
+    if (r8 && mb::axis_kernel(combo, ilog2(L), 8)) *R = 8;
+    const int tpt = L / std::min(*R, L);
+    const int elem = (combo == mb::K_CPLX) ? int(sizeof(cpx)) : int(sizeof(real));
+    if (!col)
+      ap.cpb = std::max(1, 64 / tpt);
+    else if (few)
+      ap.cpb = std::max(32 / elem, 128 / tpt);
+    else if (sizeof(real) == 8)
+      ap.cpb = std::max(64 / elem, 128 / tpt);
+    while (ap.cpb > 1 && !plain_fits(combo, L, ap.cpb, ap.flags, col ? 1 : 0, *R)) ap.cpb /= 2;
+  }
+
   // kinds whose load or store stage uses the shared-memory tile (the fused
   // type-4 passes hand each real pair's second value to the mirror element)
   static bool staged(int combo) {
@@ -823,6 +858,8 @@ struct Planner {
         while (c > 1 && !plain_fits(combo, L, c, ap.flags, ap.colmode, rr)) c /= 2;
         ap.cpb = c;
         R = rr;
+      } else {
+        choose_shape(combo, L, nbatch, ap, &R);
       }
     }
     if (four_rows(combo)) {

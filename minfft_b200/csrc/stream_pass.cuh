@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(stream_cols() * (L / R), 1)
   const int64_t gpd = (p.d0 + W - 1) / W;  // tiles per block of adjacent columns
   const int64_t ntiles = p.ntiles;
 
-  pdl_release();
   pdl_wait();
+  pdl_release();
   if (tid == 0) {
     for (int s = 0; s < S; ++s) smbar_init(mbar0 + 8 * s, tma ? 1 : NT);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(512, 1) stream_rows_kernel(const AxisParams p)
   const int64_t ntiles = p.ntiles;
   constexpr int esz = LoadOp::kComplexIn ? int(sizeof(cpx)) : int(sizeof(real));
 
-  pdl_release();
   pdl_wait();
+  pdl_release();
   if (tid == 0) {
     for (int s = 0; s < S; ++s) smbar_init(mbar0 + 8 * s, bulk ? 1 : int(blockDim.x));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(16 * TB, TB == 8 ? 4 : 2) tc256_kernel(const A
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
-  pdl_release();
   pdl_wait();
+  pdl_release();
   const uint32_t mbar_a = static_cast<uint32_t>(__cvta_generic_to_shared(mbar));
   const int64_t ntiles = (p.nbatch + TB - 1) / TB;
   if (warp == 0) {
@@ -699,8 +699,8 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
   const int64_t gpd = (p.d0 + W - 1) / W;
   const int64_t ntiles = p.ntiles;
 
-  pdl_release();
   pdl_wait();
+  pdl_release();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      static_cast<uint32_t>(__cvta_generic_to_shared(tslot))),
