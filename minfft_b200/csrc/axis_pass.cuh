@@ -839,6 +839,210 @@ struct LoadT4Chain {
   }
 };
 
+// ---- type-2, type-3 and real-DFT steps fused into the passes of a 1-D chain
+//
+// The first and last passes of the half-length chain of a long 1-D line
+// (Lt = N/2 points, N = kn reals) also do the line's pre- and
+// post-processing, which otherwise are passes over memory of their own.
+// Each step combines a point with its mirror, so the CTA holds mirror pairs
+// of sub-DFTs (MirrorPairs below), one sub-DFT of a pair in slot c < cpb/2,
+// the other in slot c + cpb/2, and hands values over through the tile:
+//  * reflected pairs (points m and Lt-1-m; the type-2 permutation and the
+//    type-3 de-interleave): element n of sub-DFT i with element L-1-n of
+//    sub-DFT M-1-i;
+//  * spectrum pairs (points m and Lt-m; the packing and unpacking of the
+//    real DFT): element n of sub-DFT i with element L-1-n of sub-DFT M-i;
+//    sub-DFTs 0 and M/2 pair with themselves (element n of sub-DFT 0 with
+//    L-n) and share a CTA's slots.
+// Bound by the same memory traffic as a plain pass: what they save is the
+// two passes over memory around the chain (dct2 + dct3 of 2^22 points in
+// f64: ten launches in 145 us before, six in 105 us now, 19 us for a plain
+// pass of 33.6 MB each way and 25 to 28 us for a fused one).
+
+// Slot and element of the mirror of element n in slot c.
+struct Mirror {
+  int slot, flip;  // partner element: (flip - n) & (L - 1)
+};
+// Reflected pairs.
+template <int L>
+__device__ __forceinline__ Mirror mirror_reflected(const AxisParams& p, int c) {
+  const int h = p.cpb / 2;
+  return Mirror{c < h ? c + h : c - h, L - 1};
+}
+// Spectrum pairs; i is the sub-DFT's index in its line.
+template <int L>
+__device__ __forceinline__ Mirror mirror_spectrum(const AxisParams& p, int c, int64_t i) {
+  const int h = p.cpb / 2;
+  if (i == 0) return Mirror{c, L};
+  if (2 * i == p.d0 * p.d1) return Mirror{c, L - 1};
+  return Mirror{c < h ? c + h : c - h, L - 1};
+}
+
+// One value of the packing step (pack_pair) for the spectrum pair (z, zm) of
+// points k and Lt-k: the conjugated inverse-DFT input at k; f = w_N^k.
+__device__ __forceinline__ cpx pack_one(cpx z, cpx zm, cpx f) {
+  const cpx m = cconj(zm);
+  return cconj(cadd(cadd(z, m), cmul(csub(z, m), cmk(f.y, f.x))));
+}
+// One value of the unpacking step (unpack_pair2): 2 X_k from Z_k, Z_(Lt-k).
+__device__ __forceinline__ cpx unpack_one2(cpx z, cpx zm, cpx f) {
+  const cpx m = cconj(zm);
+  return cadd(cadd(z, m), cmul(csub(z, m), cmk(f.y, -f.x)));
+}
+
+// Four consecutive reals, as 16-byte vectors where `vec`.
+struct Real4 {
+  real v[4];
+};
+__device__ __forceinline__ Real4 ld_real4(const real* q, bool vec) {
+  Real4 r;
+  if (vec) {
+#if MINFFT_SINGLE
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(q));
+    r.v[0] = a.x, r.v[1] = a.y, r.v[2] = a.z, r.v[3] = a.w;
+#else
+    const double2 a = __ldcs(reinterpret_cast<const double2*>(q)), b = __ldcs(reinterpret_cast<const double2*>(q) + 1);
+    r.v[0] = a.x, r.v[1] = a.y, r.v[2] = b.x, r.v[3] = b.y;
+#endif
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.v[i] = __ldcs(q + i);
+  }
+  return r;
+}
+__device__ __forceinline__ void st_real4(real* q, const Real4& r, bool vec) {
+  if (vec) {
+#if MINFFT_SINGLE
+    __stcs(reinterpret_cast<float4*>(q), make_float4(r.v[0], r.v[1], r.v[2], r.v[3]));
+#else
+    __stcs(reinterpret_cast<double2*>(q), make_double2(r.v[0], r.v[1]));
+    __stcs(reinterpret_cast<double2*>(q) + 1, make_double2(r.v[2], r.v[3]));
+#endif
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) __stcs(q + i, r.v[i]);
+  }
+}
+
+// Line and sub-DFT index of a first pass's transform, and the line's input.
+struct ChainIn {
+  const real* in;
+  int64_t i;
+};
+__device__ __forceinline__ ChainIn chain_in(const AxisParams& p, const Ctx& x) {
+  const int64_t rest = udiv(x.b, p.d0);
+  const int64_t line = udiv(rest, p.d1);
+  return ChainIn{static_cast<const real*>(p.in) + line * p.k_in_line, rest - line * p.d1};
+}
+
+// Type-2 permutation (reference minfft.c:707-710, 756-759; LoadDCT2) of
+// point g = i + n*in_n: (x[4g], x[4g+2]) for g < Lt/2 (n < L/2), and for its
+// mirror Lt-1-g the pair (x[4g+3], x[4g+1]), negated for DST-2: one vector of
+// four reals gives both points.
+struct LoadDCT2Line {
+  static constexpr bool kComplexIn = false;  // whether the raw input elements are complex
+  static constexpr bool kStaged = false;
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
+    constexpr int TPT = L / R;
+    const ChainIn ci = chain_in(p, x);
+    const real sg = (p.flags & F_DST) ? real(-1) : real(1);
+    const Mirror mi = mirror_reflected<L>(p, x.c);
+    const bool vec = (reinterpret_cast<uintptr_t>(ci.in) & 15) == 0;
+    Real4 q[R / 2];
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r) q[r] = ld_real4(ci.in + 4 * (ci.i + int64_t(x.j + r * TPT) * p.in_n), vec);
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r) {
+      v[r] = cmk(q[r].v[0], q[r].v[2]);
+      t.s[t.idx(mi.slot, L - 1 - (x.j + r * TPT))] = cmk(sg * q[r].v[3], sg * q[r].v[1]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = R / 2; r < R; ++r) v[r] = t.s[t.idx(x.c, x.j + r * TPT)];
+  }
+};
+
+// Packs the tile's spectrum values z (point g of the thread's element r in
+// v[r], k0 the value of t_0) into the conjugated inverse-DFT inputs; fw are
+// the roots w_N^g.
+template <int L, int R>
+__device__ __forceinline__ void pack_tile(const Ctx& x, const Tile& t, const Mirror& mi, bool zero, cpx k0,
+                                          const RootProgression<R>& fw, cpx (&v)[R]) {
+  constexpr int TPT = L / R;
+#pragma unroll
+  for (int r = 0; r < R; ++r) t.s[t.idx(x.c, x.j + r * TPT)] = v[r];
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const cpx zm = t.s[t.idx(mi.slot, (mi.flip - (x.j + r * TPT)) & (L - 1))];
+    v[r] = pack_one(v[r], zm, fw.at(r));
+  }
+  if (zero) v[0] = k0;
+}
+
+// Type-3 pre-rotation (reference minfft.c:807-817, 857-867; LoadDCT3) and
+// packing of point g: z_g = conj((x[g] + i x[N-g]) w_4N^g), DST-3 with
+// x[N-1-g] and x[g-1].  Roots of 4N (st_hi, st_lo): w_4N^g and w_N^g.
+struct LoadDCT3Line {
+  static constexpr bool kComplexIn = false;  // whether the raw input elements are complex
+  static constexpr bool kStaged = false;
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
+    constexpr int TPT = L / R;
+    const ChainIn ci = chain_in(p, x);
+    const bool dst = (p.flags & F_DST) != 0;
+    const int64_t N = p.kn;
+    const Mirror mi = mirror_spectrum<L>(p, x.c, ci.i);
+    const bool zero = ci.i == 0 && x.j == 0;  // element 0 is point 0: x_0 and x_Lt
+    const int64_t g0 = ci.i + int64_t(x.j) * p.in_n, st = int64_t(TPT) * p.in_n;
+    const real* qa = dst ? ci.in + (N - 1 - g0) : ci.in + g0;
+    const real* qb = dst ? ci.in + (g0 - 1) : ci.in + (N - g0);
+    const int64_t sa = dst ? -st : st;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const real* b = qb - r * sa;
+      if (r == 0 && zero) b = ci.in + (dst ? N / 2 - 1 : N / 2);
+      v[r] = cmk(__ldcs(qa + r * sa), __ldcs(b));
+    }
+    const real r2 = real(1.414213562373095048801688724209698079);
+    const cpx k0 = cmk(v[0].x + r2 * v[0].y, -(v[0].x - r2 * v[0].y));
+    {
+      const RootProgression<R> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0), uint32_t(st));
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = cconj(cmul(v[r], ew.at(r)));
+    }
+    const RootProgression<R> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(4 * g0), uint32_t(4 * st));
+    pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
+  }
+};
+
+// Packing of the inverse real DFT (reference minfft.c:628-656; LoadC2R) of
+// point g: the line's N/2 + 1 complex values at line * k_in_line (complex
+// units).  Roots of N (st_hi, st_lo).
+struct LoadC2RLine {
+  static constexpr bool kComplexIn = true;  // whether the raw input elements are complex
+  static constexpr bool kStaged = false;
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
+    constexpr int TPT = L / R;
+    const int64_t rest = udiv(x.b, p.d0), line = udiv(rest, p.d1), i = rest - line * p.d1;
+    const cpx* in = static_cast<const cpx*>(p.in) + line * p.k_in_line;
+    const Mirror mi = mirror_spectrum<L>(p, x.c, i);
+    const bool zero = i == 0 && x.j == 0;
+    const int64_t g0 = i + int64_t(x.j) * p.in_n, st = int64_t(TPT) * p.in_n;
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = __ldcs(in + g0 + r * st);
+    cpx k0 = czero();
+    if (zero) {
+      const cpx zl = in[p.kn / 2];
+      k0 = cmk(v[0].x + zl.x, -(v[0].x - zl.x));
+    }
+    const RootProgression<R> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0), uint32_t(st));
+    pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
+  }
+};
+
 // --------------------------------------------------------------- store ops
 // Each store op receives output element k = j + r*(L/R) of the length-L DFT
 // in v[r].
@@ -1203,6 +1407,109 @@ struct StoreT4Chain {
   }
 };
 
+// Unpacking of the real DFT (reference minfft.c:547-578; StoreR2C) of output
+// point m: X_m, and at m = 0 also X_Lt.  Roots of N (t1, t2, kbits); the
+// line's N/2 + 1 complex outputs at line * k_out_line (complex units; the
+// pass's os2 is 0, so a transform's output offset is its index in the line).
+struct StoreR2CLine {
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets&,
+                                             cpx (&v)[R]) {
+    constexpr int TPT = L / R;
+    cpx* out = static_cast<cpx*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
+    const Mirror mi = mirror_spectrum<L>(p, x.c, x.oout);
+    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
+    const RootProgression<R> fw(p.t1, p.t2, p.kbits, uint32_t(m0), uint32_t(st));
+    __syncthreads();  // the last Stockham exchange has finished with the tile
+    scatter_natural<L, R>(v, x.j, x.c, t);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const cpx zm = t.s[t.idx(mi.slot, (mi.flip - (x.j + r * TPT)) & (L - 1))];
+      cpx X = cscale(unpack_one2(v[r], zm, fw.at(r)), real(0.5));
+      if (r == 0 && m0 == 0) {
+        X = cmk(v[0].x + v[0].y, real(0));
+        out[p.kn / 2] = cmk(v[0].x - v[0].y, real(0));
+      }
+      out[m0 + r * st] = X;
+    }
+  }
+};
+
+// Type-2 output (reference minfft.c:714-725, 763-774; StoreDCT2) of output
+// point m: y_m = Re(2 V_m e_m) and y_(N-m) = -Im(2 V_m e_m), V_m the real
+// DFT's value and e_m = w_4N^m; DST-2 writes the same values to reversed
+// positions; at m = 0 y_0 and y_Lt.  Roots of 4N (t1, t2, kbits) for e_m and
+// w_N^m; the line's N reals at line * k_out_line.
+struct StoreDCT2Line {
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets&,
+                                             cpx (&v)[R]) {
+    constexpr int TPT = L / R;
+    real* out = static_cast<real*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
+    const bool dst = (p.flags & F_DST) != 0;
+    const int64_t N = p.kn;
+    const Mirror mi = mirror_spectrum<L>(p, x.c, x.oout);
+    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
+    __syncthreads();  // the last Stockham exchange has finished with the tile
+    scatter_natural<L, R>(v, x.j, x.c, t);
+    __syncthreads();
+    const real r2 = real(1.414213562373095048801688724209698079);
+    const real y0 = 2 * (v[0].x + v[0].y), yl = r2 * (v[0].x - v[0].y);
+    {
+      const RootProgression<R> fw(p.t1, p.t2, p.kbits, uint32_t(4 * m0), uint32_t(4 * st));
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const cpx zm = t.s[t.idx(mi.slot, (mi.flip - (x.j + r * TPT)) & (L - 1))];
+        v[r] = unpack_one2(v[r], zm, fw.at(r));
+      }
+    }
+    const RootProgression<R> ew(p.t1, p.t2, p.kbits, uint32_t(m0), uint32_t(st));
+    real* qa = dst ? out + (N - 1 - m0) : out + m0;
+    real* qb = dst ? out + (m0 - 1) : out + (N - m0);
+    const int64_t sa = dst ? -st : st;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const cpx q = cmul(v[r], ew.at(r));
+      real a = q.x, b = -q.y;
+      real* pb = qb - r * sa;
+      if (r == 0 && m0 == 0) {
+        a = y0;
+        b = yl;
+        pb = out + (dst ? N / 2 - 1 : N / 2);
+      }
+      qa[r * sa] = a;
+      *pb = b;
+    }
+  }
+};
+
+// Type-3 de-interleave (reference minfft.c:821-824, 871-874; StoreDCT3) of
+// output point m: (t_2m, t_2m+1) go to y[4m], y[4m+2] for m < Lt/2 (k < L/2)
+// and, for its mirror Lt-1-m, to y[4m+3], y[4m+1] (negated for DST-3): the
+// element of the lower half writes the four reals as one vector.
+struct StoreDCT3Line {
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets&,
+                                             cpx (&v)[R]) {
+    constexpr int TPT = L / R;
+    real* out = static_cast<real*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
+    const real sg = (p.flags & F_DST) ? real(-1) : real(1);
+    const Mirror mi = mirror_reflected<L>(p, x.c);
+    const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    __syncthreads();  // the last Stockham exchange has finished with the tile
+#pragma unroll
+    for (int r = R / 2; r < R; ++r) t.s[t.idx(mi.slot, L - 1 - (x.j + r * TPT))] = v[r];
+    __syncthreads();
+    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r) {
+      const cpx w = cconj(v[r]), u = cconj(t.s[t.idx(x.c, x.j + r * TPT)]);
+      st_real4(out + 4 * (m0 + r * st), Real4{{w.x, sg * u.y, w.y, sg * u.x}}, vec);
+    }
+  }
+};
+
 // Element-wise steps of a long real transform fused into the first or last
 // pass of a Stockham chain whose sub-DFTs hold single points of the
 // half-length sequence (one line, no mirror pairing; the mixed batch's long
@@ -1300,33 +1607,43 @@ struct StoreT4Direct {
   }
 };
 
-// The fused type-4 passes take mirror pairs of sub-DFTs into one CTA: with
-// M = d0*d1 sub-DFTs per line, slots c < cpb/2 hold sub-DFTs i of the line
-// and slots c + cpb/2 their mirrors M-1-i (the planner makes cpb even and a
-// divisor of M).
+// The fused passes of a 1-D real chain take mirror pairs of sub-DFTs into one
+// CTA: with M = d0*d1 sub-DFTs per line, slots c < cpb/2 hold sub-DFTs i of
+// the line and slots c + cpb/2 their mirrors, M-1-i for reflected pairs (and
+// the type-4 steps), M-i for spectrum pairs, where sub-DFT M/2 sits in the
+// mirror slot of sub-DFT 0 (the planner makes cpb even and a divisor of M).
+enum MirrorKind : int { kNoMirror = 0, kReflected, kSpectrum };
 template <class Op>
 struct MirrorPairs {
-  static constexpr bool value = false;
+  static constexpr MirrorKind value = kNoMirror;
 };
-template <>
-struct MirrorPairs<LoadT4Chain> {
-  static constexpr bool value = true;
-};
-template <>
-struct MirrorPairs<StoreT4Chain> {
-  static constexpr bool value = true;
-};
+#define MB_MIRROR(Op, kind)                    \
+  template <>                                  \
+  struct MirrorPairs<Op> {                     \
+    static constexpr MirrorKind value = kind;  \
+  }
+MB_MIRROR(LoadT4Chain, kReflected);
+MB_MIRROR(StoreT4Chain, kReflected);
+MB_MIRROR(LoadDCT2Line, kReflected);
+MB_MIRROR(StoreDCT3Line, kReflected);
+MB_MIRROR(LoadDCT3Line, kSpectrum);
+MB_MIRROR(LoadC2RLine, kSpectrum);
+MB_MIRROR(StoreR2CLine, kSpectrum);
+MB_MIRROR(StoreDCT2Line, kSpectrum);
+#undef MB_MIRROR
 
 // Batch index of the CTA's transform in slot c.
-template <bool kMirror>
+template <MirrorKind kMirror>
 __device__ __forceinline__ int64_t tile_batch(const AxisParams& p, int c) {
-  if constexpr (kMirror) {
+  if constexpr (kMirror != kNoMirror) {
     const int64_t M = p.d0 * p.d1;
     const int64_t per_line = udiv(M, p.cpb);  // CTAs per line
     const int64_t line = udiv(int64_t(blockIdx.x), per_line), q = int64_t(blockIdx.x) - line * per_line;
     const int h = p.cpb / 2;
     const int64_t i = q * h + (c < h ? c : c - h);
-    return line * M + (c < h ? i : M - 1 - i);
+    if (c < h) return line * M + i;
+    if constexpr (kMirror == kReflected) return line * M + (M - 1 - i);
+    return line * M + (i == 0 ? M / 2 : M - i);
   } else {
     return int64_t(blockIdx.x) * p.cpb + c;
   }
@@ -1353,7 +1670,8 @@ __global__ void __launch_bounds__(512, MinBlocks<R>::value) axis_pass_kernel(con
   TileOffsets to{offs, offs + p.cpb, int(left < p.cpb ? left : p.cpb)};
   Tile t{reinterpret_cast<cpx*>(smem_raw + 16 * ((2 * p.cpb * sizeof(int64_t) + 15) / 16)), p.lp};
 
-  constexpr bool kMirror = MirrorPairs<LoadOp>::value || MirrorPairs<StoreOp>::value;
+  constexpr MirrorKind kMirror =
+      MirrorPairs<LoadOp>::value != kNoMirror ? MirrorPairs<LoadOp>::value : MirrorPairs<StoreOp>::value;
   // offsets of the CTA's transforms, computed once per transform
   for (int c = threadIdx.x; c < p.cpb; c += blockDim.x) {
     const int64_t b = tile_batch<kMirror>(p, c);

@@ -17,6 +17,12 @@ const void* axis_kernel_r2cq(int log2L, int radix16);
 const void* axis_kernel_c2rq(int log2L, int radix16);
 const void* axis_kernel_t4in(int log2L, int radix16);
 const void* axis_kernel_t4out(int log2L, int radix16);
+const void* axis_kernel_dct2in(int log2L, int radix16);
+const void* axis_kernel_dct2out(int log2L, int radix16);
+const void* axis_kernel_dct3in(int log2L, int radix16);
+const void* axis_kernel_dct3out(int log2L, int radix16);
+const void* axis_kernel_c2rin(int log2L, int radix16);
+const void* axis_kernel_r2cout(int log2L, int radix16);
 
 const void* pipe_kernel_cplx(int log2L, int radix16);
 const void* pipe_kernel_r2c(int log2L, int radix16);
@@ -62,6 +68,12 @@ const void* axis_kernel(int combo, int log2L, int R) {
     case K_C2RQ: return axis_kernel_c2rq(log2L, R >= 16);
     case K_T4IN: return axis_kernel_t4in(log2L, R >= 16);
     case K_T4OUT: return axis_kernel_t4out(log2L, R >= 16);
+    case K_DCT2IN: return axis_kernel_dct2in(log2L, R >= 16);
+    case K_DCT2OUT: return axis_kernel_dct2out(log2L, R >= 16);
+    case K_DCT3IN: return axis_kernel_dct3in(log2L, R >= 16);
+    case K_DCT3OUT: return axis_kernel_dct3out(log2L, R >= 16);
+    case K_C2RIN: return axis_kernel_c2rin(log2L, R >= 16);
+    case K_R2COUT: return axis_kernel_r2cout(log2L, R >= 16);
     default: return nullptr;
   }
 }

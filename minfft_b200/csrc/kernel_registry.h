@@ -15,6 +15,12 @@ enum Combo : int {
   K_C2RQ,       // last radix-4 stage of an inverse column DFT across 4 rows, then their inverse real DFT
   K_T4IN,       // first pass of a 1-D type-4 chain over HBM: the pre-rotation fused into its load
   K_T4OUT,      // last pass of a 1-D type-4 chain over HBM: the post-rotation fused into its store
+  K_DCT2IN,     // first pass of a 1-D type-2 chain: the permutation fused into its load
+  K_DCT2OUT,    // last pass of a 1-D type-2 chain: unpacking and post-rotation fused into its store
+  K_DCT3IN,     // first pass of a 1-D type-3 chain: pre-rotation and packing fused into its load
+  K_DCT3OUT,    // last pass of a 1-D type-3 chain: the de-interleave fused into its store
+  K_C2RIN,      // first pass of a 1-D inverse real chain: the packing fused into its load
+  K_R2COUT,     // last pass of a 1-D real chain: the unpacking fused into its store
   K_COUNT
 };
 

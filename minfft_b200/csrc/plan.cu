@@ -517,11 +517,44 @@ struct Planner {
   // type-4 passes hand each real pair's second value to the mirror element)
   static bool staged(int combo) {
     return combo == mb::K_R2C || combo == mb::K_C2R || combo == mb::K_DCT2 || combo == mb::K_DCT3 ||
-           combo == mb::K_R2CQ || combo == mb::K_C2RQ || combo == mb::K_T4IN || combo == mb::K_T4OUT;
+           combo == mb::K_R2CQ || combo == mb::K_C2RQ || mirror_pairs(combo);
   }
 
-  // the fused type-4 passes hold mirror pairs of sub-DFTs in one CTA
-  static bool mirror_pairs(int combo) { return combo == mb::K_T4IN || combo == mb::K_T4OUT; }
+  // the fused passes of the 1-D real chains hold mirror pairs of sub-DFTs in one CTA
+  static bool mirror_pairs(int combo) { return combo >= mb::K_T4IN && combo < mb::K_COUNT; }
+
+  // kinds whose raw input / output elements are complex
+  static bool complex_in(int combo) {
+    return combo == mb::K_CPLX || combo == mb::K_C2R || combo == mb::K_C2RQ || combo == mb::K_T4OUT ||
+           combo == mb::K_DCT2OUT || combo == mb::K_DCT3OUT || combo == mb::K_C2RIN || combo == mb::K_R2COUT;
+  }
+  static bool complex_out(int combo) {
+    return combo == mb::K_CPLX || combo == mb::K_R2C || combo == mb::K_R2CQ || combo == mb::K_T4IN ||
+           combo == mb::K_DCT2IN || combo == mb::K_DCT3IN || combo == mb::K_C2RIN || combo == mb::K_R2COUT;
+  }
+
+  static const char* combo_name(int combo) {
+    static const char* names[mb::K_COUNT] = {"cplx", "r2c", "c2r", "dct2", "dct3", "t4", "r2c+col4", "col4+c2r",
+                                             "t4pre+cplx", "cplx+t4post", "dct2pre+cplx", "cplx+dct2post",
+                                             "dct3pre+cplx", "cplx+dct3post", "c2rpack+cplx", "cplx+r2cunpack"};
+    return names[combo];
+  }
+
+  // algorithmic bytes of one transform: each input element read once, each
+  // output element written once
+  static double axis_bytes(int combo, int L) {
+    const double R = sizeof(real), C = sizeof(cpx);
+    switch (combo) {
+      case mb::K_CPLX:
+      case mb::K_C2RIN:
+      case mb::K_R2COUT: return 2.0 * L * C;
+      case mb::K_R2C:
+      case mb::K_R2CQ: return 2.0 * L * R + (L + 1) * C;
+      case mb::K_C2R:
+      case mb::K_C2RQ: return (L + 1) * C + 2.0 * L * R;
+      default: return 4.0 * L * R;
+    }
+  }
 
   // the split-column kinds work on exactly four rows per CTA
   static bool four_rows(int combo) { return combo == mb::K_R2CQ || combo == mb::K_C2RQ; }
@@ -577,6 +610,15 @@ struct Planner {
   static bool t4_fuse_enabled() {
     static const bool on = [] {
       const char* e = getenv("MINFFT_B200_T4FUSE");
+      return !(e && e[0] == '0');
+    }();
+    return on;
+  }
+
+  // The same for the real DFT and types 2 and 3 (MINFFT_B200_LINEFUSE=0).
+  static bool line_fuse_enabled() {
+    static const bool on = [] {
+      const char* e = getenv("MINFFT_B200_LINEFUSE");
       return !(e && e[0] == '0');
     }();
     return on;
@@ -909,32 +951,16 @@ struct Planner {
     ln.out_buf = out_buf;
     ln.vec_in = vec_in;
     ln.vec_out = vec_out;
-    ln.in_c = (combo == mb::K_CPLX || combo == mb::K_C2R || combo == mb::K_C2RQ || combo == mb::K_T4OUT);
-    ln.out_c = (combo == mb::K_CPLX || combo == mb::K_R2C || combo == mb::K_R2CQ || combo == mb::K_T4IN);
+    ln.in_c = complex_in(combo);
+    ln.out_c = complex_out(combo);
     ln.combo = combo;
     ln.L = L;
     ln.ap = ap;
-    {
-      static const char* names[] = {"cplx", "r2c", "c2r", "dct2", "dct3", "t4", "r2c+col4", "col4+c2r",
-                                    "t4pre+cplx", "cplx+t4post"};
-      const double R = sizeof(real), C = sizeof(cpx);
-      double per = 0;
-      switch (combo) {
-        case mb::K_CPLX: per = 2.0 * L * C; break;
-        case mb::K_T4IN:
-        case mb::K_T4OUT: per = 2.0 * L * R + L * C; break;
-        case mb::K_R2C:
-        case mb::K_R2CQ: per = 2.0 * L * R + (L + 1) * C; break;
-        case mb::K_C2R:
-        case mb::K_C2RQ: per = (L + 1) * C + 2.0 * L * R; break;
-        default: per = 4.0 * L * R; break;
-      }
-      ln.bytes = per * double(nbatch);
-      char buf[160];
-      snprintf(buf, sizeof(buf), "axis_pass<%s,L=%d,%s%s> batch=%lld", names[combo], L, ap.colmode ? "col" : "row",
-               ap.st_ns > 1 ? ",hbm" : "", (long long)nbatch);
-      ln.label = buf;
-    }
+    ln.bytes = axis_bytes(combo, L) * double(nbatch);
+    char buf[160];
+    snprintf(buf, sizeof(buf), "axis_pass<%s,L=%d,%s%s> batch=%lld", combo_name(combo), L, ap.colmode ? "col" : "row",
+             ap.st_ns > 1 ? ",hbm" : "", (long long)nbatch);
+    ln.label = buf;
     prog->launches.push_back(ln);
   }
 
@@ -1097,29 +1123,15 @@ struct Planner {
     ln.out_buf = out_buf;
     ln.vec_in = vec_in;
     ln.vec_out = vec_out;
-    ln.in_c = (combo == mb::K_CPLX || combo == mb::K_C2R || combo == mb::K_C2RQ);
-    ln.out_c = (combo == mb::K_CPLX || combo == mb::K_R2C || combo == mb::K_R2CQ);
+    ln.in_c = complex_in(combo);
+    ln.out_c = complex_out(combo);
     ln.combo = combo;
     ln.L = L;
     ln.ap = ap;
-    {
-      static const char* names[] = {"cplx", "r2c", "c2r", "dct2", "dct3", "t4", "r2c+col4", "col4+c2r",
-                                    "t4pre+cplx", "cplx+t4post"};
-      const double Rb = sizeof(real), C = sizeof(cpx);
-      double per = 0;
-      switch (combo) {
-        case mb::K_CPLX: per = 2.0 * L * C; break;
-        case mb::K_R2C:
-        case mb::K_R2CQ: per = 2.0 * L * Rb + (L + 1) * C; break;
-        case mb::K_C2R:
-        case mb::K_C2RQ: per = (L + 1) * C + 2.0 * L * Rb; break;
-        default: per = 4.0 * L * Rb; break;
-      }
-      ln.bytes = per * double(nbatch);
-      char buf[160];
-      snprintf(buf, sizeof(buf), "stream_rows<%s,L=%d> batch=%lld", names[combo], L, (long long)nbatch);
-      ln.label = buf;
-    }
+    ln.bytes = axis_bytes(combo, L) * double(nbatch);
+    char buf[160];
+    snprintf(buf, sizeof(buf), "stream_rows<%s,L=%d> batch=%lld", combo_name(combo), L, (long long)nbatch);
+    ln.label = buf;
     prog->launches.push_back(ln);
   }
 
@@ -1171,28 +1183,16 @@ struct Planner {
     ln.in_buf = in_buf;
     ln.out_buf = out_buf;
     ln.vec_out = (combo == mb::K_C2R);
-    ln.in_c = (combo == mb::K_CPLX || combo == mb::K_C2R || combo == mb::K_C2RQ || combo == mb::K_T4OUT);
-    ln.out_c = (combo == mb::K_CPLX || combo == mb::K_R2C || combo == mb::K_R2CQ || combo == mb::K_T4IN);
+    ln.in_c = complex_in(combo);
+    ln.out_c = complex_out(combo);
     ln.combo = combo;
     ln.L = L;
     ln.ap = ap;
-    {
-      static const char* names[] = {"cplx", "r2c", "c2r", "dct2", "dct3", "t4", "r2c+col4", "col4+c2r",
-                                    "t4pre+cplx", "cplx+t4post"};
-      const double Rb = sizeof(real), C = sizeof(cpx);
-      double per = 0;
-      switch (combo) {
-        case mb::K_CPLX: per = 2.0 * L * C; break;
-        case mb::K_R2C: per = 2.0 * L * Rb + (L + 1) * C; break;
-        case mb::K_C2R: per = (L + 1) * C + 2.0 * L * Rb; break;
-        default: per = 4.0 * L * Rb; break;
-      }
-      ln.bytes = per * double(nbatch);
-      char buf[160];
-      snprintf(buf, sizeof(buf), "axis_pipe<%s,L=%d,%s%s> batch=%lld", names[combo], L, ap.colmode ? "col" : "row",
-               ap.st_ns > 1 ? ",hbm" : "", (long long)nbatch);
-      ln.label = buf;
-    }
+    ln.bytes = axis_bytes(combo, L) * double(nbatch);
+    char buf[160];
+    snprintf(buf, sizeof(buf), "axis_pipe<%s,L=%d,%s%s> batch=%lld", combo_name(combo), L, ap.colmode ? "col" : "row",
+             ap.st_ns > 1 ? ",hbm" : "", (long long)nbatch);
+    ln.label = buf;
     prog->launches.push_back(ln);
   }
 
@@ -1570,23 +1570,52 @@ struct Planner {
       lp.flags = s.flags;
       return lp;
     };
-    // A 1-D type-4 chain of two or more passes fuses its pre-rotation into
-    // the first pass's load and its post-rotation into the last pass's store
-    // (LoadT4Chain, StoreT4Chain): two passes over HBM instead of four.  In a
-    // tensor-core mode only an end pass on the CUDA cores of 128 to 1024
-    // points (the lengths the FP32 and FP64 type-4 chains take) fuses its
-    // rotation: the 256-point tensor-core passes take plain complex input and
-    // output.  The other rotation stays a separate element-wise step.
-    // (the fused passes form their roots from 32-bit exponents into the tables of 8N)
+    // The chain of a 1-D line of a real kind fuses the line's pre-processing
+    // into its first pass's load and the post-processing into its last
+    // pass's store, where that pass has a fused form: the rotations of type 4
+    // (LoadT4Chain, StoreT4Chain), the permutation, rotations and
+    // de-interleave of types 2 and 3 and the real DFT's unpacking and packing
+    // (the *Line ops).  Two passes over memory less: dct2 + dct3 of 2^22
+    // points in f64 144.9 -> 105.4 us.  In a tensor-core mode only an end
+    // pass on the CUDA cores fuses its step (128 to 1024 points for type 4, 16
+    // to 1024 for the others): the 256-point tensor-core passes take plain
+    // complex input and output.  The other step stays a separate
+    // element-wise kernel.
+    // (the fused passes form their roots from 32-bit exponents into tables of
+    // up to 8N roots)
     const bool t4_chain =
         s.combo == mb::K_T4 && inner == 1 && P >= 2 && s.N <= (int64_t(1) << 28) && t4_fuse_enabled();
-    auto cuda_core_pass = [&](int p) {
-      return a->precision == MINFFT_B200_PREC_FP32 ||
-             ((int64_t(1) << pb[p]) != mb::kTcLength && pb[p] >= 7 && pb[p] <= kPassCapLog2Cc);
+    const bool line_chain = (s.combo == mb::K_R2C || s.combo == mb::K_C2R || s.combo == mb::K_DCT2 ||
+                             s.combo == mb::K_DCT3) &&
+                            inner == 1 && P >= 2 && s.N <= (int64_t(1) << 28) && line_fuse_enabled();
+    const bool fp32 = a->precision == MINFFT_B200_PREC_FP32;
+    auto cuda_core_pass = [&](int p, int min_bits) {
+      return fp32 || ((int64_t(1) << pb[p]) != mb::kTcLength && pb[p] >= min_bits && pb[p] <= kPassCapLog2Cc);
     };
-    const bool t4_fused_in = t4_chain && cuda_core_pass(0);
-    const bool t4_fused_out = t4_chain && cuda_core_pass(P - 1);
-    if (!t4_fused_in &&
+    int combo_in = mb::K_CPLX, combo_out = mb::K_CPLX;  // kinds of the first and the last pass
+    if (t4_chain && cuda_core_pass(0, 7)) combo_in = mb::K_T4IN;
+    if (t4_chain && cuda_core_pass(P - 1, 7)) combo_out = mb::K_T4OUT;
+    if (line_chain) {
+      // A tensor-core chain of types 2 and 3 that ends on a pass without a
+      // fused form (2^16, 2^19, 2^20, 2^24, 2^27 points) moves its CUDA-core
+      // points to both ends instead: 16..64-point passes with the fused steps
+      // around the 256-point ones, and no sweeps of their own.
+      if (!fp32 && (s.combo == mb::K_DCT2 || s.combo == mb::K_DCT3) && bits >= 16 && !cuda_core_pass(P - 1, 4)) {
+        const int tb = ilog2(mb::kTcLength), k = (bits - tb) / tb, rest = bits - k * tb;
+        pb.assign(k + 2, tb);
+        pb.front() = (rest + 1) / 2;
+        pb.back() = rest / 2;
+        P = k + 2;
+      }
+      if (s.combo == mb::K_DCT2) combo_in = mb::K_DCT2IN, combo_out = mb::K_DCT2OUT;
+      if (s.combo == mb::K_DCT3) combo_in = mb::K_DCT3IN, combo_out = mb::K_DCT3OUT;
+      if (s.combo == mb::K_C2R) combo_in = mb::K_C2RIN;
+      if (s.combo == mb::K_R2C) combo_out = mb::K_R2COUT;
+      if (!cuda_core_pass(0, 4) || !mb::axis_kernel(combo_in, pb[0])) combo_in = mb::K_CPLX;
+      if (!cuda_core_pass(P - 1, 4) || !mb::axis_kernel(combo_out, pb[P - 1])) combo_out = mb::K_CPLX;
+    }
+    const bool fused_in = combo_in != mb::K_CPLX, fused_out = combo_out != mb::K_CPLX;
+    if (!fused_in &&
         (s.combo == mb::K_DCT2 || s.combo == mb::K_T4 || s.combo == mb::K_C2R || s.combo == mb::K_DCT3)) {
       cs = BUF_T2;
       need(cs, work_bytes);
@@ -1611,7 +1640,7 @@ struct Planner {
       }
       add_line_kernel(which, lp, items, s.in_buf, cs);
     }
-    const bool post = !t4_fused_out &&
+    const bool post = !fused_out &&
                       (s.combo == mb::K_R2C || s.combo == mb::K_DCT2 || s.combo == mb::K_DCT3 || s.combo == mb::K_T4);
 
     // --- the HBM passes
@@ -1632,7 +1661,7 @@ struct Planner {
       } else {
         dst = s.out_buf;
       }
-      const bool fuse_in = t4_fused_in && p == 0, fuse_out = t4_fused_out && last;
+      const bool fuse_in = fused_in && p == 0, fuse_out = fused_out && last;
       const int64_t Nsp = Ns * inner;
       AxisParams ap = base_params();
       ap.d0 = Nsp;
@@ -1661,22 +1690,34 @@ struct Planner {
       if (last && conj_chain && s.combo != mb::K_DCT3) ap.flags |= mb::F_CONJ_OUT;
       ap.tw = tab(TB_TW, Rp);
       int combo = mb::K_CPLX;
+      // root table pairs of the fused steps: 2N and 8N (type 4), 4N (types 2
+      // and 3: w_4N^g, and w_N^g as its fourth power's entry), N (real DFT)
+      auto roots_of = [&](int fused, bool in) -> int64_t {
+        if (fused == mb::K_T4IN || fused == mb::K_T4OUT) return in ? 2 * s.N : 8 * s.N;
+        return (fused == mb::K_C2RIN || fused == mb::K_R2COUT) ? s.N : 4 * s.N;
+      };
       if (fuse_in) {
-        combo = mb::K_T4IN;
+        combo = combo_in;
         ap.flags |= (s.flags & mb::F_DST);
-        ap.st_hi = tab(TB_STHI, 2 * s.N);  // w_2N^g, coarse x fine
-        ap.st_lo = tab(TB_STLO, 2 * s.N);
-        ap.st_lobits = (int)st_lobits_for(2 * s.N);
+        if (combo != mb::K_DCT2IN) {
+          const int64_t M = roots_of(combo, true);
+          ap.st_hi = tab(TB_STHI, M);  // coarse x fine
+          ap.st_lo = tab(TB_STLO, M);
+          ap.st_lobits = (int)st_lobits_for(M);
+        }
         ap.is2 = 0;
         ap.kn = s.N;
         ap.k_in_line = s.in_row;
       }
       if (fuse_out) {
-        combo = mb::K_T4OUT;
+        combo = combo_out;
         ap.flags |= (s.flags & mb::F_DST);
-        ap.t1 = tab(TB_STHI, 8 * s.N);  // w_8N^(2q+1), coarse x fine
-        ap.t2 = tab(TB_STLO, 8 * s.N);
-        ap.kbits = (int)st_lobits_for(8 * s.N);
+        if (combo != mb::K_DCT3OUT) {
+          const int64_t M = roots_of(combo, false);
+          ap.t1 = tab(TB_STHI, M);  // coarse x fine
+          ap.t2 = tab(TB_STLO, M);
+          ap.kbits = (int)st_lobits_for(M);
+        }
         ap.os2 = 0;
         ap.kn = s.N;
         ap.k_out_line = s.out_row;
@@ -2549,13 +2590,29 @@ Extent launch_extent(const Launch& ln) {
         e.in_max = oi + L * ap.in_n;
         e.out_max = oo + 2 * L - 1;
         break;
-      case mb::K_T4IN: {  // the real lines of the input (the pass's is2 is 0)
+      case mb::K_T4IN:
+      case mb::K_DCT2IN:
+      case mb::K_DCT3IN: {  // the real lines of the input (the pass's is2 is 0)
         const int64_t lines = ap.nbatch / (ap.d0 * ap.d1);
         e.in_max = (lines - 1) * ap.k_in_line + ap.kn - 1;
         e.out_max = oo + (L - 1) * ap.out_k;
         break;
       }
-      case mb::K_T4OUT: {  // the real lines of the output (the pass's os2 is 0)
+      case mb::K_C2RIN: {  // the spectra of the lines
+        const int64_t lines = ap.nbatch / (ap.d0 * ap.d1);
+        e.in_max = (lines - 1) * ap.k_in_line + ap.kn / 2;
+        e.out_max = oo + (L - 1) * ap.out_k;
+        break;
+      }
+      case mb::K_R2COUT: {
+        const int64_t lines = ap.nbatch / (ap.d0 * ap.d1);
+        e.in_max = oi + (L - 1) * ap.in_n;
+        e.out_max = (lines - 1) * ap.k_out_line + ap.kn / 2;
+        break;
+      }
+      case mb::K_T4OUT:
+      case mb::K_DCT2OUT:
+      case mb::K_DCT3OUT: {  // the real lines of the output (the pass's os2 is 0)
         const int64_t lines = ap.nbatch / (ap.d0 * ap.d1);
         e.in_max = oi + (L - 1) * ap.in_n;
         e.out_max = (lines - 1) * ap.k_out_line + ap.kn - 1;
