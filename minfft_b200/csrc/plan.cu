@@ -496,10 +496,22 @@ struct Planner {
   // enough for their runs of adjacent columns: 32 bytes while few points
   // share the chip, 64 bytes in double (DFT columns of 256 points x 8192 in
   // f64: 64.3 us for a round trip with 128-thread CTAs, 69.6 with 256),
-  // choose_cpb's 128 bytes in single.
+  // choose_cpb's 128 bytes in single.  The passes over memory of a long axis
+  // take 64-thread CTAs of at least four columns while few points share the
+  // chip (2^16 complex points in f64: 18.2 us for a round trip, 11.5 so), and
+  // else 128-byte runs on 128 to 256 threads (the 128-point last pass of the
+  // DCT-4 of 2^24 points in f32 takes 4 us less with 16 columns than with 32,
+  // the 128-point passes of 2^21 points in f64 1 to 2.6 us less).
   void choose_shape(int combo, int L, int64_t nbatch, AxisParams& ap, int* R) {
-    if (four_rows(combo) || mirror_pairs(combo) || ap.st_ns > 1 || (ap.flags & mb::F_STAGE_ROWS)) return;
+    if (four_rows(combo)) return;
     const bool col = ap.colmode != 0, few = nbatch * L <= int64_t(sms) * 2048;
+    if (mirror_pairs(combo) || ap.st_ns > 1 || (ap.flags & mb::F_STAGE_ROWS)) {  // a pass over memory
+      const int tpt = L / std::min(*R, L), line = int(128 / sizeof(cpx));
+      ap.cpb = few ? std::max(4, 64 / tpt) : std::max(line, 128 / tpt);
+      while (ap.cpb * tpt > 256 && ap.cpb > (few ? 4 : line / 2)) ap.cpb /= 2;
+      while (ap.cpb > 1 && !plain_fits(combo, L, ap.cpb, ap.flags, col ? 1 : 0, *R)) ap.cpb /= 2;
+      return;
+    }
     const bool r8 = L == 32 || L == 64 || (few && combo != mb::K_CPLX && L > 16);
     if (r8 && mb::axis_kernel(combo, ilog2(L), 8)) *R = 8;
     const int tpt = L / std::min(*R, L);
