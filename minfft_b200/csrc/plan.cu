@@ -884,6 +884,27 @@ struct Planner {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         ov = g_default_override;
       }
+      // Columns streamed by two groups of threads per CTA.  512 points of
+      // arrays beyond the L2 (128 MiB; 256 MiB in single): the axes of
+      // 512 x 512 x 64 in f64, round trip, 676 us with one tile per CTA, 551
+      // so; 64 DFTs of 2^18 points 518 against 458; arrays that the L2 holds
+      // gain nothing (2^21 points in f64: 63.1 against 69.0).  256 points
+      // only where every row of the tile, read and written, has a 2 MiB page
+      // of its own and the longer runs of a streamed tile pay (last pass of
+      // 2^26 points in f64: 433 us, 362 so; with rows 8 KiB apart on one side
+      // 236 us a round trip of 64 DFTs of 2^17 points became 256).  A pass
+      // that stages its output rows keeps a third 512-point tile in flight,
+      // as its stage is busy until the last store.
+      const int64_t C = int64_t(sizeof(cpx)), page = int64_t(2) << 20;
+      const bool streamed =
+          L == 512 ? nbatch * L * C >= (int64_t(1) << (sizeof(real) == 4 ? 28 : 27))
+                   : L == 256 && ap.in_n * C >= page && ap.out_k * C >= page;
+      const int col_stages = (L == 512 && (ap.flags & mb::F_STAGE_ROWS)) ? 3 : 2;
+      if (ov.pipe < 0 && ov.cpb == 0 && ov.radix == 16 && streamed &&
+          stream_fits(combo, L, nbatch, ap, 16, col_stages)) {
+        add_stream_kernel(L, nbatch, ap, in_buf, out_buf, col_stages, key, 16);
+        return;
+      }
       const bool want_pipe = ov.pipe == 1 || (ov.pipe < 0 && pipe_default());
       const int st_stages = ov.cpb > 0 ? ov.cpb : 3;
       if (ov.pipe == 2 && stream_fits(combo, L, nbatch, ap, ov.radix, st_stages)) {
@@ -1018,14 +1039,14 @@ struct Planner {
   bool stream_fits(int combo, int L, int64_t nbatch, const AxisParams& ap0, int R, int stages) const {
     AxisParams ap = ap0;
     if (!stream_normalise(combo, L, nbatch, ap)) return false;
-    if (stages < 2 || stages > 8 || !mb::stream_kernel(ilog2(L), R)) return false;
+    if (stages < 2 || stages > mb::kStreamMaxStages || !mb::stream_kernel(ilog2(L), R)) return false;
     return mb::stream_smem(L, stages) <= (size_t)dev_max_smem;
   }
 
   void add_stream_kernel(int L, int64_t nbatch, AxisParams ap, int in_buf, int out_buf, int stages,
                          const TuneKey& key, int R) {
     stream_normalise(mb::K_CPLX, L, nbatch, ap);
-    const int W = mb::stream_cols();
+    const int W = mb::stream_cols(L);
     Launch ln;
     ln.key = key;
     ln.radix = R;
@@ -1048,7 +1069,7 @@ struct Planner {
       ok = false;
       return;
     }
-    ln.block = unsigned(W * (L / R));
+    ln.block = unsigned(mb::stream_group(L, R) * std::min(mb::stream_max_groups(L, R), stages));
     int occ = 1;
     if (!a->host_only) {
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ln.fn, (int)ln.block, ln.smem) != cudaSuccess ||
@@ -2040,7 +2061,7 @@ bool stream_map(CUtensorMap* m, const Launch& ln, const AxisParams& ap) {
   const uint64_t st1 = ap.d1 > 1 ? s2 : (span1 + 15) / 16 * 16;
   const uint64_t st2 = d2 > 1 ? s3 : (st1 * uint64_t(ap.d1) + 15) / 16 * 16;
   const cuuint64_t strides[3] = {cuuint64_t(s1), cuuint64_t(st1), cuuint64_t(st2)};
-  const cuuint32_t box[4] = {cuuint32_t(2 * mb::stream_cols()), cuuint32_t(ln.L < 256 ? ln.L : 256), 1, 1};
+  const cuuint32_t box[4] = {cuuint32_t(2 * mb::stream_cols(ln.L)), cuuint32_t(ln.L < 256 ? ln.L : 256), 1, 1};
   const cuuint32_t es[4] = {1, 1, 1, 1};
   for (int i = 0; i < 3; ++i)
     if (strides[i] >= (uint64_t(1) << 40)) return false;
@@ -2711,7 +2732,7 @@ MB_EXPORT int minfft_b200_plan_selfcheck_precision(int op, int d, const int* Ns,
       fail("launch %zu (%s): output reaches byte %lld of buffer %d (%zu bytes)", i, ln.label.c_str(),
            (long long)((e.out_max + 1) * oe), ln.out_buf, cap[ln.out_buf]);
     if (ln.block < 1 || ln.block > 1024 || ln.grid < 1) fail("launch %zu: bad shape %u x %u", i, ln.grid, ln.block);
-    if (!ln.is_line && ln.block > 512) fail("launch %zu: block %u above launch bounds", i, ln.block);
+    if (!ln.is_line && !ln.stream && ln.block > 512) fail("launch %zu: block %u above launch bounds", i, ln.block);
     if (!ln.is_line && !ln.stream && !ln.tcs && ln.dctq < 0 &&
         ln.block != unsigned(ln.ap.cpb * (ln.L / std::min(ln.radix, std::max(ln.L, 1)))))
       fail("launch %zu: block %u is not cpb x L/R", i, ln.block);
@@ -2735,12 +2756,14 @@ MB_EXPORT int minfft_b200_plan_selfcheck_precision(int op, int d, const int* Ns,
     }
     if (ln.stream) {
       const AxisParams& ap = ln.ap;
-      const int W = mb::stream_cols();
+      const int W = mb::stream_cols(ln.L);
       if (ap.is0 != 1 || !ap.colmode || ln.combo != mb::K_CPLX)
         fail("launch %zu (%s): streamed pass needs adjacent unit-stride columns", i, ln.label.c_str());
       if (ap.d0 * ap.d1 * ln.st_d2 != ap.nbatch || ap.gpb * W < ap.d0 || ap.ntiles != ap.gpb * ap.d1 * ln.st_d2)
         fail("launch %zu (%s): streamed tiles do not cover the batch", i, ln.label.c_str());
-      if (ln.block != unsigned(W * (ln.L / ln.radix)) || ap.cpb < 2 || ap.cpb > 8)
+      const int nt = mb::stream_group(ln.L, ln.radix), groups = int(ln.block) / nt;
+      if (int(ln.block) != nt * groups || groups < 1 || groups > mb::stream_max_groups(ln.L, ln.radix) ||
+          groups > ap.cpb || ap.cpb < 2 || ap.cpb > mb::kStreamMaxStages)
         fail("launch %zu: streamed shape %u threads, %d stages", i, ln.block, ap.cpb);
       if (size_t(ap.stage_bytes) < size_t(W) * (ln.L + 1) * sizeof(cpx) || ap.stage_bytes % 128)
         fail("launch %zu: stage of %d bytes", i, ap.stage_bytes);

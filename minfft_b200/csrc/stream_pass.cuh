@@ -2,33 +2,40 @@
 // for strided columns (the column passes of multi-dimensional transforms and
 // the passes of a Stockham FFT over HBM).
 //
-// Tile.  W = 128 / sizeof(cpx) adjacent columns (transforms) of one block,
-// all L elements of each: 8 columns in double, 16 in single, so every
-// element row of the tile is one 128-byte line.  In shared memory the tile
-// is stored row by row, element n of column c at n*W + c -- exactly the
-// layout a 2-D bulk tensor copy (box of 2W reals x up to 256 rows) writes.
+// Tile.  W adjacent columns (transforms) of one block, all L elements of
+// each: every element row of the tile is a 128-byte run at 512 points and a
+// 256-byte run below, so that the tile stays within 64 KiB.  (Long runs pay:
+// the rows lie megabytes apart, and the 256-point pass of 2^26 points in f64
+// took 433 us one tile per CTA with 128-byte runs, 467 streamed with them,
+// 362 streamed with 256-byte ones.)  In shared memory the tile is stored row by row,
+// element n of column c at n*W + c -- exactly the layout a 2-D bulk tensor
+// copy (box of 2W reals x up to 256 rows) writes.
 //
 // Threads.  Thread t owns column c = t % W and holds elements j + r*(L/R)
 // (j = t / W) of it in registers, as in the one-tile kernel.  The threads
 // of one shared-memory wavefront (a quarter warp of 16-byte accesses in
-// double, a half warp of 8-byte accesses in single) are the W columns of
+// double, a half warp of 8-byte accesses in single) are adjacent columns of
 // one element row, so every load, Stockham scatter and gather of the tile
 // touches one whole 128-byte line: no padding and no bank conflicts,
 // whatever the element permutation.
 //
 // Pipeline.  Each CTA stays resident and walks tiles blockIdx.x,
 // blockIdx.x + gridDim.x, ...; S stages of shared memory hold the tiles in
-// flight.  Thread 0 issues a tile's copy into a free stage with an mbarrier
-// expecting its bytes; the CTA waits on the barrier, computes the tile in
-// place (the stage doubles as the exchange buffer) and stores from
-// registers, then refills the stage with the tile S steps ahead.  So while
-// one tile is transformed, the next S - 1 are already on their way from
-// HBM.  Where the strides do not allow a tensor copy (a row pitch that is
-// not a multiple of 16 bytes), every thread copies its share of the tile
-// with cp.async and the barrier counts the threads' arrivals instead.
+// flight and G groups of W*L/R threads take its tiles in turn (the k-th tile
+// sits in stage k % S and belongs to group k % G).  A group waits for its
+// tile's mbarrier, reads it into registers, transforms it with the stage as
+// its exchange buffer, and hands the stage back right after its last read of
+// it: one thread starts the copy of tile k + S and publishes that in
+// issued[], so the refill runs under the last pass and the stores.  Groups
+// synchronise among themselves only (named barriers), so one group loads or
+// stores while another computes: with one group per CTA the phases followed
+// each other (512-point passes of 2^26 points in f64, round trip: 2861 us
+// one tile per CTA, 3035 streamed by one group, 2571 by two).  Where the strides do not allow a tensor
+// copy (a row pitch that is not a multiple of 16 bytes), the group's threads
+// copy the tile with cp.async and the barrier counts their arrivals instead.
 //
-// Waits are bounded: a wait that runs out sets *status, the CTA stops
-// issuing, waits (bounded) for the copies it has in flight and returns.
+// Waits are bounded: a wait that runs out sets *status, the groups stop,
+// wait (bounded) for the copies in flight and return.
 #pragma once
 
 #include <cuda.h>
@@ -39,16 +46,19 @@ namespace mb {
 
 constexpr long long kStreamSpinLimit = 1LL << 22;
 
-__host__ __device__ constexpr int stream_cols() { return int(128 / sizeof(cpx)); }
+__host__ __device__ constexpr int stream_cols(int L) {
+  return L >= 512 ? int(128 / sizeof(cpx)) : int(256 / sizeof(cpx));
+}
 
 // Bytes of one stage for length L: the tile, plus one spare element per
 // column for the transposed staging of row-contiguous outputs.
 __host__ __device__ inline int stream_stage_bytes(int L) {
-  const int W = stream_cols();
+  const int W = stream_cols(L);
   return (W * (L + 1) * int(sizeof(cpx)) + 127) / 128 * 128;
 }
+constexpr int kStreamHeader = 256;  // barriers, issued[], the failure flag
 __host__ __device__ inline size_t stream_smem(int L, int stages) {
-  return 128 + size_t(stages) * stream_stage_bytes(L);
+  return kStreamHeader + size_t(stages) * stream_stage_bytes(L);
 }
 
 __device__ __forceinline__ void smbar_init(uint32_t mbar, int count) {
@@ -71,6 +81,13 @@ __device__ __forceinline__ bool smbar_wait(uint32_t mbar, uint32_t phase, long l
   return false;
 }
 
+// Barrier of the NT threads of group g (named barriers 1 ..; a group below a
+// warp is the whole CTA).
+template <int NT>
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(NT < 32 ? 32 : NT) : "memory");
+}
+
 // In-place Stockham pass of the streamed tile (layout n*W + c).
 template <int L, int R, int RP, int NS, int W>
 __device__ __forceinline__ void stream_scatter(const cpx (&v)[R], int j, int c, cpx* s) {
@@ -91,16 +108,19 @@ __device__ __forceinline__ void stream_gather(cpx (&v)[R], int j, int c, const c
   for (int r = 0; r < R; ++r) v[r] = s[(j + r * TPT) * W + c];
 }
 
-template <int L, int R, int NS, int W>
-__device__ __forceinline__ void stream_passes(cpx (&v)[R], int j, int c, cpx* s, const cpx* __restrict__ tw) {
+// `freed` runs once the group has read the tile for the last time.
+template <int L, int R, int NS, int W, class Freed>
+__device__ __forceinline__ void stream_passes(cpx (&v)[R], int j, int c, int g, cpx* s, const cpx* __restrict__ tw,
+                                              const Freed& freed) {
   constexpr int RP = (L / NS >= R) ? R : (L / NS);
+  if constexpr (NS * RP == L) freed();
   pass_compute<L, R, RP, NS>(v, j, tw);
   if constexpr (NS * RP < L) {
-    __syncthreads();
+    group_sync<W * (L / R)>(g);
     stream_scatter<L, R, RP, NS, W>(v, j, c, s);
-    __syncthreads();
+    group_sync<W * (L / R)>(g);
     stream_gather<L, R, W>(v, j, c, s);
-    stream_passes<L, R, NS * RP, W>(v, j, c, s, tw);
+    stream_passes<L, R, NS * RP, W>(v, j, c, g, s, tw, freed);
   }
 }
 
@@ -109,20 +129,32 @@ enum : int {
   F_STREAM_TMA = 1 << 8,  // the tile copies are tensor copies (else per-thread cp.async)
 };
 
+// Threads of a CTA: up to 16 warps in double (128 registers each), 32 in
+// single (64).
+constexpr int kStreamThreads = sizeof(real) == 8 ? 512 : 1024;
+constexpr int kStreamMaxStages = 16;
+__host__ __device__ constexpr int stream_group(int L, int R) { return stream_cols(L) * (L / R); }
+__host__ __device__ constexpr int stream_max_groups(int L, int R) {
+  const int nt = stream_group(L, R);
+  return nt < 32 ? 1 : (kStreamThreads / nt < 8 ? (kStreamThreads / nt < 1 ? 1 : kStreamThreads / nt) : 8);
+}
+
 template <int L, int R>
-__global__ void __launch_bounds__(stream_cols() * (L / R), 1)
+__global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 1)
     stream_pass_kernel(const AxisParams p, const __grid_constant__ CUtensorMap tmap) {
-  constexpr int W = stream_cols();
+  constexpr int W = stream_cols(L);
   constexpr int TPT = L / R;
-  constexpr int NT = W * TPT;
+  constexpr int NT = stream_group(L, R);
   constexpr int BOX = L < 256 ? L : 256;
   constexpr int C = int(sizeof(cpx));
   extern __shared__ __align__(128) unsigned char smem[];
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);  // one per stage (at most 8)
-  int* bad = reinterpret_cast<int*>(smem + 64);
-  unsigned char* stages = smem + 128;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);  // one per stage
+  volatile int* issued = reinterpret_cast<volatile int*>(smem + 128);  // last tile (by its ordinal) started into a stage
+  volatile int* bad = reinterpret_cast<volatile int*>(smem + 192);
+  unsigned char* stages = smem + kStreamHeader;
   const int S = p.cpb;  // stages
-  const int tid = threadIdx.x;
+  const int G = blockDim.x / NT;
+  const int g = threadIdx.x / NT, tid = threadIdx.x % NT;
   const int c = tid % W, j = tid / W;
   const bool tma = (p.flags & F_STREAM_TMA) != 0;
   const uint32_t mbar0 = static_cast<uint32_t>(__cvta_generic_to_shared(mbar));
@@ -130,14 +162,16 @@ __global__ void __launch_bounds__(stream_cols() * (L / R), 1)
   const int64_t gpd = (p.d0 + W - 1) / W;  // tiles per block of adjacent columns
   const int64_t ntiles = p.ntiles;
 
-  pdl_wait();
-  pdl_release();
-  if (tid == 0) {
-    for (int s = 0; s < S; ++s) smbar_init(mbar0 + 8 * s, tma ? 1 : NT);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      smbar_init(mbar0 + 8 * s, tma ? 1 : NT);
+      issued[s] = -1;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *bad = 0;
   }
   __syncthreads();
+  pdl_wait();
 
   // tile t -> first column, block indices
   auto tile_pos = [&](int64_t t, int64_t& col0, int64_t& b1, int64_t& b2) {
@@ -147,15 +181,19 @@ __global__ void __launch_bounds__(stream_cols() * (L / R), 1)
     b1 = rest - b2 * p.d1;
   };
 
-  // start the copy of tile t into stage s
-  auto issue = [&](int64_t t, int s) {
+  // start the copy of the CTA's k-th tile into its stage (all threads of one
+  // group call it)
+  auto issue = [&](int k) {
+    const int64_t t = blockIdx.x + int64_t(k) * gridDim.x;
     if (t >= ntiles) return;
+    const int s = k % S;
     int64_t col0, b1, b2;
     tile_pos(t, col0, b1, b2);
     const uint32_t mb = mbar0 + 8 * s;
     const uint32_t dst = st0 + uint32_t(s) * uint32_t(p.stage_bytes);
     if (tma) {
       if (tid == 0) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(L * W * C) : "memory");
 #pragma unroll
         for (int n0 = 0; n0 < L; n0 += BOX) {
@@ -176,35 +214,44 @@ __global__ void __launch_bounds__(stream_cols() * (L / R), 1)
         const int e = tid + i * NT;
         const int n = e / W, cc = e % W;
         if (cc < nv) {
-          const char* g = src + (int64_t(n) * p.in_n + cc * p.is0) * C;
+          const char* q = src + (int64_t(n) * p.in_n + cc * p.is0) * C;
           const uint32_t d = dst + uint32_t(e * C);
           if constexpr (C == 16)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(q) : "memory");
           else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(g) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(q) : "memory");
         }
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(mb) : "memory");
     }
+    if (tid == 0) issued[s] = k;
   };
 
-  for (int s = 0; s < S; ++s) issue(blockIdx.x + int64_t(s) * gridDim.x, s);
+  // Wait (bounded) until tile k has arrived: its copy must have been started
+  // (otherwise the barrier's phase would be ambiguous), then its phase
+  // completes.
+  auto arrived = [&](int k) {
+    const int s = k % S;
+    long long n = 0;
+    while (issued[s] != k)
+      if (++n > kStreamSpinLimit || *bad) return false;
+    return smbar_wait(mbar0 + 8 * s, uint32_t(k / S) & 1u, kStreamSpinLimit);
+  };
+
+  // the first S tiles: group 0 starts them all
+  if (g == 0)
+    for (int k = 0; k < S; ++k) issue(k);
+  pdl_release();
 
   const bool cj_in = (p.flags & F_CONJ_IN) != 0, cj_out = (p.flags & F_CONJ_OUT) != 0;
   const bool rows_out = (p.flags & F_STAGE_ROWS) != 0;
-  int it = 0;
-  bool ok = true;
-  int64_t t = blockIdx.x;
-  for (; t < ntiles; t += gridDim.x, ++it) {
-    const int s = it % S;
-    const uint32_t phase = uint32_t(it / S) & 1u;
-    if (!smbar_wait(mbar0 + 8 * s, phase, kStreamSpinLimit)) atomicExch(bad, 1);
-    __syncthreads();
-    if (*bad) {
-      ok = false;
-      break;
-    }
-    cpx* tile = reinterpret_cast<cpx*>(stages + size_t(s) * p.stage_bytes);
+  for (int k = g;; k += G) {
+    const int64_t t = blockIdx.x + int64_t(k) * gridDim.x;
+    if (t >= ntiles) break;
+    if (!arrived(k)) *bad = 1;
+    group_sync<NT>(g);
+    if (*bad) break;
+    cpx* tile = reinterpret_cast<cpx*>(stages + size_t(k % S) * p.stage_bytes);
     int64_t col0, b1, b2;
     tile_pos(t, col0, b1, b2);
     const int64_t col = col0 + c;
@@ -217,7 +264,13 @@ __global__ void __launch_bounds__(stream_cols() * (L / R), 1)
       for (int r = 0; r < R; ++r) v[r].y = -v[r].y;
     }
     if (p.st_ns > 1) hbm_pretwiddle<L, R>(v, p, col, j);
-    stream_passes<L, R, 1, W>(v, j, c, tile, p.tw);
+    auto refill = [&] {
+      group_sync<NT>(g);
+      issue(k + S);
+    };
+    stream_passes<L, R, 1, W>(v, j, c, g, tile, p.tw, [&] {
+      if (!rows_out) refill();
+    });
     if (cj_out) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r].y = -v[r].y;
@@ -234,31 +287,28 @@ __global__ void __launch_bounds__(stream_cols() * (L / R), 1)
     } else {
       // outputs of a column contiguous (out_k = 1): transpose through the
       // stage (column c at c*(L+1)), then store with k running fastest
-      __syncthreads();
+      group_sync<NT>(g);
 #pragma unroll
       for (int r = 0; r < R; ++r) tile[c * (L + 1) + j + r * TPT] = v[r];
-      __syncthreads();
+      group_sync<NT>(g);
       const int nv = int(p.d0 - col0 < W ? p.d0 - col0 : W);
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         const int e = tid + i * NT;
-        const int cc = e / L, k = e % L;
-        if (cc < nv) out[ob + (col0 + cc) * p.os0 + int64_t(k) * p.out_k] = tile[cc * (L + 1) + k];
+        const int cc = e / L, q = e % L;
+        if (cc < nv) out[ob + (col0 + cc) * p.os0 + int64_t(q) * p.out_k] = tile[cc * (L + 1) + q];
       }
+      refill();
     }
-    __syncthreads();  // the stage is free: refill it with the tile S steps ahead
-    if (tma && tid == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    issue(t + int64_t(S) * gridDim.x, s);
   }
 
-  if (!ok) {
-    if (tid == 0 && p.status) atomicExch(p.status, 1);
-    // copies already issued into the stages must land before the CTA's
-    // shared memory is released: wait for each outstanding stage (bounded)
-    for (int k = 0; k < S; ++k, ++it, t += gridDim.x) {
-      if (t >= ntiles) break;
-      smbar_wait(mbar0 + 8 * (it % S), uint32_t(it / S) & 1u, kStreamSpinLimit);
-    }
+  __syncthreads();
+  if (*bad) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1);
+    // copies already started must land before the CTA's shared memory is
+    // released: wait for the last one of each stage (bounded)
+    for (int s = 0; s < S; ++s)
+      if (issued[s] >= 0) smbar_wait(mbar0 + 8 * s, uint32_t(issued[s] / S) & 1u, kStreamSpinLimit);
   }
 }
 
