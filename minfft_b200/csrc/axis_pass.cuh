@@ -1510,103 +1510,6 @@ struct StoreDCT3Line {
   }
 };
 
-// Element-wise steps of a long real transform fused into the first or last
-// pass of a Stockham chain whose sub-DFTs hold single points of the
-// half-length sequence (one line, no mirror pairing; the mixed batch's long
-// items).  Point g of sub-DFT b is b1 + n*in_n (first pass, b1 = b % d1),
-// point m of the output is the sub-DFT's normal offset + k*out_k (last
-// pass); N = kn reals in the line.
-
-// Type-2 permutation (Op_dct2_pre): t_g = (u_2g, u_2g+1), u_i = x[2i] for
-// i < N/2, else sg * x[2N-1-2i].
-struct LoadDCT2Chain {
-  static constexpr bool kComplexIn = false;  // whether the raw input elements are complex
-  static constexpr bool kStaged = false;
-  template <int L, int R>
-  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, cpx (&v)[R]) {
-    constexpr int TPT = L / R;
-    const real* in = static_cast<const real*>(p.in);
-    const int64_t N = p.kn, H = N / 2;
-    const real sg = (p.flags & F_DST) ? real(-1) : real(1);
-    const int64_t b1 = umod(x.b, p.d1);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t g = b1 + int64_t(x.j + r * TPT) * p.in_n;
-      const int64_t i0 = 2 * g, i1 = 2 * g + 1;
-      v[r] = cmk(i0 < H ? in[2 * i0] : sg * in[2 * N - 1 - 2 * i0], i1 < H ? in[2 * i1] : sg * in[2 * N - 1 - 2 * i1]);
-    }
-  }
-};
-
-// Type-4 pre-rotation (Op_t4_pre) with a direct root table t1 = w_2N^g.
-struct LoadT4Direct {
-  static constexpr bool kComplexIn = false;  // whether the raw input elements are complex
-  static constexpr bool kStaged = false;
-  template <int L, int R>
-  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, cpx (&v)[R]) {
-    constexpr int TPT = L / R;
-    const real* in = static_cast<const real*>(p.in);
-    const int64_t N = p.kn;
-    const bool dst = (p.flags & F_DST) != 0;
-    const int64_t b1 = umod(x.b, p.d1);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t g = b1 + int64_t(x.j + r * TPT) * p.in_n;
-      const real a = in[2 * g], b = in[N - 1 - 2 * g];
-      const cpx w = ldg(p.t1 + g);
-      if (!dst) {
-        v[r] = cmul(w, cmk(a, b));
-      } else {
-        const cpx q = cmul(w, cmk(a, -b));
-        v[r] = cmk(-q.x, -q.y);
-      }
-    }
-  }
-};
-
-// Type-3 de-interleave (Op_dct3_post) of point m of the forward result.
-struct StoreDCT3Chain {
-  template <int L, int R>
-  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, const TileOffsets&,
-                                             cpx (&v)[R]) {
-    if (!x.active) return;
-    constexpr int TPT = L / R;
-    real* out = static_cast<real*>(p.out);
-    const int64_t N = p.kn, H = N / 2;
-    const bool dst = (p.flags & F_DST) != 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t m = x.oout + int64_t(x.j + r * TPT) * p.out_k;
-      const cpx w = cconj(v[r]);
-      const int64_t i0 = 2 * m, i1 = 2 * m + 1;
-      out[i0 < H ? 2 * i0 : 2 * N - 1 - 2 * i0] = (dst && i0 >= H) ? -w.x : w.x;
-      out[i1 < H ? 2 * i1 : 2 * N - 1 - 2 * i1] = (dst && i1 >= H) ? -w.y : w.y;
-    }
-  }
-};
-
-// Type-4 post-rotation (Op_t4_post) with a direct root table t2 = w_8N^(2q+1).
-struct StoreT4Direct {
-  template <int L, int R>
-  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, const TileOffsets&,
-                                             cpx (&v)[R]) {
-    if (!x.active) return;
-    constexpr int TPT = L / R;
-    real* out = static_cast<real*>(p.out);
-    const int64_t N = p.kn;
-    const bool dst = (p.flags & F_DST) != 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t m = x.oout + int64_t(x.j + r * TPT) * p.out_k;
-      const cpx T = v[r];
-      const cpx a = cmul(ldg(p.t2 + 2 * m), T);
-      const cpx b = cmul(ldg(p.t2 + (N - 1 - 2 * m)), cconj(T));
-      out[2 * m] = 2 * (dst ? a.y : a.x);
-      out[N - 1 - 2 * m] = 2 * (dst ? b.y : b.x);
-    }
-  }
-};
-
 // The fused passes of a 1-D real chain take mirror pairs of sub-DFTs into one
 // CTA: with M = d0*d1 sub-DFTs per line, slots c < cpb/2 hold sub-DFTs i of
 // the line and slots c + cpb/2 their mirrors, M-1-i for reflected pairs (and
@@ -1632,20 +1535,20 @@ MB_MIRROR(StoreR2CLine, kSpectrum);
 MB_MIRROR(StoreDCT2Line, kSpectrum);
 #undef MB_MIRROR
 
-// Batch index of the CTA's transform in slot c.
+// Batch index of the transform in slot c of a tile (one CTA per tile).
 template <MirrorKind kMirror>
-__device__ __forceinline__ int64_t tile_batch(const AxisParams& p, int c) {
+__device__ __forceinline__ int64_t tile_batch(const AxisParams& p, int c, int64_t tile) {
   if constexpr (kMirror != kNoMirror) {
     const int64_t M = p.d0 * p.d1;
     const int64_t per_line = udiv(M, p.cpb);  // CTAs per line
-    const int64_t line = udiv(int64_t(blockIdx.x), per_line), q = int64_t(blockIdx.x) - line * per_line;
+    const int64_t line = udiv(tile, per_line), q = tile - line * per_line;
     const int h = p.cpb / 2;
     const int64_t i = q * h + (c < h ? c : c - h);
     if (c < h) return line * M + i;
     if constexpr (kMirror == kReflected) return line * M + (M - 1 - i);
     return line * M + (i == 0 ? M / 2 : M - i);
   } else {
-    return int64_t(blockIdx.x) * p.cpb + c;
+    return tile * p.cpb + c;
   }
 }
 
@@ -1674,7 +1577,7 @@ __global__ void __launch_bounds__(512, MinBlocks<R>::value) axis_pass_kernel(con
       MirrorPairs<LoadOp>::value != kNoMirror ? MirrorPairs<LoadOp>::value : MirrorPairs<StoreOp>::value;
   // offsets of the CTA's transforms, computed once per transform
   for (int c = threadIdx.x; c < p.cpb; c += blockDim.x) {
-    const int64_t b = tile_batch<kMirror>(p, c);
+    const int64_t b = tile_batch<kMirror>(p, c, blockIdx.x);
     int64_t b0, oi, oo;
     batch_offsets(p, b < p.nbatch ? b : 0, b0, oi, oo);
     to.in_off[c] = oi;
@@ -1690,7 +1593,7 @@ __global__ void __launch_bounds__(512, MinBlocks<R>::value) axis_pass_kernel(con
     x.j = threadIdx.x % TPT;
     x.c = threadIdx.x / TPT;
   }
-  x.b = tile_batch<kMirror>(p, x.c);
+  x.b = tile_batch<kMirror>(p, x.c, blockIdx.x);
   x.active = x.b < p.nbatch;
   x.oin = to.in_off[x.c];
   x.oout = to.out_off[x.c];

@@ -3,44 +3,46 @@
 // graph.
 //
 // Planning (host).  Jobs are grouped by (kind, direction, length).  Each
-// group of transforms whose DFT fits in one CTA is cut into work items of up
-// to `cpb` transforms (the tile shape: the items of a length-L group use
-// L/16 threads per transform, so a 512-thread CTA holds 512*16/L of them);
-// every longer transform (64 K points at most) is one work item by itself.
-// Items are ordered by estimated cost, largest first, so the long ones start
-// early and the short ones fill the tail.
+// group of transforms whose DFT fits in one CTA (4096 points) is cut into
+// work items of up to `cpb` transforms (the items of a length-L group use
+// L/16 threads per transform, so a 256-thread CTA holds 256*16/L of them).
+// A longer transform (2^13 .. 2^16 complex points) is a Stockham chain of
+// two passes through a scratch slot, and each pass is cut into tiles of 4096
+// points, one work item each, with the kind's pre- and post-processing fused
+// into the passes (the *Line and type-4 chain stages of axis_pass.cuh, which
+// work on mirror pairs of sub-DFTs).
 //
 // Execution (device).  Every resident CTA takes the next item from an
-// atomic counter until the list is exhausted.  Short items run the same
-// load -> Stockham passes -> store code as the axis passes, with each
-// transform's own input and output pointers.  Long items (2^14 .. 2^16
-// complex points) run by default on one CTA each: two Stockham passes over
-// global memory through the CTA's private scratch slice, with the kind's
-// element-wise steps fused into them where they need no (k, L-k) pairing
-// and run as sweeps of the CTA before or after them otherwise.  With
-// MINFFT_B200_MIXED_CLUSTER=1 (where the device can co-schedule the clusters)
-// they run instead on clusters of eight CTAs entirely in distributed shared
-// memory (mixed_cluster_kernel, run_cluster_big): the clusters take the long
-// items first, one per cluster, then every CTA takes short items on its own.
-// That form moves each element through HBM once but measured slower.
+// atomic counter until the list is exhausted.  The list interleaves the
+// first-pass tiles of later transforms with the last-pass tiles of earlier
+// ones, so that a transform's last pass comes more than one grid of items
+// after its first (whose tiles are then done) and only about 1.5 grids of
+// scratch are live: the scratch stays in the L2, and each long transform
+// crosses HBM once each way.  (One CTA per long transform, two passes and
+// element-wise sweeps through a private slice, kept 300 MB of scratch live
+// and each CTA's phases in sequence: 20000 jobs of 2^4 .. 2^16 points in f32
+// took 1102 us, 1056 so.)
 //
-// No CTA ever waits on a CTA outside its own cluster (the queues are a
-// single atomicAdd per item; the CTAs of a cluster are co-resident by
-// construction), so the kernel cannot deadlock whatever the residency.
-#include <cooperative_groups.h>
+// Waits.  A last-pass tile waits until its transform's first-pass tiles are
+// done, a first-pass tile until the last transform that used its scratch
+// slot is.  What an item waits for stands before it in the list, so it has
+// been taken by a running CTA, and first-pass tiles of the first users of a
+// slot wait for nothing: the waits end whatever the residency.  They are
+// bounded all the same; one that runs out sets *status and every CTA stops.
 #include <cuda_runtime.h>
 #include <stdio.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <deque>
 #include <map>
 #include <mutex>
 #include <tuple>
 #include <vector>
 
 #include "kernel_registry.h"
-#include "line_ops.cuh"
+#include "axis_pass.cuh"
 #include "minfft_b200.h"
 
 #define MB_EXPORT extern "C" __attribute__((visibility("default")))
@@ -58,11 +60,18 @@ cudaError_t dev_malloc(T** p, size_t bytes) {
 namespace mb {
 namespace mixed {
 
-constexpr int kThreads = 512;
-constexpr int kSlots = 18;           // table slots by log2 length, 0 .. 17
-constexpr int kSmallMaxLog2L = 13;   // one-CTA DFTs up to 8192 points
-constexpr int kBigMaxLog2L = 16;     // two passes over global memory up to 65536
+constexpr int kThreads = 256;
+constexpr int kSlots = 21;           // table slots by log2 length, 0 .. 20
+constexpr int kSmallMaxLog2L = 12;   // one-CTA DFTs up to 4096 points
+constexpr int kBigMaxLog2L = 16;     // two passes through scratch up to 65536
+constexpr int kTilePoints = 16 * kThreads;  // points of a long item's tile
 constexpr int kOffsetsBytes = 1024;  // tile offsets of the long-item passes (<= 64 transforms)
+constexpr int kMinBlocks = sizeof(real) == 8 ? 2 : 4;  // CTAs per SM: 128 / 64 registers
+// Scratch of each long length: about 2.5 grids of tiles, small enough to stay
+// in the L2 beside the streams (20000 jobs in f32: 1056 us with 32 MiB, 1083
+// with 64, 1085 with 24).
+constexpr size_t kSlotBytes = size_t(32) << 20;
+constexpr long long kWaitLimit = 1LL << 22;
 
 struct Job {
   const void* in;
@@ -71,39 +80,46 @@ struct Job {
   int log2n;
 };
 
-// combo < 0: length-1 transforms (a scale or a type change per job)
-struct Item {
+enum ItemKind : int { kShort = 0, kUnit, kFirst, kLast };
+
+struct __align__(16) Item {
+  int kind;
   int combo;
   int log2L;
   int flags;
-  int count;
-  int first;  // index into the job order
-  int big;
+  int count;  // short items: transforms
+  int first;  // short items: index of the first job
+  int tile;   // long items: tile of the pass
+  int id;     // long items: index of the transform's completion counters
+  int dep;    // first-pass tiles: transform whose last pass frees the slot, or -1
   int op;
-  int pad;
+  int64_t scratch;  // long items: offset of the slot (complex elements)
+  const void* in;   // long items: the job's arrays
+  void* out;
 };
 
 struct Params {
-  const Job* jobs;
-  const int* order;
+  const Job* jobs;  // in item order
   const Item* items;
   int nitems;
-  int nbig;            // items [0, nbig) are long items (cluster form), the rest short ones
-  unsigned* counter;   // [0]: next short item, [1]: next long item (cluster form)
+  int nbig;           // long transforms
+  unsigned* counter;  // the queue, then nbig counters of finished first-pass tiles and nbig of last-pass tiles
+  int* status;        // host-mapped; set when a wait ran out
   cpx* scratch;
-  int64_t scratch_stride;  // complex elements per CTA (two buffers)
   const cpx* tw[kSlots];    // w_L^m, by log2 L
   const cpx* rft[kSlots];   // real-DFT roots, by log2 N
   const cpx* t23[kSlots];   // type-2/3 roots, by log2 N
   const cpx* t4a[kSlots];   // type-4 pre-rotation, by log2 N
   const cpx* t4b[kSlots];   // type-4 post-rotation, by log2 N
-  const cpx* sthi[kSlots];  // coarse roots of a long length, by log2 L
-  const cpx* stlo[kSlots];  // fine roots of a long length, by log2 L
+  const cpx* sthi[kSlots];  // coarse roots of a long length, by log2 of it
+  const cpx* stlo[kSlots];  // fine roots of a long length
 };
 
 __host__ __device__ constexpr int small_radix(int L) { return L < 16 ? L : 16; }
 __host__ __device__ constexpr int log2c(int v) { return v <= 1 ? 0 : 1 + log2c(v / 2); }
 __host__ __device__ constexpr int small_cpb(int L) { return kThreads / (L / small_radix(L)); }
+__host__ __device__ constexpr int first_bits(int lg) { return (lg + 1) / 2; }  // pass lengths of a long DFT
+__host__ __device__ constexpr int root_bits(int lg) { return (lg + 1) / 2; }   // fine bits of a root pair
 
 // ---------------------------------------------------------------- device
 template <int L, class LoadOp, class StoreOp>
@@ -114,7 +130,7 @@ __device__ __noinline__ void run_small(const Params& mp, const Item& it, unsigne
   const int c = threadIdx.x / TPT, j = threadIdx.x % TPT;
   const bool active = c < it.count;
   Job job{};
-  if (active) job = mp.jobs[mp.order[it.first + c]];
+  if (active) job = mp.jobs[it.first + c];
   const int log2N = (it.combo == K_CPLX) ? it.log2L : it.log2L + 1;
   AxisParams p;
   memset(&p, 0, sizeof(p));
@@ -166,180 +182,190 @@ __device__ __noinline__ void run_small(const Params& mp, const Item& it, unsigne
   StoreOp::template run<L, R>(p, x, t, to, v);
 }
 
-// One Stockham pass over global memory of a long transform of length 2^LG,
-// sub-DFTs of length RP, span NS (1 or the length of the first pass).
-// Ld / St: the load and store stages (complex by default; the fused type-2
-// permutation and type-4 pre-rotation in the first pass, the fused type-3
-// de-interleave and type-4 post-rotation in the last, with the line's real
-// length kn and direct root tables t1, t2).
-template <int LG, int RP, int NS, class Ld = LoadCplx, class St = StoreCplx>
-__device__ __forceinline__ void big_pass(const Params& mp, const void* src, void* dst, int flags,
-                                         unsigned char* smem, int64_t kn = 0, const cpx* t1 = nullptr,
-                                         const cpx* t2 = nullptr) {
-  constexpr int Lc = 1 << LG;
-  constexpr int R = 16;
-  constexpr int TPT = RP / R;
-  constexpr int CPB = kThreads / TPT;
-  constexpr int NJ = Lc / RP;
+// Real rows read and written as complex pairs, by scalars where the row is
+// not aligned for pairs (the first pass of the real DFT, the last of its
+// inverse).
+struct LoadRealPairs {
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
+    if (p.flags & F_VEC) {
+      LoadCplx::run<L, R>(p, x, t, v);
+      return;
+    }
+    const real* in = static_cast<const real*>(p.in);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const real* q = in + 2 * (x.oin + int64_t(x.j + r * (L / R)) * p.in_n);
+      v[r] = cmk(q[0], q[1]);
+    }
+  }
+};
+struct StoreRealPairs {
+  template <int L, int R>
+  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets& to,
+                                             cpx (&v)[R]) {
+    if (p.flags & F_VEC) {
+      StoreCplx::run<L, R>(p, x, t, to, v);
+      return;
+    }
+    real* out = static_cast<real*>(p.out);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      real* q = out + 2 * (x.oout + int64_t(x.j + r * (L / R)) * p.out_k);
+      q[0] = v[r].x;
+      q[1] = -v[r].y;
+    }
+  }
+};
+
+// Finished tiles of a long transform's pass, counted in global memory.
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// Waits (bounded) until *p reaches n; all threads of the CTA call it.
+__device__ __forceinline__ bool tiles_done(const Params& mp, const unsigned* p, unsigned n) {
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    long long i = 0;
+    while (ld_acquire(p) < n)
+      if (++i > kWaitLimit) {
+        ok = false;
+        *reinterpret_cast<volatile int*>(mp.status) = 1;
+        break;
+      }
+  }
+  return __syncthreads_and(ok) != 0;
+}
+// Counts one finished tile.  The barrier orders every thread's writes before
+// thread 0's release, which is cumulative: no fence of their own.
+__device__ __forceinline__ void tile_done(unsigned* p) {
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
+
+// One tile of a pass of a long transform of 2^lg points: CPB sub-DFTs of RP
+// points (16 values per thread).  The first pass reads the job's input and
+// writes its sub-DFTs contiguously into the scratch slot; the last pass
+// reads that with the Stockham pre-twiddle and writes the job's output.
+template <int RP, bool kIsLast, class Ld, class St>
+__device__ __noinline__ void run_tile(const Params& mp, const Item& it, unsigned char* smem) {
+  constexpr int R = 16, TPT = RP / R, CPB = kThreads / TPT;
   static_assert(CPB * 2 * sizeof(int64_t) <= kOffsetsBytes, "offsets region");
+  const int lg = it.log2L;
+  const int M = (1 << lg) / RP;  // sub-DFTs of the pass
+  const int log2N = it.combo == K_CPLX ? lg : lg + 1;
   AxisParams p;
   memset(&p, 0, sizeof(p));
-  p.in = src;
-  p.out = dst;
-  p.nbatch = NJ;
-  p.d0 = NS;
-  p.d1 = Lc / (NS * RP);
-  p.is0 = 1;
-  p.is1 = NS;
-  p.is2 = Lc;
-  p.in_n = Lc / RP;
-  p.os0 = 1;
-  p.os1 = NS * RP;
-  p.os2 = Lc;
-  p.out_k = NS;
-  p.st_ns = NS;
+  p.nbatch = M;
+  p.d0 = kIsLast ? M : 1;
+  p.d1 = kIsLast ? 1 : M;
+  p.is0 = p.is1 = 1;
+  p.in_n = M;
+  p.out_k = kIsLast ? M : 1;
+  p.st_ns = kIsLast ? M : 1;
   p.st_div = 1;
-  p.st_shift = 0;
-  p.st_lobits = (LG + 1) / 2;
-  p.st_hi = mp.sthi[LG];
-  p.st_lo = mp.stlo[LG];
   p.tw = mp.tw[log2c(RP)];
   p.cpb = CPB;
   p.colmode = 1;
-  p.flags = flags | (NS == 1 ? F_STAGE_ROWS : 0);
   p.lp = tile_pitch(RP, R, CPB, 1);
-  p.kn = kn;
-  p.t1 = t1;
-  p.t2 = t2;
+  p.kn = int64_t(1) << log2N;
+  // root pairs of the fused step: 2N before and 8N after a type-4 chain, 4N
+  // for types 2 and 3, N for the real DFT
+  const int lr = it.combo == K_T4                               ? log2N + (kIsLast ? 3 : 1)
+                 : (it.combo == K_DCT2 || it.combo == K_DCT3) ? log2N + 2
+                                                              : log2N;
+  if constexpr (kIsLast) {
+    p.in = mp.scratch + it.scratch;
+    p.out = it.out;
+    p.flags = (it.flags & (F_DST | F_CONJ_OUT | F_VEC)) | F_SRC_SMEM;  // scratch by plain loads: it stays in the L2
+    p.st_lobits = root_bits(lg);
+    p.st_hi = mp.sthi[lg];
+    p.st_lo = mp.stlo[lg];
+    p.t1 = mp.sthi[lr];
+    p.t2 = mp.stlo[lr];
+    p.kbits = root_bits(lr);
+  } else {
+    p.in = it.in;
+    p.out = mp.scratch + it.scratch;
+    p.flags = (it.flags & (F_DST | F_CONJ_IN | F_VEC)) | F_STAGE_ROWS;
+    p.st_lobits = root_bits(lr);
+    p.st_hi = mp.sthi[lr];
+    p.st_lo = mp.stlo[lr];
+  }
+  constexpr MirrorKind kMirror = MirrorPairs<Ld>::value != kNoMirror ? MirrorPairs<Ld>::value : MirrorPairs<St>::value;
   int64_t* offs = reinterpret_cast<int64_t*>(smem);
+  if (!kIsLast && threadIdx.x < CPB) offs[threadIdx.x] = tile_batch<kMirror>(p, threadIdx.x, it.tile) * RP;
   Tile t{reinterpret_cast<cpx*>(smem + kOffsetsBytes), p.lp};
-  const int c = threadIdx.x % CPB, j = threadIdx.x / CPB;
-  for (int round = 0; round * CPB < NJ; ++round) {
-    const int64_t base = int64_t(round) * CPB;
-    if (threadIdx.x < CPB) {
-      int64_t b0, oi, oo;
-      batch_offsets(p, base + threadIdx.x < NJ ? base + threadIdx.x : 0, b0, oi, oo);
-      offs[threadIdx.x] = oi;
-      offs[CPB + threadIdx.x] = oo;
-    }
-    __syncthreads();
-    const int left = int(NJ - base);
-    TileOffsets to{offs, offs + CPB, left < CPB ? left : CPB};
-    Ctx x;
-    x.c = c;
-    x.j = j;
-    x.b = base + c;
-    x.active = x.b < NJ;
-    x.b0 = umod(x.b, p.d0);
-    x.oin = offs[c];
-    x.oout = offs[CPB + c];
-    cpx v[R];
-    Ld::template run<RP, R>(p, x, t, v);
-    run_passes<RP, R, 1>(v, j, c, t, p.tw);
-    St::template run<RP, R>(p, x, t, to, v);
-    __syncthreads();
+  TileOffsets to{offs, offs, CPB};
+  Ctx x;
+  x.c = threadIdx.x % CPB;
+  x.j = threadIdx.x / CPB;
+  x.b = tile_batch<kMirror>(p, x.c, it.tile);
+  x.b0 = kIsLast ? x.b : 0;
+  x.oin = x.b;
+  x.oout = kIsLast ? x.b : x.b * RP;
+  x.active = true;
+  cpx v[R];
+  Ld::template run<RP, R>(p, x, t, v);
+  run_passes<RP, R, 1>(v, x.j, x.c, t, p.tw);
+  St::template run<RP, R>(p, x, t, to, v);
+}
+
+template <int RP>
+__device__ __forceinline__ void run_first(const Params& mp, const Item& it, unsigned char* smem) {
+  switch (it.combo) {
+    case K_CPLX: run_tile<RP, false, LoadCplx, StoreCplx>(mp, it, smem); break;
+    case K_R2C: run_tile<RP, false, LoadRealPairs, StoreCplx>(mp, it, smem); break;
+    case K_C2R: run_tile<RP, false, LoadC2RLine, StoreCplx>(mp, it, smem); break;
+    case K_DCT2: run_tile<RP, false, LoadDCT2Line, StoreCplx>(mp, it, smem); break;
+    case K_DCT3: run_tile<RP, false, LoadDCT3Line, StoreCplx>(mp, it, smem); break;
+    default: run_tile<RP, false, LoadT4Chain, StoreCplx>(mp, it, smem); break;
   }
 }
 
-// A line step over one long item by the whole CTA: each thread takes items
-// tid, tid + blockDim.x, ... and issues the loads of kBatch of them before
-// computing and storing any, so the CTA keeps several loads per thread in
-// flight instead of one (this walk is a single CTA's, not a grid's).
-template <class Op>
-__device__ __forceinline__ void cta_line(const LineParams& lp) {
-  constexpr int kBatch = sizeof(typename Op::In) <= 3 * sizeof(cpx) ? 4 : 2;
-  const int64_t total = Op::count(lp);
-  const int64_t step = blockDim.x;
-  // one line (outer = inner = 1): item e is point e of the line
-  int64_t e = threadIdx.x;
-  for (; e + (kBatch - 1) * step < total; e += kBatch * step) {
-    typename Op::In v[kBatch];
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) v[u] = Op::load_at(lp, ItemIdx{0, e + u * step, 0});
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) Op::finish_at(lp, ItemIdx{0, e + u * step, 0}, v[u]);
+template <int RP>
+__device__ __forceinline__ void run_last(const Params& mp, const Item& it, unsigned char* smem) {
+  switch (it.combo) {
+    case K_CPLX: run_tile<RP, true, LoadCplx, StoreCplx>(mp, it, smem); break;
+    case K_R2C: run_tile<RP, true, LoadCplx, StoreR2CLine>(mp, it, smem); break;
+    case K_C2R: run_tile<RP, true, LoadCplx, StoreRealPairs>(mp, it, smem); break;
+    case K_DCT2: run_tile<RP, true, LoadCplx, StoreDCT2Line>(mp, it, smem); break;
+    case K_DCT3: run_tile<RP, true, LoadCplx, StoreDCT3Line>(mp, it, smem); break;
+    default: run_tile<RP, true, LoadCplx, StoreT4Chain>(mp, it, smem); break;
   }
-  for (; e < total; e += step) Op::finish_at(lp, ItemIdx{0, e, 0}, Op::load_at(lp, ItemIdx{0, e, 0}));
 }
 
-template <int LG>
-__device__ __noinline__ void run_big(const Params& mp, const Item& it, unsigned char* smem) {
-  constexpr int Lc = 1 << LG;
-  constexpr int B1 = (LG + 1) / 2, B2 = LG - B1;
-  constexpr int R1 = 1 << B1, R2 = 1 << B2;
-  const Job job = mp.jobs[mp.order[it.first]];
-  cpx* S1 = mp.scratch + int64_t(blockIdx.x) * mp.scratch_stride;
-  cpx* S2 = S1 + mp.scratch_stride / 2;
-  const int log2N = (it.combo == K_CPLX) ? LG : LG + 1;
-  LineParams lp;
-  memset(&lp, 0, sizeof(lp));
-  lp.outer = 1;
-  lp.inner = 1;
-  lp.L = Lc;
-  lp.in_sn = 1;
-  lp.out_sn = 1;
-  lp.flags = it.flags;
-  const int64_t N = int64_t(1) << log2N;  // the real length (real kinds)
-  const cpx* src = static_cast<const cpx*>(job.in);
-  // element-wise pre-processing into S1 where it needs the pair (k, L-k)
-  // (the type-2 permutation and type-4 pre-rotation are fused into the
-  // first pass instead)
-  if (it.combo == K_C2R || it.combo == K_DCT3) {
-    lp.in = job.in;
-    lp.out = S1;
-    if (it.combo == K_C2R) {
-      lp.t2 = mp.rft[log2N];
-      cta_line<Op_c2r_pack>(lp);
-    } else {
-      lp.t1 = mp.t23[log2N];
-      lp.t2 = mp.rft[log2N];
-      cta_line<Op_dct3_pack>(lp);
+__device__ __forceinline__ bool run_long(const Params& mp, const Item& it, unsigned char* smem) {
+  unsigned* firsts = mp.counter + 1;
+  unsigned* lasts = firsts + mp.nbig;
+  const unsigned tiles = unsigned(1 << it.log2L) / kTilePoints;
+  if (it.kind == kFirst) {
+    // the slot's previous user has the same length, hence as many tiles
+    if (it.dep >= 0 && !tiles_done(mp, lasts + it.dep, tiles)) return false;
+    if (first_bits(it.log2L) == 7)
+      run_first<128>(mp, it, smem);
+    else
+      run_first<256>(mp, it, smem);
+    tile_done(firsts + it.id);
+  } else {
+    if (!tiles_done(mp, firsts + it.id, tiles)) return false;
+    switch (it.log2L - first_bits(it.log2L)) {
+      case 6: run_last<64>(mp, it, smem); break;
+      case 7: run_last<128>(mp, it, smem); break;
+      default: run_last<256>(mp, it, smem); break;
     }
-    src = S1;
-    __syncthreads();
+    tile_done(lasts + it.id);
   }
-  cpx* mid = (src == S1) ? S2 : S1;
-  const bool inv_cplx = (it.combo == K_CPLX) && (it.flags & F_CONJ_IN);
-  const int kf = it.flags & F_DST;
-  if (it.combo == K_DCT2)
-    big_pass<LG, R1, 1, LoadDCT2Chain>(mp, job.in, mid, kf, smem, N);
-  else if (it.combo == K_T4)
-    big_pass<LG, R1, 1, LoadT4Direct>(mp, job.in, mid, kf, smem, N, mp.t4a[log2N]);
-  else
-    big_pass<LG, R1, 1>(mp, src, mid, inv_cplx ? F_CONJ_IN : 0, smem);
-  __syncthreads();
-  // the last pass writes the output itself for the complex DFT, the
-  // inverse real DFT and the fused type-3 de-interleave and type-4
-  // post-rotation; the real DFT and the DCT-2 unpack the pairs afterwards
-  const bool pairs = it.combo == K_R2C || it.combo == K_DCT2;
-  cpx* fin = pairs ? (mid == S1 ? S2 : S1) : static_cast<cpx*>(job.out);
-  const bool conj_out = inv_cplx || it.combo == K_C2R;
-  if (it.combo == K_DCT3)
-    big_pass<LG, R2, R1, LoadCplx, StoreDCT3Chain>(mp, mid, job.out, kf, smem, N);
-  else if (it.combo == K_T4)
-    big_pass<LG, R2, R1, LoadCplx, StoreT4Direct>(mp, mid, job.out, kf, smem, N, nullptr, mp.t4b[log2N]);
-  else
-    big_pass<LG, R2, R1>(mp, mid, fin, conj_out ? F_CONJ_OUT : 0, smem);
-  __syncthreads();
-  if (pairs) {
-    lp.in = fin;
-    lp.out = job.out;
-    if (it.combo == K_R2C) {
-      lp.t1 = mp.rft[log2N];
-      cta_line<Op_r2c_unpack>(lp);
-    } else {
-      lp.t1 = mp.t23[log2N];
-      lp.t2 = mp.rft[log2N];
-      cta_line<Op_dct2_post>(lp);
-    }
-  }
+  return true;
 }
 
 // length-1 transforms: y = 2x (type 2), x (type 3), sqrt(2) x (type 4),
 // (x, 0) (real DFT), Re z (inverse real DFT), z (complex DFT)
 __device__ __noinline__ void run_unit(const Params& mp, const Item& it) {
   for (int c = threadIdx.x; c < it.count; c += blockDim.x) {
-    const Job job = mp.jobs[mp.order[it.first + c]];
+    const Job job = mp.jobs[it.first + c];
     switch (job.op) {
       case MINFFT_B200_DFT:
       case MINFFT_B200_INVDFT: *static_cast<cpx*>(job.out) = *static_cast<const cpx*>(job.in); break;
@@ -372,29 +398,45 @@ __device__ __forceinline__ void run_small_any(const Params& mp, const Item& it, 
     case 10: run_small<1024, Ld, St>(mp, it, smem); break;
     case 11: run_small<2048, Ld, St>(mp, it, smem); break;
     case 12: run_small<4096, Ld, St>(mp, it, smem); break;
-    case 13: run_small<8192, Ld, St>(mp, it, smem); break;
     default: break;
   }
 }
 
-__global__ void __launch_bounds__(kThreads, MinBlocks<16>::value) mixed_kernel(const __grid_constant__ Params mp) {
+__global__ void __launch_bounds__(kThreads, kMinBlocks) mixed_kernel(const __grid_constant__ Params mp) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_item;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = int(atomicAdd(mp.counter, 1u));
+  __shared__ int s_item[2];
+  __shared__ Item s_desc[2];
+  // Thread 0 keeps one index ahead of the item being prepared: while item n
+  // runs, the descriptor of item n + 1 is on its way into shared memory and
+  // the index of item n + 2 is taken from the queue.
+  unsigned ahead = 0;
+  auto fetch = [&](int idx, int slot) {
+    s_item[slot] = idx;
+    if (idx < mp.nitems) {
+      const char* src = reinterpret_cast<const char*>(mp.items + idx);
+      const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(&s_desc[slot]));
+#pragma unroll
+      for (int i = 0; i < int(sizeof(Item)); i += 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i), "l"(src + i) : "memory");
+    }
+  };
+  if (threadIdx.x == 0) {
+    fetch(int(atomicAdd(mp.counter, 1u)), 0);
+    ahead = atomicAdd(mp.counter, 1u);
+  }
+  for (int n = 0;; ++n) {
+    if (threadIdx.x == 0) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int idx = s_item;
-    __syncthreads();
-    if (idx >= mp.nitems) break;
-    const Item it = mp.items[idx];
-    if (it.big) {
-      switch (it.log2L) {
-        case 14: run_big<14>(mp, it, smem); break;
-        case 15: run_big<15>(mp, it, smem); break;
-        case 16: run_big<16>(mp, it, smem); break;
-        default: break;
-      }
-    } else if (it.combo < 0) {
+    if (s_item[n & 1] >= mp.nitems) break;
+    const Item it = s_desc[n & 1];
+    if (threadIdx.x == 0) {
+      fetch(int(ahead), (n + 1) & 1);
+      ahead = atomicAdd(mp.counter, 1u);
+    }
+    bool ok = true;
+    if (it.kind >= kFirst) {
+      ok = run_long(mp, it, smem);
+    } else if (it.kind == kUnit) {
       run_unit(mp, it);
     } else {
       switch (it.combo) {
@@ -406,324 +448,8 @@ __global__ void __launch_bounds__(kThreads, MinBlocks<16>::value) mixed_kernel(c
         default: run_small_any<LoadT4, StoreT4>(mp, it, smem); break;
       }
     }
-    __syncthreads();
+    if (!ok) break;
   }
-}
-
-// ------------------------------------------------- long items on a cluster
-// A long item (L = 2^14 .. 2^16 complex points) is computed by a cluster of
-// kCluster CTAs entirely in their shared memory (the four-step split
-// n = 256*n1 + n2, k = k1 + N1*k2, N1 = L/256): CTA r holds the 32 columns
-// n2 = 32r .. 32r+31 of all N1 rows, computes their length-N1 DFTs over n1
-// (with the kind's pre-processing fused into the global loads) and the
-// twiddles w_L^(n2 k1); after a cluster barrier it gathers, through
-// distributed shared memory, rows k1 = r*N1/8 .. (r+1)*N1/8-1 from all eight
-// CTAs and computes their length-256 DFTs over n2, then applies the kind's
-// post-processing (reading the partner outputs z_{L-k} of the real DFT and
-// DCT-2 from the CTA that holds them) and stores.  Each element is read from
-// and written to global memory once.
-constexpr int kCluster = 8;
-constexpr int kN2 = 256;
-constexpr int kColsPerCta = kN2 / kCluster;  // 32
-
-// Element n (< L) of the complex sequence whose length-L DFT a long item of
-// kind it.combo needs: the pre-processing steps of line_ops.cuh, per element.
-__device__ __forceinline__ cpx big_pre(const Params& mp, const Item& it, const Job& job, int LG, int64_t n) {
-  const int64_t L = int64_t(1) << LG, N = 2 * L;
-  const int log2N = LG + 1;
-  const bool dst = (it.flags & F_DST) != 0;
-  switch (it.combo) {
-    case K_CPLX: {
-      cpx x = static_cast<const cpx*>(job.in)[n];
-      if (it.flags & F_CONJ_IN) x.y = -x.y;
-      return x;
-    }
-    case K_R2C:
-      return static_cast<const cpx*>(job.in)[n];  // the real row as pairs (aligned: checked at planning)
-    case K_DCT2: {
-      const real* in = static_cast<const real*>(job.in);
-      const real sg = dst ? real(-1) : real(1);
-      const int64_t i0 = 2 * n, i1 = 2 * n + 1;
-      const real a = i0 < L ? in[2 * i0] : sg * in[2 * N - 1 - 2 * i0];
-      const real b = i1 < L ? in[2 * i1] : sg * in[2 * N - 1 - 2 * i1];
-      return cmk(a, b);
-    }
-    case K_T4: {
-      const real* in = static_cast<const real*>(job.in);
-      const real a = in[2 * n], b = in[N - 1 - 2 * n];
-      const cpx w = ldg(mp.t4a[log2N] + n);
-      if (!dst) return cmul(w, cmk(a, b));
-      const cpx q = cmul(w, cmk(a, -b));
-      return cmk(-q.x, -q.y);
-    }
-    default: {  // K_C2R and K_DCT3: packing of the pair (n, L-n), conjugated
-      const cpx* zin = static_cast<const cpx*>(job.in);
-      const real* rin = static_cast<const real*>(job.in);
-      auto z = [&](int64_t k) -> cpx {
-        if (it.combo == K_C2R) return zin[k];
-        auto rd = [&](int i) { return rin[i]; };
-        return LoadDCT3::zval_r(rd, int(k), int(L), dst, mp.t23[log2N]);
-      };
-      const cpx* rft = mp.rft[log2N];
-      if (n == 0) {
-        const cpx z0 = z(0), z1 = z(L);
-        return cmk(z0.x + z1.x, -(z0.x - z1.x));
-      }
-      if (2 * n == L) {
-        const cpx z0 = z(n);
-        return cmk(2 * z0.x, 2 * z0.y);
-      }
-      cpx ta, tb;
-      if (2 * n < L) {
-        pack_pair(z(n), z(L - n), ldg(rft + n), ta, tb);
-        return cconj(ta);
-      }
-      pack_pair(z(L - n), z(n), ldg(rft + (L - n)), ta, tb);
-      return cconj(tb);
-    }
-  }
-}
-
-// Outputs of a long item for DFT output z_k of a kind without pairing.
-__device__ __forceinline__ void big_post_single(const Params& mp, const Item& it, const Job& job, int LG, int64_t k,
-                                                cpx zk) {
-  const int64_t L = int64_t(1) << LG, N = 2 * L;
-  const int log2N = LG + 1;
-  const bool dst = (it.flags & F_DST) != 0;
-  switch (it.combo) {
-    case K_CPLX:
-      if (it.flags & F_CONJ_OUT) zk.y = -zk.y;
-      static_cast<cpx*>(job.out)[k] = zk;
-      break;
-    case K_C2R:
-      static_cast<cpx*>(job.out)[k] = cconj(zk);  // the real output as pairs (aligned: checked at planning)
-      break;
-    case K_DCT3: {
-      real* out = static_cast<real*>(job.out);
-      const cpx w = cconj(zk);
-      const int64_t i0 = 2 * k, i1 = 2 * k + 1;
-      const real a = (dst && i0 >= L) ? -w.x : w.x;
-      const real b = (dst && i1 >= L) ? -w.y : w.y;
-      out[i0 < L ? 2 * i0 : 2 * N - 1 - 2 * i0] = a;
-      out[i1 < L ? 2 * i1 : 2 * N - 1 - 2 * i1] = b;
-      break;
-    }
-    default: {  // K_T4
-      real* out = static_cast<real*>(job.out);
-      const cpx* t4b = mp.t4b[log2N];
-      const cpx a = cmul(ldg(t4b + 2 * k), zk);
-      const cpx b = cmul(ldg(t4b + (N - 1 - 2 * k)), cconj(zk));
-      out[2 * k] = 2 * (dst ? a.y : a.x);
-      out[N - 1 - 2 * k] = 2 * (dst ? b.y : b.x);
-      break;
-    }
-  }
-}
-
-// Outputs of the pairing kinds (real DFT, DCT-2) from z_k and z_{L-k}, for
-// 0 <= k <= L/2 (k = 0 also covers X_L; zb is unused there and at k = L/2).
-__device__ __forceinline__ void big_post_pair(const Params& mp, const Item& it, const Job& job, int LG, int64_t k,
-                                              cpx za, cpx zb) {
-  const int64_t L = int64_t(1) << LG, N = 2 * L;
-  const int log2N = LG + 1;
-  const cpx* rft = mp.rft[log2N];
-  if (it.combo == K_R2C) {
-    cpx* out = static_cast<cpx*>(job.out);
-    if (k == 0) {
-      out[0] = cmk(za.x + za.y, real(0));
-      out[L] = cmk(za.x - za.y, real(0));
-    } else if (2 * k == L) {
-      out[k] = cconj(za);
-    } else {
-      cpx xa, xb;
-      unpack_pair(za, zb, ldg(rft + k), xa, xb);
-      out[k] = xa;
-      out[L - k] = xb;
-    }
-    return;
-  }
-  real* out = static_cast<real*>(job.out);
-  const bool dst = (it.flags & F_DST) != 0;
-  const cpx* t23 = mp.t23[log2N];
-  if (k == 0) {
-    const real r2 = real(1.414213562373095048801688724209698079);
-    out[dst ? N - 1 : 0] = 2 * (za.x + za.y);
-    out[dst ? L - 1 : L] = r2 * (za.x - za.y);
-  } else if (2 * k == L) {
-    StoreDCT2::emit(out, 1, int(k), int(N), dst, cconj(za), ldg(t23 + k));
-  } else {
-    cpx xa, xb;
-    unpack_pair2(za, zb, ldg(rft + k), xa, xb);
-    StoreDCT2::emit2(out, 1, int(k), int(N), dst, xa, ldg(t23 + k));
-    StoreDCT2::emit2(out, 1, int(L - k), int(N), dst, xb, ldg(t23 + (L - k)));
-  }
-}
-
-// Row k1 of step 2 held by CTA `rank` at local index kk < K1.  The pairing
-// kinds (real DFT, DCT-2) need z_k beside z_{L-k}: with k = k1 + N1*k2, the
-// partner sits in row N1 - k1 (rows 0 and N1/2 are their own partners), so
-// their CTAs take the rows in mirrored pairs (base + p, N1 - base - p),
-// base = rank*K1/2 (CTA 0: rows 0 and N1/2, then its pairs) and every partner
-// is local.  The other kinds take K1 consecutive rows, so that their stores
-// run along k1.
-template <int N1, int K1>
-__device__ __forceinline__ int step2_row(bool pairs, int rank, int kk) {
-  if (!pairs) return rank * K1 + kk;
-  const int p = kk >> 1, base = rank * (K1 / 2);
-  if (rank == 0 && p == 0) return (kk & 1) ? N1 / 2 : 0;
-  return (kk & 1) ? N1 - (base + p) : base + p;
-}
-
-// One long item on the cluster.  Two cluster barriers: after step 1 (every
-// CTA's columns are in its tile) and after the gather of step 2 (no CTA reads
-// another's tile any more, so each may overwrite its own, for step 2's
-// exchanges and for the next item).  `next` is the index of the cluster's next
-// item, which cluster rank 0 has written to its slot before this item began;
-// it is read once the first barrier has made it visible.
-template <int LG>
-__device__ __noinline__ int run_cluster_big(const Params& mp, const Item& it, unsigned char* smem, const int* next) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  constexpr int L = 1 << LG;
-  constexpr int N1 = L / kN2;                 // 64, 128, 256
-  constexpr int TPT1 = kThreads / kColsPerCta;  // 16 threads per column in step 1
-  constexpr int R1 = N1 / TPT1;               // 4, 8, 16
-  constexpr int K1 = N1 / kCluster;           // rows k1 per CTA in step 2: 8, 16, 32
-  constexpr int TPT2 = kThreads / K1;         // 64, 32, 16
-  constexpr int R2 = kN2 / TPT2;              // 4, 8, 16
-  static_assert(R1 >= 4 && R2 >= 4 && TPT1 * kColsPerCta == kThreads && K1 >= 4, "shape");
-  const int rank = int(cl.block_rank());
-  const Job job = mp.jobs[mp.order[it.first]];
-  cpx* tile = reinterpret_cast<cpx*>(smem + kOffsetsBytes);
-  const int lp1 = tile_pitch(N1, R1, kColsPerCta, 1);
-  const int lp2 = tile_pitch(kN2, R2, K1, 1);
-  const int lobits = (LG + 1) / 2;
-  const int64_t lomask = (int64_t(1) << lobits) - 1;
-  const bool pairs = it.combo == K_R2C || it.combo == K_DCT2;
-
-  // ---- step 1: DFTs over n1 of the columns n2 = 32*rank + c
-  {
-    const int c = threadIdx.x % kColsPerCta, j = threadIdx.x / kColsPerCta;
-    const int n2 = rank * kColsPerCta + c;
-    Tile t{tile, lp1};
-    cpx v[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) v[r] = big_pre(mp, it, job, LG, int64_t(kN2) * (j + r * TPT1) + n2);
-    run_passes<N1, R1, 1>(v, j, c, t, mp.tw[log2c(N1)]);
-    // v[r] = output k1 = j + r*TPT1; twiddle w_L^(n2 k1)
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      const int64_t g = int64_t(n2) * (j + r * TPT1);
-      v[r] = cmul(v[r], cmul(ldg(mp.sthi[LG] + (g >> lobits)), ldg(mp.stlo[LG] + (g & lomask))));
-    }
-    __syncthreads();
-    scatter_natural<N1, R1>(v, j, c, t);
-  }
-  cl.sync();
-  const int nxt = *cl.map_shared_rank(next, 0);
-
-  // ---- step 2: DFTs over n2 of the CTA's K1 rows
-  const int kk = threadIdx.x % K1, j2 = threadIdx.x / K1;
-  const int k1 = step2_row<N1, K1>(pairs, rank, kk);
-  cpx v[R2];
-#pragma unroll
-  for (int r = 0; r < R2; ++r) {
-    const int n2 = j2 + r * TPT2;
-    const cpx* src = cl.map_shared_rank(tile, n2 / kColsPerCta);
-    v[r] = src[(n2 % kColsPerCta) * lp1 + pad16(k1)];
-  }
-  cl.sync();  // every remote read of this CTA's tile is done
-  Tile t2{tile, lp2};
-  run_passes<kN2, R2, 1>(v, j2, kk, t2, mp.tw[log2c(kN2)]);
-  // v[r] = z_k, k = k1 + N1*k2, k2 = j2 + r*TPT2
-  if (pairs) {
-    __syncthreads();
-    scatter_natural<kN2, R2>(v, j2, kk, t2);
-    __syncthreads();
-    // partner row: the other member of the pair (rows 0 and N1/2: the row itself)
-    const int pkk = (rank == 0 && kk < 2) ? kk : (kk ^ 1);
-#pragma unroll
-    for (int r = 0; r < R2; ++r) {
-      const int k2 = j2 + r * TPT2;
-      const int64_t k = int64_t(k1) + int64_t(N1) * k2;
-      if (2 * k > L) continue;
-      cpx zb = czero();
-      if (k != 0 && 2 * k != L) {
-        const int pk2 = k1 == 0 ? kN2 - k2 : kN2 - 1 - k2;
-        zb = tile[pkk * lp2 + pad16(pk2)];
-      }
-      big_post_pair(mp, it, job, LG, k, v[r], zb);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < R2; ++r) big_post_single(mp, it, job, LG, int64_t(k1) + int64_t(N1) * (j2 + r * TPT2), v[r]);
-  }
-  __syncthreads();  // the local tile may be reused
-  return nxt;
-}
-
-// Shared memory a CTA needs for its part of a long item.
-__host__ __device__ inline size_t cluster_big_smem() {
-  size_t m = 0;
-  for (int lg = 14; lg <= kBigMaxLog2L; ++lg) {
-    const int N1 = (1 << lg) / kN2, R1 = N1 / (kThreads / kColsPerCta);
-    const int K1 = N1 / kCluster, R2 = kN2 / (kThreads / K1);
-    const size_t a = size_t(kColsPerCta) * tile_pitch(N1, R1, kColsPerCta, 1) * sizeof(cpx);
-    const size_t b = size_t(K1) * tile_pitch(kN2, R2, K1, 1) * sizeof(cpx);
-    m = m > a ? m : a;
-    m = m > b ? m : b;
-  }
-  return kOffsetsBytes + 16 * ((m + 15) / 16);
-}
-
-// The persistent kernel in cluster form: long items first, each on a whole
-// cluster (cluster rank 0 takes the next one from counter[1] and the others
-// read its index through distributed shared memory), then every CTA takes
-// short items from counter[0] on its own.
-__global__ void __launch_bounds__(kThreads, MinBlocks<16>::value) mixed_cluster_kernel(const __grid_constant__ Params mp) {
-  namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_item;
-  __shared__ int s_next[2];  // cluster rank 0: the cluster's next long item, by item parity
-  cg::cluster_group cl = cg::this_cluster();
-  const bool lead = cl.block_rank() == 0 && threadIdx.x == 0;
-  if (lead) s_next[0] = int(atomicAdd(mp.counter + 1, 1u));
-  cl.sync();
-  int idx = *cl.map_shared_rank(&s_next[0], 0);
-  for (int n = 0; idx < mp.nbig; ++n) {
-    // the index after this one, read by the cluster after this item's first
-    // barrier (the slot it replaces was read during the previous item)
-    if (lead) s_next[(n + 1) & 1] = int(atomicAdd(mp.counter + 1, 1u));
-    const Item it = mp.items[idx];
-    switch (it.log2L) {
-      case 14: idx = run_cluster_big<14>(mp, it, smem, &s_next[(n + 1) & 1]); break;
-      case 15: idx = run_cluster_big<15>(mp, it, smem, &s_next[(n + 1) & 1]); break;
-      default: idx = run_cluster_big<16>(mp, it, smem, &s_next[(n + 1) & 1]); break;
-    }
-  }
-  cl.sync();  // rank 0's slot has been read by all before anyone moves on
-  for (;;) {
-    if (threadIdx.x == 0) s_item = mp.nbig + int(atomicAdd(mp.counter, 1u));
-    __syncthreads();
-    const int idx = s_item;
-    __syncthreads();
-    if (idx >= mp.nitems) break;
-    const Item it = mp.items[idx];
-    if (it.combo < 0) {
-      run_unit(mp, it);
-    } else {
-      switch (it.combo) {
-        case K_CPLX: run_small_any<LoadCplx, StoreCplx>(mp, it, smem); break;
-        case K_R2C: run_small_any<LoadR2C, StoreR2C>(mp, it, smem); break;
-        case K_C2R: run_small_any<LoadC2R, StoreC2R>(mp, it, smem); break;
-        case K_DCT2: run_small_any<LoadDCT2, StoreDCT2>(mp, it, smem); break;
-        case K_DCT3: run_small_any<LoadDCT3, StoreDCT3>(mp, it, smem); break;
-        default: run_small_any<LoadT4, StoreT4>(mp, it, smem); break;
-      }
-    }
-    __syncthreads();
-  }
-  cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // shared memory of the kernel: offsets + the largest tile of any item
@@ -734,7 +460,7 @@ size_t kernel_smem() {
     const int cpb = small_cpb(L);
     m = std::max(m, size_t(cpb) * tile_pitch(L, small_radix(L), cpb, 0) * sizeof(cpx));
   }
-  for (int rp : {64, 128, 256}) {
+  for (int rp : {64, 128, 256}) {  // long items' tiles
     const int cpb = kThreads / (rp / 16);
     m = std::max(m, size_t(cpb) * tile_pitch(rp, 16, cpb, 1) * sizeof(cpx));
   }
@@ -753,20 +479,21 @@ struct minfft_b200_mixed {
   int device = 0;
   int count = 0;
   std::vector<Job> jobs;
-  std::vector<int> order;
   std::vector<Item> items;
   Params params;
   void* d_jobs = nullptr;
-  void* d_order = nullptr;
   void* d_items = nullptr;
   unsigned* d_counter = nullptr;
+  size_t counter_bytes = 0;
   cpx* d_scratch = nullptr;
+  int* h_status = nullptr;  // host-mapped: set by a kernel whose bounded wait ran out
+  int64_t slot_base[kSlots] = {};  // scratch of each long length (complex elements)
+  int slots[kSlots] = {};
   std::vector<void*> tables;
   int grid = 0;
   int per_sm = 1;
   size_t smem = 0;
   int split = 1;  // jobs per short item = slots / split
-  bool cluster = false;  // long items on clusters (mixed_cluster_kernel)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -831,9 +558,9 @@ void release_graph(minfft_b200_mixed* m) {
 }
 
 // Cut the job groups into items (short groups: slots/split jobs per item),
-// order them by cost, upload, and capture counter reset + kernel in a graph.
+// order them, upload, and capture counter reset + kernel in a graph.
 bool build_items(minfft_b200_mixed* m) {
-  std::map<std::tuple<int, int, int, int>, std::vector<int>> groups;  // (big, combo, flags, log2L) -> jobs
+  std::map<std::tuple<int, int, int, int>, std::vector<int>> groups;  // (long, combo, flags, log2L) -> jobs
   for (int i = 0; i < m->count; ++i) {
     const Job& j = m->jobs[i];
     const int combo = combo_of(j.op);
@@ -845,81 +572,126 @@ bool build_items(minfft_b200_mixed* m) {
     const int lgL = combo == mb::K_CPLX ? j.log2n : j.log2n - 1;
     groups[std::make_tuple(lgL > kSmallMaxLog2L ? 1 : 0, combo, flags_of(j.op), lgL)].push_back(i);
   }
-  std::vector<std::pair<double, Item>> its;
-  m->order.clear();
+  std::vector<std::pair<double, Item>> its;  // short items by cost
+  std::vector<Item> longs;                   // one prototype per long transform
+  std::vector<Job> order;
   for (auto& g : groups) {
-    const int big = std::get<0>(g.first), combo = std::get<1>(g.first), flags = std::get<2>(g.first),
-              lgL = std::get<3>(g.first);
+    const int combo = std::get<1>(g.first), flags = std::get<2>(g.first), lgL = std::get<3>(g.first);
     const std::vector<int>& js = g.second;
+    Item it{};
+    it.combo = combo;
+    it.log2L = lgL;
+    it.flags = flags;
+    it.dep = -1;
+    if (std::get<0>(g.first)) {
+      for (int i : js) {
+        const Job& j = m->jobs[i];
+        Item l = it;
+        l.op = j.op;
+        l.in = j.in;
+        l.out = j.out;
+        // rows read or written as complex pairs: an unaligned one by scalars
+        const void* row = combo == mb::K_C2R ? j.out : j.in;
+        if (reinterpret_cast<uintptr_t>(row) % sizeof(cpx) == 0) l.flags |= mb::F_VEC;
+        // the inverse real DFT's chain ends conjugated, as the complex inverse's does
+        if (combo == mb::K_C2R) l.flags |= mb::F_CONJ_OUT;
+        longs.push_back(l);
+      }
+      continue;
+    }
     const int L = 1 << lgL;
-    int per = big ? 1 : (combo < 0 ? kThreads : std::max(1, small_cpb(L) / m->split));
+    const int per = combo < 0 ? kThreads : std::max(1, small_cpb(L) / m->split);
     for (size_t s = 0; s < js.size(); s += per) {
-      Item it{};
-      it.combo = combo;
-      it.log2L = lgL;
-      it.flags = flags;
+      it.kind = combo < 0 ? kUnit : kShort;
       it.count = int(std::min<size_t>(per, js.size() - s));
-      it.first = int(m->order.size());
-      it.big = big;
+      it.first = int(order.size());
       it.op = m->jobs[js[s]].op;
-      for (int k = 0; k < it.count; ++k) m->order.push_back(js[s + k]);
-      // cost: points processed (x2 passes and pre/post for the long ones)
-      const double cost = double(L) * std::max(1, lgL) * (big ? 3.0 : 1.0) * (big ? 1 : it.count);
-      its.push_back(std::make_pair(cost, it));
+      for (int k = 0; k < it.count; ++k) order.push_back(m->jobs[js[s + k]]);
+      its.push_back(std::make_pair(double(L) * std::max(1, lgL) * it.count, it));  // cost: points processed
     }
   }
   std::stable_sort(its.begin(), its.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-  // long items first (the cluster form takes them from their own queue)
-  std::stable_partition(its.begin(), its.end(), [](const auto& a) { return a.second.big != 0; });
+  std::stable_sort(longs.begin(), longs.end(), [](const Item& a, const Item& b) { return a.log2L > b.log2L; });
+  // The list: first-pass tiles until the oldest transform's are `lag` items
+  // back (or its length's slots are used up), then that transform's
+  // last-pass tiles; short items fill the lag once the long ones run out,
+  // and the rest follow, largest first.
   m->items.clear();
-  int nbig = 0;
-  for (auto& p : its) {
-    m->items.push_back(p.second);
-    nbig += p.second.big ? 1 : 0;
+  const size_t lag = size_t(m->grid) + size_t(m->grid) / 2;
+  struct Open {
+    int id;
+    size_t end;  // list position after its first-pass tiles
+  };
+  std::deque<Open> open;
+  std::map<int, std::vector<int>> users;  // log2L -> transforms in slot order
+  std::map<int, int> live;                // log2L -> slots in use by open transforms
+  size_t next = 0, nshort = 0;
+  auto emit = [&](int id, int kind) {
+    const int tiles = (1 << longs[id].log2L) / kTilePoints;
+    for (int t = 0; t < tiles; ++t) {
+      Item it = longs[id];
+      it.kind = kind;
+      it.tile = t;
+      it.id = id;
+      if (kind == kLast) it.dep = -1;
+      m->items.push_back(it);
+    }
+  };
+  while (next < longs.size() || !open.empty()) {
+    const bool old = !open.empty() && m->items.size() - open.front().end >= lag;
+    if (next < longs.size() && !old && live[longs[next].log2L] < m->slots[longs[next].log2L]) {
+      Item& l = longs[next];
+      std::vector<int>& u = users[l.log2L];
+      const int S = m->slots[l.log2L], k = int(u.size());
+      l.scratch = m->slot_base[l.log2L] + int64_t(k % S) * (int64_t(1) << l.log2L);
+      l.dep = k >= S ? u[k - S] : -1;
+      u.push_back(int(next));
+      ++live[l.log2L];
+      emit(int(next), kFirst);
+      open.push_back(Open{int(next), m->items.size()});
+      ++next;
+    } else if (!old && next == longs.size() && nshort < its.size()) {
+      m->items.push_back(its[nshort++].second);
+    } else {
+      emit(open.front().id, kLast);
+      --live[longs[open.front().id].log2L];
+      open.pop_front();
+    }
   }
-  if (m->d_order) cudaFree(m->d_order);
+  while (nshort < its.size()) m->items.push_back(its[nshort++].second);
+  const int nbig = int(longs.size());
+
+  if (m->d_jobs) cudaFree(m->d_jobs);
   if (m->d_items) cudaFree(m->d_items);
-  m->d_order = m->d_items = nullptr;
-  if (!ok(mb::dev_malloc(&m->d_order, std::max<size_t>(1, m->order.size()) * sizeof(int)), "cudaMalloc(order)") ||
-      !ok(mb::dev_malloc(&m->d_items, std::max<size_t>(1, m->items.size()) * sizeof(Item)), "cudaMalloc(items)"))
+  if (m->d_counter) cudaFree(m->d_counter);
+  m->d_jobs = m->d_items = nullptr;
+  m->d_counter = nullptr;
+  m->counter_bytes = (1 + 2 * size_t(nbig)) * sizeof(unsigned);
+  if (!ok(mb::dev_malloc(&m->d_jobs, std::max<size_t>(1, order.size()) * sizeof(Job)), "cudaMalloc(jobs)") ||
+      !ok(mb::dev_malloc(&m->d_items, std::max<size_t>(1, m->items.size()) * sizeof(Item)), "cudaMalloc(items)") ||
+      !ok(mb::dev_malloc(&m->d_counter, m->counter_bytes), "cudaMalloc(counter)"))
     return false;
-  if (!m->order.empty() &&
-      !ok(cudaMemcpy(m->d_order, m->order.data(), m->order.size() * sizeof(int), cudaMemcpyHostToDevice),
-          "cudaMemcpy(order)"))
+  if (!order.empty() && !ok(cudaMemcpy(m->d_jobs, order.data(), order.size() * sizeof(Job), cudaMemcpyHostToDevice),
+                            "cudaMemcpy(jobs)"))
     return false;
   if (!m->items.empty() &&
       !ok(cudaMemcpy(m->d_items, m->items.data(), m->items.size() * sizeof(Item), cudaMemcpyHostToDevice),
           "cudaMemcpy(items)"))
     return false;
-  m->params.order = static_cast<const int*>(m->d_order);
+  m->params.jobs = static_cast<const Job*>(m->d_jobs);
   m->params.items = static_cast<const Item*>(m->d_items);
   m->params.nitems = int(m->items.size());
-  m->params.nbig = m->cluster ? nbig : 0;
-  // graph: reset the queue counter, run the persistent kernel
+  m->params.nbig = nbig;
+  m->params.counter = m->d_counter;
+  // graph: reset the queue and the tile counters, run the persistent kernel
   release_graph(m);
   cudaStream_t cs;
   if (!ok(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
   bool good = ok(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   if (good) {
-    cudaMemsetAsync(m->d_counter, 0, 2 * sizeof(unsigned), cs);
+    cudaMemsetAsync(m->d_counter, 0, m->counter_bytes, cs);
     void* args[1] = {&m->params};
-    if (m->cluster) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(m->grid);
-      cfg.blockDim = dim3(kThreads);
-      cfg.dynamicSmemBytes = m->smem;
-      cfg.stream = cs;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = kCluster;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      cudaLaunchKernelExC(&cfg, (const void*)mixed_cluster_kernel, args);
-    } else {
-      cudaLaunchKernel((const void*)mixed_kernel, dim3(m->grid), dim3(kThreads), args, m->smem, cs);
-    }
+    cudaLaunchKernel((const void*)mixed_kernel, dim3(m->grid), dim3(kThreads), args, m->smem, cs);
     good = ok(cudaStreamEndCapture(cs, &m->graph), "cudaStreamEndCapture");
   }
   if (good) good = ok(cudaGraphInstantiate(&m->exec, m->graph, 0), "cudaGraphInstantiate");
@@ -934,10 +706,10 @@ MB_EXPORT void minfft_b200_mixed_free(minfft_b200_mixed* m) {
   release_graph(m);
   for (void* t : m->tables) cudaFree(t);
   cudaFree(m->d_jobs);
-  cudaFree(m->d_order);
   cudaFree(m->d_items);
   cudaFree(m->d_counter);
   cudaFree(m->d_scratch);
+  if (m->h_status) cudaFreeHost(m->h_status);
   delete m;
 }
 
@@ -953,8 +725,7 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
   }
   m->count = count;
   m->jobs.resize(count);
-  int max_big = 0;
-  std::vector<int> need_tw(kSlots, 0), need_n(kSlots, 0), need_st(kSlots, 0);
+  std::vector<int> need_tw(kSlots, 0), need_st(kSlots, 0), nlong(kSlots, 0);
   std::vector<int> need_kind(kSlots * mb::K_COUNT, 0);
   for (int i = 0; i < count; ++i) {
     const minfft_b200_job& j = jobs[i];
@@ -974,10 +745,11 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
       minfft_b200_mixed_free(m);
       return nullptr;
     }
-    // complex arrays are accessed as aligned pairs; so are the real arrays a
-    // long real DFT reads (or a long inverse writes) as complex values
-    const bool cin = combo == mb::K_CPLX || combo == mb::K_C2R || (combo == mb::K_R2C && lgL > kSmallMaxLog2L);
-    const bool cout = combo == mb::K_CPLX || combo == mb::K_R2C || (combo == mb::K_C2R && lgL > kSmallMaxLog2L);
+    // complex arrays are accessed as aligned pairs; real arrays of a real DFT
+    // (or its inverse) of more than 16384 reals are required to be aligned so too
+    const bool pairs = lgL > 13;
+    const bool cin = combo == mb::K_CPLX || combo == mb::K_C2R || (combo == mb::K_R2C && pairs);
+    const bool cout = combo == mb::K_CPLX || combo == mb::K_R2C || (combo == mb::K_C2R && pairs);
     if ((cin && reinterpret_cast<uintptr_t>(j.in) % sizeof(cpx)) ||
         (cout && reinterpret_cast<uintptr_t>(j.out) % sizeof(cpx))) {
       fail(MINFFT_B200_EINVAL, "mixed plan: complex data must be aligned to its size");
@@ -987,15 +759,15 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
     m->jobs[i] = Job{j.in, j.out, j.op, lgn};
     if (n == 1) continue;
     if (lgL > kSmallMaxLog2L) {
-      max_big = std::max(max_big, lgL);
-      need_st[lgL] = 1;
-      need_tw[(lgL + 1) / 2] = 1;  // scratch form: its two passes
-      need_tw[lgL - (lgL + 1) / 2] = 1;
-      need_tw[lgL - ilog2i(kN2)] = 1;  // cluster form: the L/256-point column DFTs
-      need_tw[ilog2i(kN2)] = 1;        // and the 256-point row DFTs
-    } else {
-      need_tw[lgL] = 1;
+      ++nlong[lgL];
+      need_tw[first_bits(lgL)] = need_tw[lgL - first_bits(lgL)] = 1;
+      need_st[lgL] = 1;  // the last pass's pre-twiddle, then the fused steps' roots (run_tile)
+      if (combo == mb::K_R2C || combo == mb::K_C2R) need_st[lgn] = 1;
+      if (combo == mb::K_DCT2 || combo == mb::K_DCT3) need_st[lgn + 2] = 1;
+      if (combo == mb::K_T4) need_st[lgn + 1] = need_st[lgn + 3] = 1;
+      continue;
     }
+    need_tw[lgL] = 1;
     need_kind[combo * kSlots + lgn] = 1;
   }
   if (!ok(cudaGetDevice(&m->device), "cudaGetDevice")) {
@@ -1035,48 +807,22 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
               "occupancy query");
   m->per_sm = std::max(1, occ);
   m->grid = sms * m->per_sm;
-  // long items: the cluster form with MINFFT_B200_MIXED_CLUSTER=1, where the
-  // device can co-schedule clusters of eight CTAs with this shared memory
-  // (measured slower than the per-CTA scratch form on the 20000-job batch,
-  // so not the default)
-  const char* ce = getenv("MINFFT_B200_MIXED_CLUSTER");
-  if (good && max_big > 0 && ce && ce[0] == '1') {
-    const size_t csmem = std::max(kernel_smem(), cluster_big_smem());
-    int nclusters = 0;
-    if (cudaFuncSetAttribute((const void*)mixed_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(csmem)) == cudaSuccess) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(kCluster);
-      cfg.blockDim = dim3(kThreads);
-      cfg.dynamicSmemBytes = csmem;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = kCluster;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&nclusters, (const void*)mixed_cluster_kernel, &cfg) != cudaSuccess)
-        nclusters = 0;
-    }
-    cudaGetLastError();
-    if (nclusters > 0) {
-      m->cluster = true;
-      m->smem = csmem;
-      m->grid = nclusters * kCluster;
-      m->per_sm = std::max(1, m->grid / sms);
-    }
+  // scratch slots of each long length, in kSlotBytes
+  int64_t scratch = 0;
+  for (int lg = kSmallMaxLog2L + 1; lg <= kBigMaxLog2L; ++lg) {
+    const size_t bytes = (size_t(1) << lg) * sizeof(cpx);
+    m->slots[lg] = int(std::min<size_t>(nlong[lg], kSlotBytes / bytes));
+    m->slot_base[lg] = scratch;
+    scratch += int64_t(m->slots[lg]) << lg;
   }
-  if (good) good = ok(mb::dev_malloc(&m->d_jobs, count * sizeof(Job)), "cudaMalloc(jobs)");
+  if (good && scratch > 0) good = ok(mb::dev_malloc(&m->d_scratch, size_t(scratch) * sizeof(cpx)), "cudaMalloc(scratch)");
   if (good)
-    good = ok(cudaMemcpy(m->d_jobs, m->jobs.data(), count * sizeof(Job), cudaMemcpyHostToDevice), "cudaMemcpy(jobs)");
-  if (good) good = ok(mb::dev_malloc(&m->d_counter, 2 * sizeof(unsigned)), "cudaMalloc(counter)");
-  if (good && max_big > 0 && !m->cluster) {
-    P.scratch_stride = int64_t(2) << kBigMaxLog2L;
-    good = ok(mb::dev_malloc(&m->d_scratch, size_t(m->grid) * P.scratch_stride * sizeof(cpx)), "cudaMalloc(scratch)");
+    good = ok(cudaHostAlloc(reinterpret_cast<void**>(&m->h_status), sizeof(int), cudaHostAllocMapped),
+              "cudaHostAlloc(status)");
+  if (good) {
+    *m->h_status = 0;
+    good = ok(cudaHostGetDevicePointer(reinterpret_cast<void**>(&P.status), m->h_status, 0), "status address");
   }
-  P.jobs = static_cast<const Job*>(m->d_jobs);
-  P.counter = m->d_counter;
   P.scratch = m->d_scratch;
   if (good) good = build_items(m);
   if (!good) {
@@ -1088,6 +834,10 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
 
 MB_EXPORT int minfft_b200_mixed_execute(minfft_b200_mixed* m, void* stream) {
   if (!m || !m->exec) return fail(MINFFT_B200_EINVAL, "mixed execute: NULL plan");
+  if (*static_cast<volatile int*>(m->h_status)) {
+    *m->h_status = 0;
+    return fail(MINFFT_B200_ETIMEOUT, "mixed execute: an earlier run gave up waiting for a pass of a long job");
+  }
   return ok(cudaGraphLaunch(m->exec, static_cast<cudaStream_t>(stream)), "cudaGraphLaunch") ? MINFFT_B200_OK
                                                                                              : MINFFT_B200_ECUDA;
 }
@@ -1110,14 +860,9 @@ MB_EXPORT int minfft_b200_mixed_autotune(minfft_b200_mixed* m, int reps) {
   cudaEventCreate(&e1);
   float best = 1e30f;
   int best_split = m->split, best_per = m->per_sm;
-  const int grid_cap = m->grid;  // scratch is sized for this many CTAs
-  // the cluster form keeps every co-resident cluster (its grid is the
-  // occupancy query's cluster count, not a multiple of the SMs)
-  auto grid_for = [&](int per) {
-    return m->cluster ? grid_cap : std::min(grid_cap, sms * per);
-  };
+  auto grid_for = [&](int per) { return sms * per; };
   for (int split : {1, 2, 4, 8}) {
-    for (int per = 1; per <= (m->cluster ? 1 : max_per_sm); ++per) {
+    for (int per = 1; per <= max_per_sm; ++per) {
       m->split = split;
       m->grid = grid_for(per);
       if (!build_items(m)) continue;
