@@ -264,6 +264,27 @@ __device__ __forceinline__ T src_ld(const T* q, bool smem) {
   return smem ? *q : __ldcs(q);
 }
 
+// A pointer that walks a strided run: step() moves it by one stride.  kUnit
+// runs have a compile-time stride, so the compiler folds every position into
+// the access's immediate offset; the others add the stride to the pointer
+// (two integer instructions per access -- indexing by r * stride cost four,
+// 12 of the 52 instructions per point of a 256-point column pass; the asm
+// keeps the compiler from turning the additions back into products).
+template <typename T, bool kUnit, int kStep>
+struct Walk {
+  T* q;
+  int64_t st;  // stride of one element
+  __device__ __forceinline__ Walk(T* base, int64_t stride) : q(base), st(kUnit ? 0 : stride * kStep) {}
+  __device__ __forceinline__ void step() {
+    if constexpr (kUnit) {
+      q += kStep;
+    } else {
+      q += st;
+      asm("" : "+l"(q));
+    }
+  }
+};
+
 // ------------------------------------------------------------- row staging
 // In row mode a transform's real row (N = 2L contiguous reals) is moved
 // between global memory and the transform's tile slot in shared memory by its
@@ -329,8 +350,9 @@ template <int L, int R>
 __device__ __forceinline__ void col_g2s(real* sr, const real* g, int64_t s, int j, bool smem = false) {
   constexpr int TPT = L / R;
   real r[2 * R];
+  Walk<const real, false, TPT> w(g + int64_t(j) * s, s);
 #pragma unroll
-  for (int m = 0; m < 2 * R; ++m) r[m] = src_ld(g + int64_t(j + m * TPT) * s, smem);
+  for (int m = 0; m < 2 * R; ++m, w.step()) r[m] = src_ld(w.q, smem);
 #pragma unroll
   for (int m = 0; m < 2 * R; ++m) sr[j + m * TPT] = r[m];
 }
@@ -436,10 +458,9 @@ struct LoadCplx {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = src_ld(q + r * TPT, (p.flags & F_SRC_SMEM) != 0);
     } else {
-      const cpx* q = in + x.j * p.in_n;
-      const int64_t st = int64_t(TPT) * p.in_n;
+      Walk<const cpx, false, TPT> w(in + x.j * p.in_n, p.in_n);
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = src_ld(q + r * st, (p.flags & F_SRC_SMEM) != 0);
+      for (int r = 0; r < R; ++r, w.step()) v[r] = src_ld(w.q, (p.flags & F_SRC_SMEM) != 0);
     }
     if (p.flags & F_CONJ_IN) {
 #pragma unroll
@@ -479,31 +500,33 @@ struct LoadR2C {
 struct LoadDCT2 {
   static constexpr bool kComplexIn = false;  // whether the raw input elements are complex
   static constexpr bool kStaged = false;
+  // element m = j + r*TPT lies in the first half (m < L/2) exactly when r < R/2:
+  // pair (x[4m], x[4m+2]) there, (x[2N-1-4m], x[2N-3-4m]) (times sg) after
+  template <bool kUnit, int L, int R>
+  static __device__ __forceinline__ void pairs(const real* in, int64_t s, int j, real sg, cpx (&v)[R]) {
+    constexpr int N = 2 * L, TPT = L / R, m0 = (R / 2) * TPT;
+    Walk<const real, kUnit, 4 * TPT> a(in + int64_t(4 * j) * s, s), b(in + int64_t(4 * j + 2) * s, s);
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r, a.step(), b.step()) v[r] = cmk(*a.q, *b.q);
+    Walk<const real, kUnit, -4 * TPT> c(in + int64_t(2 * N - 1 - 4 * (j + m0)) * s, s),
+        d(in + int64_t(2 * N - 3 - 4 * (j + m0)) * s, s);
+#pragma unroll
+    for (int r = R / 2; r < R; ++r, c.step(), d.step()) v[r] = cmk(sg * *c.q, sg * *d.q);
+  }
   template <int L, int R>
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, cpx (&v)[R]) {
     const real* in = static_cast<const real*>(p.in) + x.oin;
     const real sg = (p.flags & F_DST) ? real(-1) : real(1);
-    constexpr int N = 2 * L;
-    constexpr int TPT = L / R;
     if (!x.active) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = czero();
       return;
     }
     if constexpr (L >= 2) {
-      // element m = j + r*TPT lies in the first half (m < L/2) exactly when r < R/2:
-      // pair (x[4m], x[4m+2]) there, (x[2N-1-4m], x[2N-3-4m]) (times sg) after
-      const int64_t s = p.in_n;
-      const real* lo = in + int64_t(4 * x.j) * s;
-      const real* hi = in + int64_t(2 * N - 1 - 4 * x.j) * s;
-      const int64_t st = int64_t(4 * TPT) * s;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (r < R / 2)
-          v[r] = cmk(lo[r * st], lo[r * st + 2 * s]);
-        else
-          v[r] = cmk(sg * hi[-r * st], sg * hi[-r * st - 2 * s]);
-      }
+      if (p.in_n == 1)
+        pairs<true, L, R>(in, 1, x.j, sg, v);
+      else
+        pairs<false, L, R>(in, p.in_n, x.j, sg, v);
     } else {
       v[0] = cmk(in[0], sg * in[p.in_n]);  // L = 1: u = (x0, +-x1)
     }
@@ -520,22 +543,27 @@ struct LoadT4 {
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, cpx (&v)[R]) {
     const real* in = static_cast<const real*>(p.in) + x.oin;
     const bool dst = (p.flags & F_DST) != 0;
-    constexpr int N = 2 * L;
     constexpr int TPT = L / R;
     if (!x.active) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = czero();
       return;
     }
-    const int64_t s = p.in_n;
-    const real* lo = in + int64_t(2 * x.j) * s;
-    const real* hi = in + int64_t(N - 1 - 2 * x.j) * s;
-    const int64_t st = int64_t(2 * TPT) * s;
     const cpx e = kind_base<TPT>(p.t1, x.j);  // w_2N^j; w_2N^(j + r*TPT) = e * w_4R^r
+    if (p.in_n == 1)
+      rotate<true, L, R>(in, 1, x.j, e, dst, v);
+    else
+      rotate<false, L, R>(in, p.in_n, x.j, e, dst, v);
+  }
+  template <bool kUnit, int L, int R>
+  static __device__ __forceinline__ void rotate(const real* in, int64_t s, int j, cpx e, bool dst, cpx (&v)[R]) {
+    constexpr int N = 2 * L, TPT = L / R;
+    Walk<const real, kUnit, 2 * TPT> lo(in + int64_t(2 * j) * s, s);
+    Walk<const real, kUnit, -2 * TPT> hi(in + int64_t(N - 1 - 2 * j) * s, s);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const real a = lo[r * st];
-      const real b = hi[-r * st];
+    for (int r = 0; r < R; ++r, lo.step(), hi.step()) {
+      const real a = *lo.q;
+      const real b = *hi.q;
       const cpx w = cmul(e, w128(r * (32 / R)));
       if (!dst) {
         v[r] = cmul(w, cmk(a, b));
@@ -638,7 +666,7 @@ struct LoadC2R {
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
     const cpx* in = static_cast<const cpx*>(p.in) + x.oin;
     const cpx b2 = kind_base<L / R>(p.t2, x.j);
-    pair_loop<L, R>(x, [&](int k) { return x.active ? in[int64_t(k) * p.in_n] : czero(); },
+    pair_loop<L, R>(x, [&](int k) { return x.active ? in[k] : czero(); },
                     [&](int i, int k, cpx z0, cpx z1) { pack_into(t, x.c, k, L, z0, z1, rft_root<R>(b2, i)); });
     __syncthreads();
     gather_natural<L, R>(v, x.j, x.c, t);
@@ -666,7 +694,7 @@ struct LoadC2RQ {
     const int64_t bs = p.is0;
     // column col of the four blocks -> the four rows' spectra at col
     auto gather4 = [&](int col, cpx (&X)[4]) {
-      const cpx* q = in + int64_t(col) * p.in_n;
+      const cpx* q = in + col;
       const cpx u0 = q[0], u1 = cmul(q[bs], w1), u2 = cmul(q[2 * bs], w2), u3 = cmul(q[3 * bs], w3);
       const cpx a0 = cadd(u0, u2), a1 = csub(u0, u2), c0 = cadd(u1, u3), c1 = csub(u1, u3);
       const cpx ic1 = cmk(-c1.y, c1.x);  // i * c1
@@ -1073,10 +1101,9 @@ struct StoreCplx {
 #pragma unroll
         for (int r = 0; r < R; ++r) q[r * TPT] = v[r];
       } else {
-        cpx* q = out + x.oout + x.j * p.out_k;
-        const int64_t st = int64_t(TPT) * p.out_k;
+        Walk<cpx, false, TPT> w(out + x.oout + x.j * p.out_k, p.out_k);
 #pragma unroll
-        for (int r = 0; r < R; ++r) q[r * st] = v[r];
+        for (int r = 0; r < R; ++r, w.step()) *w.q = v[r];
       }
       return;
     }
@@ -1109,14 +1136,14 @@ struct StoreR2C {
     pair_loop<L, R>(x, [&](int k) { return t.s[t.idx(x.c, k & (L - 1))]; }, [&](int i, int k, cpx za, cpx zb) {
       if (k == 0) {
         out[0] = cmk(za.x + za.y, real(0));
-        out[int64_t(L) * p.out_k] = cmk(za.x - za.y, real(0));
+        out[L] = cmk(za.x - za.y, real(0));
       } else if (2 * k == L) {
-        out[int64_t(k) * p.out_k] = cconj(za);
+        out[k] = cconj(za);
       } else {
         cpx xa, xb;
         unpack_pair(za, zb, rft_root<R>(b1, i), xa, xb);
-        out[int64_t(k) * p.out_k] = xa;
-        out[int64_t(L - k) * p.out_k] = xb;
+        out[k] = xa;
+        out[L - k] = xb;
       }
     });
   }
@@ -1155,24 +1182,43 @@ struct StoreDCT2 {
     __syncthreads();
     if (!x.active) return;
     real* out = static_cast<real*>(p.out) + x.oout;
+    if (p.out_k == 1)
+      rotate<true, L, R>(p, out, 1, x, t);
+    else
+      rotate<false, L, R>(p, out, p.out_k, x, t);
+  }
+  // The four outputs of the pair (k, L-k), k = j + i*TPT: positions k, N-k,
+  // L-k and L+k (one less for DST-2, which swaps each two of one value).
+  template <bool kUnit, int L, int R>
+  static __device__ __forceinline__ void rotate(const AxisParams& p, real* out, int64_t s, const Ctx& x,
+                                                const Tile& t) {
+    constexpr int N = 2 * L, TPT = L / R;
     const bool dst = (p.flags & F_DST) != 0;
-    constexpr int N = 2 * L;
+    if (dst) out -= s;
     const real r2 = real(1.414213562373095048801688724209698079);
-    const cpx b1 = kind_base<L / R>(p.t1, x.j), b2 = kind_base<L / R>(p.t2, x.j);
+    const cpx b1 = kind_base<TPT>(p.t1, x.j), b2 = kind_base<TPT>(p.t2, x.j);
+    Walk<real, kUnit, TPT> lo(out + int64_t(x.j) * s, s), up(out + int64_t(L + x.j) * s, s);
+    Walk<real, kUnit, -TPT> hi(out + int64_t(N - x.j) * s, s), dn(out + int64_t(L - x.j) * s, s);
+    auto put = [&](real* a, real* b, cpx q) {  // y_n = Re, y_(N-n) = -Im
+      *a = dst ? -q.y : q.x;
+      *b = dst ? q.x : -q.y;
+    };
     pair_loop<L, R>(x, [&](int k) { return t.s[t.idx(x.c, k & (L - 1))]; }, [&](int i, int k, cpx za, cpx zb) {
       if (k == 0) {
         const real v0 = za.x + za.y, vl = za.x - za.y;
-        out[int64_t(dst ? N - 1 : 0) * p.out_k] = 2 * v0;
-        out[int64_t(dst ? L - 1 : L) * p.out_k] = r2 * vl;
+        *(dst ? hi.q : lo.q) = 2 * v0;
+        *up.q = r2 * vl;
       } else if (2 * k == L) {
-        emit(out, p.out_k, k, N, dst, cconj(za), w128(8));  // w_4N^(L/2) = w_16
+        const cpx q = cmul(cconj(za), w128(8));  // w_4N^(L/2) = w_16
+        put(lo.q, hi.q, cmk(2 * q.x, 2 * q.y));
       } else {
         cpx xa2, xb2;
         unpack_pair2(za, zb, rft_root<R>(b2, i), xa2, xb2);
         const cpx e = t23_root<R>(b1, i);  // w_4N^k
-        emit2(out, p.out_k, k, N, dst, xa2, e);
-        emit2(out, p.out_k, L - k, N, dst, xb2, t23_mirror(e));
+        put(lo.q, hi.q, cmul(xa2, e));
+        put(dn.q, up.q, cmul(xb2, t23_mirror(e)));
       }
+      lo.step(), up.step(), hi.step(), dn.step();
     });
   }
 };
@@ -1207,7 +1253,7 @@ struct StoreR2CQ {
     auto emit = [&](int col, const cpx (&X)[4]) {
       const cpx a0 = cadd(X[0], X[2]), a1 = csub(X[0], X[2]), c0 = cadd(X[1], X[3]), c1 = csub(X[1], X[3]);
       const cpx mic1 = cmk(c1.y, -c1.x);  // -i * c1
-      cpx* q = out + int64_t(col) * p.out_k;
+      cpx* q = out + col;
       q[0] = cadd(a0, c0);
       q[bs] = cmul(cadd(a1, mic1), w1);
       q[2 * bs] = cmul(csub(a0, c0), w2);
@@ -1269,6 +1315,26 @@ struct StoreC2R {
 // DFT's reals t_i go to y[2i] (i < N/2) and y[2N-1-2i] (i >= N/2, negated
 // for DST-3).
 struct StoreDCT3 {
+  // reals t_2m, t_2m+1 (m = j + r*TPT) go to y[4m], y[4m+2] while r < R/2,
+  // else to y[2N-1-4m], y[2N-3-4m] (negated for DST-3)
+  template <bool kUnit, int L, int R>
+  static __device__ __forceinline__ void spread(real* out, int64_t s, int j, bool dst, const cpx (&v)[R]) {
+    constexpr int N = 2 * L, TPT = L / R, m0 = (R / 2) * TPT;
+    const real sg = dst ? real(-1) : real(1);
+    Walk<real, kUnit, 4 * TPT> a(out + int64_t(4 * j) * s, s), b(out + int64_t(4 * j + 2) * s, s);
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r, a.step(), b.step()) {
+      *a.q = v[r].x;
+      *b.q = -v[r].y;
+    }
+    Walk<real, kUnit, -4 * TPT> c(out + int64_t(2 * N - 1 - 4 * (j + m0)) * s, s),
+        d(out + int64_t(2 * N - 3 - 4 * (j + m0)) * s, s);
+#pragma unroll
+    for (int r = R / 2; r < R; ++r, c.step(), d.step()) {
+      *c.q = sg * v[r].x;
+      *d.q = sg * -v[r].y;
+    }
+  }
   template <int L, int R>
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets&,
                                              cpx (&v)[R]) {
@@ -1285,27 +1351,12 @@ struct StoreDCT3 {
       }
     }
     const bool dst = (p.flags & F_DST) != 0;
-    constexpr int N = 2 * L;
-    constexpr int TPT = L / R;
     if constexpr (L >= 2) {
-      // reals t_2m, t_2m+1 (m = j + r*TPT) go to y[4m], y[4m+2] while r < R/2,
-      // else to y[2N-1-4m], y[2N-3-4m] (negated for DST-3)
-      const real sg = dst ? real(-1) : real(1);
       if (x.active) {
-        real* lo = out + int64_t(4 * x.j) * s;
-        real* hi = out + int64_t(2 * N - 1 - 4 * x.j) * s;
-        const int64_t st = int64_t(4 * TPT) * s;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const cpx w = cconj(v[r]);
-          if (r < R / 2) {
-            lo[r * st] = w.x;
-            lo[r * st + 2 * s] = w.y;
-          } else {
-            hi[-r * st] = sg * w.x;
-            hi[-r * st - 2 * s] = sg * w.y;
-          }
-        }
+        if (s == 1)
+          spread<true, L, R>(out, 1, x.j, dst, v);
+        else
+          spread<false, L, R>(out, s, x.j, dst, v);
       }
       if (staged) {
         __syncthreads();
@@ -1330,23 +1381,28 @@ struct StoreT4 {
     if (!x.active) return;
     real* out = static_cast<real*>(p.out) + x.oout;
     const bool dst = (p.flags & F_DST) != 0;
-    constexpr int N = 2 * L;
-    constexpr int TPT = L / R;
-    const int64_t s = p.out_k;
-    real* lo = out + int64_t(2 * x.j) * s;
-    real* hi = out + int64_t(N - 1 - 2 * x.j) * s;
-    const int64_t st = int64_t(2 * TPT) * s;
+    if (p.out_k == 1)
+      rotate<true, L, R>(p, out, 1, x.j, dst, v);
+    else
+      rotate<false, L, R>(p, out, p.out_k, x.j, dst, v);
+  }
+  template <bool kUnit, int L, int R>
+  static __device__ __forceinline__ void rotate(const AxisParams& p, real* out, int64_t s, int j, bool dst,
+                                                cpx (&v)[R]) {
+    constexpr int N = 2 * L, TPT = L / R;
+    Walk<real, kUnit, 2 * TPT> lo(out + int64_t(2 * j) * s, s);
+    Walk<real, kUnit, -2 * TPT> hi(out + int64_t(N - 1 - 2 * j) * s, s);
     // t2[q] = w_8N^(2q+1): t2[2m] = t2[2j] * w_4R^r and t2[N-1-2m] =
     // t2[N-1-2j] * conj(w_4R^r) for m = j + r*TPT
-    const cpx glo = ldg(p.t2 + 2 * x.j);
-    const cpx ghi = ldg(p.t2 + (N - 1 - 2 * x.j));
+    const cpx glo = ldg(p.t2 + 2 * j);
+    const cpx ghi = ldg(p.t2 + (N - 1 - 2 * j));
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < R; ++r, lo.step(), hi.step()) {
       const cpx T = v[r];
       const cpx a = cmul(cmul(glo, w128(r * (32 / R))), T);
       const cpx b = cmul(cmulc(ghi, w128(r * (32 / R))), cconj(T));
-      lo[r * st] = 2 * (dst ? a.y : a.x);
-      hi[-r * st] = 2 * (dst ? b.y : b.x);
+      *lo.q = 2 * (dst ? a.y : a.x);
+      *hi.q = 2 * (dst ? b.y : b.x);
     }
   }
 };

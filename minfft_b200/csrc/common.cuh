@@ -30,8 +30,33 @@ __device__ __forceinline__ cpx cmk(real re, real im) {
   c.y = im;
   return c;
 }
+#if MINFFT_SINGLE
+// A complex sum or difference in single precision as one packed instruction
+// on the register pair (each half rounded as the scalar form rounds it).
+__device__ __forceinline__ unsigned long long cpack(cpx a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ cpx cunpack(unsigned long long a) {
+  cpx r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ cpx cadd(cpx a, cpx b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(cpack(a)), "l"(cpack(b)));
+  return cunpack(r);
+}
+__device__ __forceinline__ cpx csub(cpx a, cpx b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(cpack(a)), "l"(cpack(b)));
+  return cunpack(r);
+}
+#else
 __device__ __forceinline__ cpx cadd(cpx a, cpx b) { return cmk(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ cpx csub(cpx a, cpx b) { return cmk(a.x - b.x, a.y - b.y); }
+#endif
 __device__ __forceinline__ cpx cmul(cpx a, cpx b) { return cmk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 // a * conj(b)
 __device__ __forceinline__ cpx cmulc(cpx a, cpx b) { return cmk(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y); }
@@ -103,7 +128,10 @@ template <int H, int P, int K>
 __device__ __forceinline__ void bfly2(cpx* v) {
   cpx a = v[P], b = v[P + H];
   v[P] = cadd(a, b);
-  v[P + H] = twc<2 * H, K>(csub(a, b));
+  if constexpr (4 * K == 2 * H)
+    v[P + H] = cmk(a.y - b.y, b.x - a.x);  // times -i
+  else
+    v[P + H] = twc<2 * H, K>(csub(a, b));
 }
 
 template <int H, int... I>
