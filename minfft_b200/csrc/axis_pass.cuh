@@ -558,19 +558,15 @@ struct LoadT4 {
   template <bool kUnit, int L, int R>
   static __device__ __forceinline__ void rotate(const real* in, int64_t s, int j, cpx e, bool dst, cpx (&v)[R]) {
     constexpr int N = 2 * L, TPT = L / R;
+    const real sg = dst ? real(-1) : real(1);
     Walk<const real, kUnit, 2 * TPT> lo(in + int64_t(2 * j) * s, s);
     Walk<const real, kUnit, -2 * TPT> hi(in + int64_t(N - 1 - 2 * j) * s, s);
 #pragma unroll
     for (int r = 0; r < R; ++r, lo.step(), hi.step()) {
-      const real a = *lo.q;
+      // DST: -(a - ib) = -a + ib
+      const real a = sg * *lo.q;
       const real b = *hi.q;
-      const cpx w = cmul(e, w128(r * (32 / R)));
-      if (!dst) {
-        v[r] = cmul(w, cmk(a, b));
-      } else {
-        const cpx q = cmul(w, cmk(a, -b));
-        v[r] = cmk(-q.x, -q.y);
-      }
+      v[r] = cmul(cmul(e, w128(r * (32 / R))), cmk(a, b));
     }
   }
 };
@@ -610,19 +606,53 @@ __device__ __forceinline__ void unpack_pair2(cpx za, cpx zb, cpx f, cpx& xa, cpx
   xb = cconj(csub(u, vv));
 }
 
+// One value of the packing step (pack_pair) for the spectrum pair (z, zm) of
+// points k and L-k: the conjugated inverse-DFT input at k,
+// conj(z + conj(zm) + (z - conj(zm)) i conj(f)); f = w_N^k.
+__device__ __forceinline__ cpx pack_one(cpx z, cpx zm, cpx f) {
+  const real a = z.x + zm.x, b = z.y - zm.y, p = z.x - zm.x, q = z.y + zm.y;
+  return cmk(a + (p * f.y - q * f.x), -(b + (p * f.x + q * f.y)));
+}
+// One value of the unpacking step (unpack_pair2): 2 X_k from Z_k, Z_(L-k),
+// z + conj(zm) + (z - conj(zm)) f/i.
+__device__ __forceinline__ cpx unpack_one2(cpx z, cpx zm, cpx f) {
+  const real a = z.x + zm.x, b = z.y - zm.y, p = z.x - zm.x, q = z.y + zm.y;
+  return cmk(a + (p * f.y + q * f.x), b + (q * f.y - p * f.x));
+}
+
+// The same pairs' values at L-k (f = w_N^k as above): from the sums of
+// pack_one and unpack_one2 with the other signs.
+__device__ __forceinline__ cpx pack_mirror(cpx z, cpx zm, cpx f) {
+  const real a = z.x + zm.x, b = z.y - zm.y, p = z.x - zm.x, q = z.y + zm.y;
+  return cmk(a - (p * f.y - q * f.x), b - (p * f.x + q * f.y));
+}
+__device__ __forceinline__ cpx unpack_mirror2(cpx z, cpx zm, cpx f) {
+  const real a = z.x + zm.x, b = z.y - zm.y, p = z.x - zm.x, q = z.y + zm.y;
+  return cmk(a - (p * f.y + q * f.x), (q * f.y - p * f.x) - b);
+}
+
 // Visits the spectrum pairs (k, L-k), k = 0 .. L/2, owned by thread j of a
 // transform: k = j + i*TPT for i = 0 .. R/2 (only j = 0 reaches k = L/2).
-// zf(k) reads a spectrum value -- for k = 0 also zf(L), which readers of an
-// L-element tile must fold back into range; body(i, k, z_k, z_{L-k})
-// consumes the pair.
-template <int L, int R, class Zf, class Body>
-__device__ __forceinline__ void pair_loop(const Ctx& x, const Zf& zf, const Body& body) {
+// ends(i, k) handles k = 0 and k = L/2, the self-paired ends; body(i, k) the
+// pairs inside.  i is a compile-time constant once unrolled, so only i = 0
+// and i = R/2 test for an end; step() runs after each.
+template <int L, int R, class Ends, class Body, class Step>
+__device__ __forceinline__ void pair_loop(const Ctx& x, const Ends& ends, const Body& body, const Step& step) {
   constexpr int TPT = L / R;
 #pragma unroll
   for (int i = 0; i <= R / 2; ++i) {
     const int k = x.j + i * TPT;
-    if (i == R / 2 && x.j != 0) break;
-    body(i, k, zf(k), zf(L - k));
+    if (i == R / 2) {
+      if (x.j == 0) ends(i, k);
+    } else if (i == 0) {
+      if (x.j == 0)
+        ends(i, k);
+      else
+        body(i, k);
+    } else {
+      body(i, k);
+    }
+    step();
   }
 }
 
@@ -656,6 +686,31 @@ __device__ __forceinline__ void pack_into(const Tile& t, int c, int k, int L, cp
   }
 }
 
+// Tile addresses of the pairs (k, L-k), k = j + i*TPT, of thread j: element k
+// is at lo + nat_off(i), element L-k at hi + nat_off(R-1-i) (thread TPT-j's
+// element; for j = 0 that is thread 0's element R-i, see at()).
+template <int L, int R>
+struct PairSlots {
+  static constexpr int TPT = L / R;
+  cpx *lo, *hi;
+  bool first;  // j = 0
+  __device__ __forceinline__ PairSlots(const Tile& t, int c, int j) : first(j == 0) {
+    cpx* s = t.s + c * t.lp;
+    if constexpr (TPT >= 16) {  // offsets linear in i: thread 0's shift goes into the base
+      lo = s + pad16(j);
+      hi = s + (j == 0 ? nat_off<TPT>(1) : pad16(TPT - j));
+    } else {
+      lo = s + j;
+      hi = s + (j == 0 ? 0 : TPT - j);
+    }
+  }
+  __device__ __forceinline__ cpx& at(int i) const { return lo[nat_off<TPT>(i)]; }
+  // element L-k, 0 < k (thread 0's pairs lie one element further)
+  __device__ __forceinline__ cpx& mirror(int i) const {
+    return hi[TPT < 16 && first ? nat_off<TPT>((R - i) % R) : nat_off<TPT>(R - 1 - i)];
+  }
+};
+
 // Inverse real DFT input: spectrum X_k, k = 0..L, packed into L complex
 // values, staged in shared memory.  Stored conjugated: the inverse DFT is
 // computed as conj(DFT(conj(t))).  t2 = w_N^k, k < L/2.
@@ -666,8 +721,25 @@ struct LoadC2R {
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
     const cpx* in = static_cast<const cpx*>(p.in) + x.oin;
     const cpx b2 = kind_base<L / R>(p.t2, x.j);
-    pair_loop<L, R>(x, [&](int k) { return x.active ? in[k] : czero(); },
-                    [&](int i, int k, cpx z0, cpx z1) { pack_into(t, x.c, k, L, z0, z1, rft_root<R>(b2, i)); });
+    const PairSlots<L, R> at(t, x.c, x.j);
+    auto z = [&](int k) { return x.active ? in[k] : czero(); };
+    pair_loop<L, R>(
+        x,
+        [&](int i, int k) {
+          const cpx z0 = z(k);
+          if (k == 0) {
+            const cpx zl = z(L);
+            at.at(0) = cmk(z0.x + zl.x, -(z0.x - zl.x));
+          } else {
+            at.at(i) = cmk(2 * z0.x, 2 * z0.y);
+          }
+        },
+        [&](int i, int k) {
+          const cpx za = z(k), zb = z(L - k), f = rft_root<R>(b2, i);
+          at.at(i) = pack_one(za, zb, f);
+          at.mirror(i) = pack_mirror(za, zb, f);
+        },
+        [] {});
     __syncthreads();
     gather_natural<L, R>(v, x.j, x.c, t);
   }
@@ -766,21 +838,40 @@ struct LoadDCT3 {
             row_g2s<L, R>(sr, in, x.j, (p.flags & F_SRC_SMEM) != 0);
         }
         __syncthreads();
-        constexpr int NP = R / 2 + 1;
+        // positions of the reals of z_k and z_(L-k): DCT-3 (k, N-k) and
+        // (L-k, L+k), DST-3 (N-1-k, k-1) and (L-1+k, L-k-1), walked by i
+        constexpr int N = 2 * L, NP = R / 2 + 1;
+        const int sa = dst ? -TPT : TPT;
+        const real* pa = sr + (dst ? N - 1 - x.j : x.j);
+        const real* pb = sr + (dst ? x.j - 1 : N - x.j);
+        const real* pc = sr + (dst ? L - 1 + x.j : L - x.j);
+        const real* pd = sr + (dst ? L - 1 - x.j : L + x.j);
+        const real r2 = real(1.414213562373095048801688724209698079);
         cpx za[NP], zb[NP];
-        auto rd = [&](int m) { return sr[m]; };
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-          const int k = x.j + i * TPT;
-          const bool own = x.active && (i < R / 2 || x.j == 0);
           const cpx rk = t23_root<R>(b1, i);  // w_4N^k
-          za[i] = own ? zval_w(rd, k, L, dst, [&](int) { return rk; }) : czero();
-          zb[i] = own ? zval_w(rd, L - k, L, dst, [&](int) { return t23_mirror(rk); }) : czero();
+          if (i == 0 && x.j == 0) {
+            za[0] = cmk(*pa, real(0));
+            zb[0] = cmk(r2 * *pc, real(0));
+          } else if (i < R / 2 || x.j == 0) {
+            za[i] = cconj(cmul(cmk(pa[i * sa], pb[-i * sa]), rk));
+            if (i < R / 2) zb[i] = cconj(cmul(cmk(pc[-i * sa], pd[i * sa]), t23_mirror(rk)));
+          }
         }
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < NP; ++i)
-          if (i < R / 2 || x.j == 0) pack_into(t, x.c, x.j + i * TPT, L, za[i], zb[i], rft_root<R>(b2, i));
+        const PairSlots<L, R> at(t, x.c, x.j);
+        pair_loop<L, R>(
+            x,
+            [&](int i, int k) {
+              at.at(i) = k == 0 ? cmk(za[0].x + zb[0].x, -(za[0].x - zb[0].x)) : cmk(2 * za[i].x, 2 * za[i].y);
+            },
+            [&](int i, int) {
+              const cpx f = rft_root<R>(b2, i);
+              at.at(i) = pack_one(za[i], zb[i], f);
+              at.mirror(i) = pack_mirror(za[i], zb[i], f);
+            },
+            [] {});
         __syncthreads();
         gather_natural<L, R>(v, x.j, x.c, t);
         return;
@@ -831,39 +922,31 @@ struct LoadT4Chain {
     const int pc = x.c < h ? x.c + h : x.c - h;  // the mirror sub-DFT's slot
     real* sb = reinterpret_cast<real*>(t.s);
     const bool vec = (reinterpret_cast<uintptr_t>(in) % sizeof(cpx)) == 0;
+    const real sg = dst ? real(-1) : real(1);
     real a[R];
+    Walk<const real, false, TPT> w(in + 2 * (b1 * p.is1 + int64_t(x.j) * p.in_n), 2 * p.in_n);
+    real* put = sb + pc * 2 * t.lp + (L - 1 - x.j);
+    const real* get = sb + x.c * 2 * t.lp + x.j;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int n = x.j + r * TPT;
-      const int64_t g = b1 * p.is1 + int64_t(n) * p.in_n;
+    for (int r = 0; r < R; ++r, w.step()) {
       real lo, hi;
       if (vec) {
-        const cpx q = __ldcs(reinterpret_cast<const cpx*>(in + 2 * g));
+        const cpx q = __ldcs(reinterpret_cast<const cpx*>(w.q));
         lo = q.x;
         hi = q.y;
       } else {
-        lo = __ldcs(in + 2 * g);
-        hi = __ldcs(in + 2 * g + 1);
+        lo = __ldcs(w.q);
+        hi = __ldcs(w.q + 1);
       }
-      a[r] = lo;
-      sb[pc * 2 * t.lp + (L - 1 - n)] = hi;
+      a[r] = sg * lo;  // DST: -(a - ib) = -a + ib
+      put[-r * TPT] = hi;
     }
     __syncthreads();
     // w_2N^g for g = g0 + r*TPT*in_n
     const RootProgression<R> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(b1 * p.is1 + int64_t(x.j) * p.in_n),
                                 uint32_t(int64_t(TPT) * p.in_n));
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int n = x.j + r * TPT;
-      const real b = sb[x.c * 2 * t.lp + n];
-      const cpx e = ew.at(r);
-      if (!dst) {
-        v[r] = cmul(e, cmk(a[r], b));
-      } else {
-        const cpx q = cmul(e, cmk(a[r], -b));
-        v[r] = cmk(-q.x, -q.y);
-      }
-    }
+    for (int r = 0; r < R; ++r) v[r] = cmul(ew.at(r), cmk(a[r], get[r * TPT]));
   }
 };
 
@@ -887,35 +970,48 @@ struct LoadT4Chain {
 // f64: ten launches in 145 us before, six in 105 us now, 19 us for a plain
 // pass of 33.6 MB each way and 25 to 28 us for a fused one).
 
-// Slot and element of the mirror of element n in slot c.
+// Slot of the mirror sub-DFT, and the thread whose elements mirror this
+// thread's: element j + r*TPT pairs with element jm + (R-1-r)*TPT of that
+// slot (jm = TPT-1-j; TPT-j in sub-DFT 0 of spectrum pairs).  In sub-DFT 0
+// thread 0 pairs its elements r and R-r among themselves: it puts element r
+// where the others put r-1 (`turned`), so that it reads its partners at the
+// same places; its element 0 is point 0, which every step treats apart.
 struct Mirror {
-  int slot, flip;  // partner element: (flip - n) & (L - 1)
+  int slot, jm;
+  bool turned;
 };
 // Reflected pairs.
-template <int L>
-__device__ __forceinline__ Mirror mirror_reflected(const AxisParams& p, int c) {
+template <int TPT>
+__device__ __forceinline__ Mirror mirror_reflected(const AxisParams& p, const Ctx& x) {
   const int h = p.cpb / 2;
-  return Mirror{c < h ? c + h : c - h, L - 1};
+  return Mirror{x.c < h ? x.c + h : x.c - h, TPT - 1 - x.j, false};
 }
 // Spectrum pairs; i is the sub-DFT's index in its line.
-template <int L>
-__device__ __forceinline__ Mirror mirror_spectrum(const AxisParams& p, int c, int64_t i) {
+template <int TPT>
+__device__ __forceinline__ Mirror mirror_spectrum(const AxisParams& p, const Ctx& x, int64_t i) {
   const int h = p.cpb / 2;
-  if (i == 0) return Mirror{c, L};
-  if (2 * i == p.d0 * p.d1) return Mirror{c, L - 1};
-  return Mirror{c < h ? c + h : c - h, L - 1};
+  if (i == 0) return Mirror{x.c, x.j == 0 ? 0 : TPT - x.j, x.j == 0};
+  if (2 * i == p.d0 * p.d1) return Mirror{x.c, TPT - 1 - x.j, false};
+  return Mirror{x.c < h ? x.c + h : x.c - h, TPT - 1 - x.j, false};
 }
-
-// One value of the packing step (pack_pair) for the spectrum pair (z, zm) of
-// points k and Lt-k: the conjugated inverse-DFT input at k; f = w_N^k.
-__device__ __forceinline__ cpx pack_one(cpx z, cpx zm, cpx f) {
-  const cpx m = cconj(zm);
-  return cconj(cadd(cadd(z, m), cmul(csub(z, m), cmk(f.y, f.x))));
+// Tile address of element j of slot c; element j + r*TPT is at nat_off<TPT>(r) from it.
+template <int TPT>
+__device__ __forceinline__ cpx* slot_at(const Tile& t, int c, int j) {
+  return t.s + c * t.lp + (TPT >= 16 ? pad16(j) : j);
 }
-// One value of the unpacking step (unpack_pair2): 2 X_k from Z_k, Z_(Lt-k).
-__device__ __forceinline__ cpx unpack_one2(cpx z, cpx zm, cpx f) {
-  const cpx m = cconj(zm);
-  return cadd(cadd(z, m), cmul(csub(z, m), cmk(f.y, -f.x)));
+// The thread's elements into its slot, where their mirrors' threads read
+// them: element r's partner is then at slot_at(mi.slot, mi.jm) + nat_off(R-1-r).
+template <int L, int R>
+__device__ __forceinline__ void scatter_mirror(const cpx (&v)[R], const Ctx& x, const Mirror& mi, const Tile& t) {
+  constexpr int TPT = L / R;
+  cpx* q = slot_at<TPT>(t, x.c, x.j);
+  if (mi.turned) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) q[nat_off<TPT>((r + R - 1) % R)] = v[r];
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) q[nat_off<TPT>(r)] = v[r];
+  }
 }
 
 // Four consecutive reals, as 16-byte vectors where `vec`.
@@ -975,19 +1071,22 @@ struct LoadDCT2Line {
     constexpr int TPT = L / R;
     const ChainIn ci = chain_in(p, x);
     const real sg = (p.flags & F_DST) ? real(-1) : real(1);
-    const Mirror mi = mirror_reflected<L>(p, x.c);
+    const Mirror mi = mirror_reflected<TPT>(p, x);
     const bool vec = (reinterpret_cast<uintptr_t>(ci.in) & 15) == 0;
+    Walk<const real, false, TPT> w(ci.in + 4 * (ci.i + int64_t(x.j) * p.in_n), 4 * p.in_n);
     Real4 q[R / 2];
 #pragma unroll
-    for (int r = 0; r < R / 2; ++r) q[r] = ld_real4(ci.in + 4 * (ci.i + int64_t(x.j + r * TPT) * p.in_n), vec);
+    for (int r = 0; r < R / 2; ++r, w.step()) q[r] = ld_real4(w.q, vec);
+    cpx* put = slot_at<TPT>(t, mi.slot, mi.jm);
+    const cpx* get = slot_at<TPT>(t, x.c, x.j);
 #pragma unroll
     for (int r = 0; r < R / 2; ++r) {
       v[r] = cmk(q[r].v[0], q[r].v[2]);
-      t.s[t.idx(mi.slot, L - 1 - (x.j + r * TPT))] = cmk(sg * q[r].v[3], sg * q[r].v[1]);
+      put[nat_off<TPT>(R - 1 - r)] = cmk(sg * q[r].v[3], sg * q[r].v[1]);
     }
     __syncthreads();
 #pragma unroll
-    for (int r = R / 2; r < R; ++r) v[r] = t.s[t.idx(x.c, x.j + r * TPT)];
+    for (int r = R / 2; r < R; ++r) v[r] = get[nat_off<TPT>(r)];
   }
 };
 
@@ -998,14 +1097,11 @@ template <int L, int R>
 __device__ __forceinline__ void pack_tile(const Ctx& x, const Tile& t, const Mirror& mi, bool zero, cpx k0,
                                           const RootProgression<R>& fw, cpx (&v)[R]) {
   constexpr int TPT = L / R;
-#pragma unroll
-  for (int r = 0; r < R; ++r) t.s[t.idx(x.c, x.j + r * TPT)] = v[r];
+  scatter_mirror<L, R>(v, x, mi, t);
   __syncthreads();
+  const cpx* zm = slot_at<TPT>(t, mi.slot, mi.jm);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const cpx zm = t.s[t.idx(mi.slot, (mi.flip - (x.j + r * TPT)) & (L - 1))];
-    v[r] = pack_one(v[r], zm, fw.at(r));
-  }
+  for (int r = 0; r < R; ++r) v[r] = pack_one(v[r], zm[nat_off<TPT>(R - 1 - r)], fw.at(r));
   if (zero) v[0] = k0;
 }
 
@@ -1021,24 +1117,27 @@ struct LoadDCT3Line {
     const ChainIn ci = chain_in(p, x);
     const bool dst = (p.flags & F_DST) != 0;
     const int64_t N = p.kn;
-    const Mirror mi = mirror_spectrum<L>(p, x.c, ci.i);
-    const bool zero = ci.i == 0 && x.j == 0;  // element 0 is point 0: x_0 and x_Lt
+    const Mirror mi = mirror_spectrum<TPT>(p, x, ci.i);
+    const bool zero = mi.turned;  // element 0 is point 0: x_0 and x_Lt
     const int64_t g0 = ci.i + int64_t(x.j) * p.in_n, st = int64_t(TPT) * p.in_n;
-    const real* qa = dst ? ci.in + (N - 1 - g0) : ci.in + g0;
-    const real* qb = dst ? ci.in + (g0 - 1) : ci.in + (N - g0);
-    const int64_t sa = dst ? -st : st;
+    const int64_t sa = dst ? -p.in_n : p.in_n;
+    Walk<const real, false, TPT> wa(dst ? ci.in + (N - 1 - g0) : ci.in + g0, sa);
+    Walk<const real, false, -TPT> wb(dst ? ci.in + (g0 - 1) : ci.in + (N - g0), sa);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const real* b = qb - r * sa;
+    for (int r = 0; r < R; ++r, wa.step(), wb.step()) {
+      const real* b = wb.q;
       if (r == 0 && zero) b = ci.in + (dst ? N / 2 - 1 : N / 2);
-      v[r] = cmk(__ldcs(qa + r * sa), __ldcs(b));
+      v[r] = cmk(__ldcs(wa.q), __ldcs(b));
     }
     const real r2 = real(1.414213562373095048801688724209698079);
     const cpx k0 = cmk(v[0].x + r2 * v[0].y, -(v[0].x - r2 * v[0].y));
     {
       const RootProgression<R> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0), uint32_t(st));
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = cconj(cmul(v[r], ew.at(r)));
+      for (int r = 0; r < R; ++r) {
+        const cpx e = ew.at(r);
+        v[r] = cmk(v[r].x * e.x - v[r].y * e.y, -(v[r].x * e.y) - v[r].y * e.x);
+      }
     }
     const RootProgression<R> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(4 * g0), uint32_t(4 * st));
     pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
@@ -1056,11 +1155,12 @@ struct LoadC2RLine {
     constexpr int TPT = L / R;
     const int64_t rest = udiv(x.b, p.d0), line = udiv(rest, p.d1), i = rest - line * p.d1;
     const cpx* in = static_cast<const cpx*>(p.in) + line * p.k_in_line;
-    const Mirror mi = mirror_spectrum<L>(p, x.c, i);
-    const bool zero = i == 0 && x.j == 0;
+    const Mirror mi = mirror_spectrum<TPT>(p, x, i);
+    const bool zero = mi.turned;
     const int64_t g0 = i + int64_t(x.j) * p.in_n, st = int64_t(TPT) * p.in_n;
+    Walk<const cpx, false, TPT> w(in + g0, p.in_n);
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = __ldcs(in + g0 + r * st);
+    for (int r = 0; r < R; ++r, w.step()) v[r] = __ldcs(w.q);
     cpx k0 = czero();
     if (zero) {
       const cpx zl = in[p.kn / 2];
@@ -1133,19 +1233,24 @@ struct StoreR2C {
     if (!x.active) return;
     cpx* out = static_cast<cpx*>(p.out) + x.oout;
     const cpx b1 = kind_base<L / R>(p.t1, x.j);
-    pair_loop<L, R>(x, [&](int k) { return t.s[t.idx(x.c, k & (L - 1))]; }, [&](int i, int k, cpx za, cpx zb) {
-      if (k == 0) {
-        out[0] = cmk(za.x + za.y, real(0));
-        out[L] = cmk(za.x - za.y, real(0));
-      } else if (2 * k == L) {
-        out[k] = cconj(za);
-      } else {
-        cpx xa, xb;
-        unpack_pair(za, zb, rft_root<R>(b1, i), xa, xb);
-        out[k] = xa;
-        out[L - k] = xb;
-      }
-    });
+    const PairSlots<L, R> at(t, x.c, x.j);
+    pair_loop<L, R>(
+        x,
+        [&](int i, int k) {
+          const cpx za = at.at(i);
+          if (k == 0) {
+            out[0] = cmk(za.x + za.y, real(0));
+            out[L] = cmk(za.x - za.y, real(0));
+          } else {
+            out[k] = cconj(za);
+          }
+        },
+        [&](int i, int k) {
+          const cpx za = at.at(i), zb = at.mirror(i), f = rft_root<R>(b1, i);
+          out[k] = cscale(unpack_one2(za, zb, f), real(0.5));
+          out[L - k] = cscale(unpack_mirror2(za, zb, f), real(0.5));
+        },
+        [] {});
   }
 };
 
@@ -1203,23 +1308,26 @@ struct StoreDCT2 {
       *a = dst ? -q.y : q.x;
       *b = dst ? q.x : -q.y;
     };
-    pair_loop<L, R>(x, [&](int k) { return t.s[t.idx(x.c, k & (L - 1))]; }, [&](int i, int k, cpx za, cpx zb) {
-      if (k == 0) {
-        const real v0 = za.x + za.y, vl = za.x - za.y;
-        *(dst ? hi.q : lo.q) = 2 * v0;
-        *up.q = r2 * vl;
-      } else if (2 * k == L) {
-        const cpx q = cmul(cconj(za), w128(8));  // w_4N^(L/2) = w_16
-        put(lo.q, hi.q, cmk(2 * q.x, 2 * q.y));
-      } else {
-        cpx xa2, xb2;
-        unpack_pair2(za, zb, rft_root<R>(b2, i), xa2, xb2);
-        const cpx e = t23_root<R>(b1, i);  // w_4N^k
-        put(lo.q, hi.q, cmul(xa2, e));
-        put(dn.q, up.q, cmul(xb2, t23_mirror(e)));
-      }
-      lo.step(), up.step(), hi.step(), dn.step();
-    });
+    const PairSlots<L, R> at(t, x.c, x.j);
+    pair_loop<L, R>(
+        x,
+        [&](int i, int k) {
+          const cpx za = at.at(i);
+          if (k == 0) {
+            const real v0 = za.x + za.y, vl = za.x - za.y;
+            *(dst ? hi.q : lo.q) = 2 * v0;
+            *up.q = r2 * vl;
+          } else {
+            const cpx q = cmul(cconj(za), w128(8));  // w_4N^(L/2) = w_16
+            put(lo.q, hi.q, cmk(2 * q.x, 2 * q.y));
+          }
+        },
+        [&](int i, int) {
+          const cpx za = at.at(i), zb = at.mirror(i), f = rft_root<R>(b2, i), e = t23_root<R>(b1, i);
+          put(lo.q, hi.q, cmul(unpack_one2(za, zb, f), e));
+          put(dn.q, up.q, cmul(unpack_mirror2(za, zb, f), t23_mirror(e)));
+        },
+        [&] { lo.step(), up.step(), hi.step(), dn.step(); });
   }
 };
 
@@ -1392,17 +1500,15 @@ struct StoreT4 {
     constexpr int N = 2 * L, TPT = L / R;
     Walk<real, kUnit, 2 * TPT> lo(out + int64_t(2 * j) * s, s);
     Walk<real, kUnit, -2 * TPT> hi(out + int64_t(N - 1 - 2 * j) * s, s);
-    // t2[q] = w_8N^(2q+1): t2[2m] = t2[2j] * w_4R^r and t2[N-1-2m] =
-    // t2[N-1-2j] * conj(w_4R^r) for m = j + r*TPT
-    const cpx glo = ldg(p.t2 + 2 * j);
-    const cpx ghi = ldg(p.t2 + (N - 1 - 2 * j));
+    // t2[q] = w_8N^(2q+1): g_2m = t2[2j] * w_4R^r for m = j + r*TPT, and
+    // g_{N-1-2m} = -i conj(g_2m), so that one product A = g_2m T_m gives both
+    // outputs: 2 Re(g_{N-1-2m} conj(T_m)) = -2 Im A (Im: -2 Re A)
+    const cpx g = cscale(ldg(p.t2 + 2 * j), real(2));
 #pragma unroll
     for (int r = 0; r < R; ++r, lo.step(), hi.step()) {
-      const cpx T = v[r];
-      const cpx a = cmul(cmul(glo, w128(r * (32 / R))), T);
-      const cpx b = cmul(cmulc(ghi, w128(r * (32 / R))), cconj(T));
-      *lo.q = 2 * (dst ? a.y : a.x);
-      *hi.q = 2 * (dst ? b.y : b.x);
+      const cpx A = cmul(cmul(g, w128(r * (32 / R))), v[r]);
+      *lo.q = dst ? A.y : A.x;
+      *hi.q = dst ? -A.x : -A.y;
     }
   }
 };
@@ -1434,30 +1540,26 @@ struct StoreT4Chain {
     const RootProgression<R> gw(p.t1, p.t2, p.kbits, uint32_t(4 * (x.oout + int64_t(x.j) * p.out_k) + 1),
                                 uint32_t(4 * int64_t(TPT) * p.out_k));
     __syncthreads();  // the last Stockham exchange has finished with the tile
+    // a slot holds 2*lp >= 2L reals: the mirror's values below L, its own above
+    real* own = sb + x.c * 2 * t.lp + x.j;
+    real* put = sb + pc * 2 * t.lp + (L - 1 - x.j);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int k = x.j + r * TPT;
-      const cpx ga = gw.at(r);
-      const cpx gb = cmk(-ga.y, -ga.x);  // -i conj(ga) = w_8N^(2N-1-4m)
-      const cpx T = v[r];
-      const cpx A = cmul(ga, T);
-      const cpx B = cmul(gb, cconj(T));
-      // a slot holds 2*lp >= 2L reals: the mirror's values below L, its own above
-      sb[x.c * 2 * t.lp + L + k] = 2 * (dst ? A.y : A.x);
-      sb[pc * 2 * t.lp + (L - 1 - k)] = 2 * (dst ? B.y : B.x);
+      // with g_{N-1-2m} = -i conj(g_2m), A = g_2m T_m gives both outputs (StoreT4)
+      const cpx A = cmul(gw.at(r), v[r]);
+      own[L + r * TPT] = 2 * (dst ? A.y : A.x);
+      put[-r * TPT] = -2 * (dst ? A.x : A.y);
     }
     __syncthreads();
+    Walk<real, false, TPT> w(out + 2 * (x.oout + int64_t(x.j) * p.out_k), 2 * p.out_k);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int k = x.j + r * TPT;
-      const int64_t m = x.oout + int64_t(k) * p.out_k;
-      const real own = sb[x.c * 2 * t.lp + L + k];
-      const real part = sb[x.c * 2 * t.lp + k];
+    for (int r = 0; r < R; ++r, w.step()) {
+      const real a = own[L + r * TPT], b = own[r * TPT];
       if (vec) {
-        __stcs(reinterpret_cast<cpx*>(out + 2 * m), cmk(own, part));
+        __stcs(reinterpret_cast<cpx*>(w.q), cmk(a, b));
       } else {
-        __stcs(out + 2 * m, own);
-        __stcs(out + 2 * m + 1, part);
+        __stcs(w.q, a);
+        __stcs(w.q + 1, b);
       }
     }
   }
@@ -1473,21 +1575,22 @@ struct StoreR2CLine {
                                              cpx (&v)[R]) {
     constexpr int TPT = L / R;
     cpx* out = static_cast<cpx*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
-    const Mirror mi = mirror_spectrum<L>(p, x.c, x.oout);
+    const Mirror mi = mirror_spectrum<TPT>(p, x, x.oout);
     const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
     const RootProgression<R> fw(p.t1, p.t2, p.kbits, uint32_t(m0), uint32_t(st));
     __syncthreads();  // the last Stockham exchange has finished with the tile
-    scatter_natural<L, R>(v, x.j, x.c, t);
+    scatter_mirror<L, R>(v, x, mi, t);
     __syncthreads();
+    const cpx* zm = slot_at<TPT>(t, mi.slot, mi.jm);
+    Walk<cpx, false, TPT> w(out + m0, p.out_k);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const cpx zm = t.s[t.idx(mi.slot, (mi.flip - (x.j + r * TPT)) & (L - 1))];
-      cpx X = cscale(unpack_one2(v[r], zm, fw.at(r)), real(0.5));
-      if (r == 0 && m0 == 0) {
+    for (int r = 0; r < R; ++r, w.step()) {
+      cpx X = cscale(unpack_one2(v[r], zm[nat_off<TPT>(R - 1 - r)], fw.at(r)), real(0.5));
+      if (r == 0 && mi.turned) {
         X = cmk(v[0].x + v[0].y, real(0));
         out[p.kn / 2] = cmk(v[0].x - v[0].y, real(0));
       }
-      out[m0 + r * st] = X;
+      *w.q = X;
     }
   }
 };
@@ -1505,36 +1608,34 @@ struct StoreDCT2Line {
     real* out = static_cast<real*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
     const bool dst = (p.flags & F_DST) != 0;
     const int64_t N = p.kn;
-    const Mirror mi = mirror_spectrum<L>(p, x.c, x.oout);
+    const Mirror mi = mirror_spectrum<TPT>(p, x, x.oout);
     const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
     __syncthreads();  // the last Stockham exchange has finished with the tile
-    scatter_natural<L, R>(v, x.j, x.c, t);
+    scatter_mirror<L, R>(v, x, mi, t);
     __syncthreads();
     const real r2 = real(1.414213562373095048801688724209698079);
     const real y0 = 2 * (v[0].x + v[0].y), yl = r2 * (v[0].x - v[0].y);
+    const cpx* zm = slot_at<TPT>(t, mi.slot, mi.jm);
     {
       const RootProgression<R> fw(p.t1, p.t2, p.kbits, uint32_t(4 * m0), uint32_t(4 * st));
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const cpx zm = t.s[t.idx(mi.slot, (mi.flip - (x.j + r * TPT)) & (L - 1))];
-        v[r] = unpack_one2(v[r], zm, fw.at(r));
-      }
+      for (int r = 0; r < R; ++r) v[r] = unpack_one2(v[r], zm[nat_off<TPT>(R - 1 - r)], fw.at(r));
     }
     const RootProgression<R> ew(p.t1, p.t2, p.kbits, uint32_t(m0), uint32_t(st));
-    real* qa = dst ? out + (N - 1 - m0) : out + m0;
-    real* qb = dst ? out + (m0 - 1) : out + (N - m0);
-    const int64_t sa = dst ? -st : st;
+    const int64_t sa = dst ? -p.out_k : p.out_k;
+    Walk<real, false, TPT> wa(dst ? out + (N - 1 - m0) : out + m0, sa);
+    Walk<real, false, -TPT> wb(dst ? out + (m0 - 1) : out + (N - m0), sa);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const cpx q = cmul(v[r], ew.at(r));
-      real a = q.x, b = -q.y;
-      real* pb = qb - r * sa;
-      if (r == 0 && m0 == 0) {
+    for (int r = 0; r < R; ++r, wa.step(), wb.step()) {
+      const cpx e = ew.at(r);
+      real a = v[r].x * e.x - v[r].y * e.y, b = -(v[r].x * e.y) - v[r].y * e.x;
+      real* pb = wb.q;
+      if (r == 0 && mi.turned) {
         a = y0;
         b = yl;
         pb = out + (dst ? N / 2 - 1 : N / 2);
       }
-      qa[r * sa] = a;
+      *wa.q = a;
       *pb = b;
     }
   }
@@ -1551,17 +1652,19 @@ struct StoreDCT3Line {
     constexpr int TPT = L / R;
     real* out = static_cast<real*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
     const real sg = (p.flags & F_DST) ? real(-1) : real(1);
-    const Mirror mi = mirror_reflected<L>(p, x.c);
+    const Mirror mi = mirror_reflected<TPT>(p, x);
     const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    cpx* put = slot_at<TPT>(t, mi.slot, mi.jm);
+    const cpx* get = slot_at<TPT>(t, x.c, x.j);
     __syncthreads();  // the last Stockham exchange has finished with the tile
 #pragma unroll
-    for (int r = R / 2; r < R; ++r) t.s[t.idx(mi.slot, L - 1 - (x.j + r * TPT))] = v[r];
+    for (int r = R / 2; r < R; ++r) put[nat_off<TPT>(R - 1 - r)] = v[r];
     __syncthreads();
-    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
+    Walk<real, false, TPT> w(out + 4 * (x.oout + int64_t(x.j) * p.out_k), 4 * p.out_k);
 #pragma unroll
-    for (int r = 0; r < R / 2; ++r) {
-      const cpx w = cconj(v[r]), u = cconj(t.s[t.idx(x.c, x.j + r * TPT)]);
-      st_real4(out + 4 * (m0 + r * st), Real4{{w.x, sg * u.y, w.y, sg * u.x}}, vec);
+    for (int r = 0; r < R / 2; ++r, w.step()) {
+      const cpx u = get[nat_off<TPT>(r)];  // conjugated, as v is
+      st_real4(w.q, Real4{{v[r].x, -sg * u.y, -v[r].y, sg * u.x}}, vec);
     }
   }
 };
