@@ -61,7 +61,15 @@ __device__ __forceinline__ cpx cmul(cpx a, cpx b) { return cmk(a.x * b.x - a.y *
 // a * conj(b)
 __device__ __forceinline__ cpx cmulc(cpx a, cpx b) { return cmk(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y); }
 __device__ __forceinline__ cpx cconj(cpx a) { return cmk(a.x, -a.y); }
+#if MINFFT_SINGLE
+__device__ __forceinline__ cpx cscale(cpx a, real s) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(cpack(a)), "l"(cpack(cmk(s, s))));
+  return cunpack(r);
+}
+#else
 __device__ __forceinline__ cpx cscale(cpx a, real s) { return cmk(a.x * s, a.y * s); }
+#endif
 // a * (-i)
 __device__ __forceinline__ cpx cmul_negi(cpx a) { return cmk(a.y, -a.x); }
 __device__ __forceinline__ cpx czero() { return cmk(real(0), real(0)); }

@@ -657,8 +657,8 @@ struct Planner {
 
   // Form of the tensor-core pass: the streamed form (tc_stream_kernel) by
   // default, the one-tile form with MINFFT_B200_TC_FORM=tile; stages of the
-  // streamed form from MINFFT_B200_TC_STAGES (2 .. 6; default 2, which fits
-  // four CTAs per SM in FP16 and three in BF16).
+  // streamed form from MINFFT_B200_TC_STAGES (1 .. 6; default 1, which fits
+  // five CTAs per SM in FP16 and four in BF16).
   static bool tc_stream_default() {
     static const bool on = [] {
       const char* e = getenv("MINFFT_B200_TC_FORM");
@@ -670,9 +670,9 @@ struct Planner {
     static const int n = [] {
       const char* e = getenv("MINFFT_B200_TC_STAGES");
       const int v = e ? atoi(e) : 0;
-      return v <= 0 ? 0 : (v < 2 ? 2 : (v > 6 ? 6 : v));
+      return v <= 0 ? 0 : (v > 6 ? 6 : v);
     }();
-    return n ? n : 2;
+    return n ? n : 1;
   }
 
   // Normalised layout of the streamed tensor-core pass: b0 indexes the
@@ -2801,7 +2801,7 @@ MB_EXPORT int minfft_b200_plan_selfcheck_precision(int op, int d, const int* Ns,
           fail("launch %zu (%s): streamed tensor-core tile layout", i, ln.label.c_str());
         if (ap.d0 * ap.d1 * ln.st_d2 != ap.nbatch || ap.gpb * W < ap.d0 || ap.ntiles != ap.gpb * ap.d1 * ln.st_d2)
           fail("launch %zu (%s): streamed tensor-core tiles do not cover the batch", i, ln.label.c_str());
-        if (ln.block != unsigned(mb::kTcStreamThreads) || ap.cpb < 2 || ap.cpb > 8 || ln.grid < 1 ||
+        if (ln.block != unsigned(mb::kTcStreamThreads) || ap.cpb < 1 || ap.cpb > 8 || ln.grid < 1 ||
             int64_t(ln.grid) > ap.ntiles)
           fail("launch %zu: streamed tensor-core shape", i);
       } else {

@@ -549,16 +549,22 @@ __global__ void __launch_bounds__(16 * TB, TB == 8 ? 4 : 2) tc256_kernel(const A
 // into another) and commits them to an mbarrier; every thread reads its row
 // of both accumulators with one tcgen05.ld each, adds them and unscales.
 //
-// Between the stages the twiddled values go back into the stage, which then
-// holds y1 in a layout chosen per tile kind so that the writes (lanes over
-// n2) and the reads (lanes over k1) are both conflict-free: column tiles
-// (16 k1 + (n2 ^ (k1 & 1))) * 8 + c (a warp's four k1 rows of 64 bytes then
-// fall on both halves of the banks), row tiles c * 256 + 16 k1 + (n2 ^ k1).
+// Between the stages the twiddled values go into the operand buffer, which
+// the finished MMAs have left free, in a layout chosen per tile kind so that
+// the writes (lanes over n2) and the reads (lanes over k1) are both
+// conflict-free: column tiles (16 k1 + (n2 ^ (k1 & 1))) * 8 + c (a warp's
+// four k1 rows of 64 bytes then fall on both halves of the banks), row tiles
+// c * 256 + 16 k1 + (n2 ^ k1).  So the input stage is free as soon as stage 1
+// has read it, and the next tile's copy runs under the two contractions: one
+// stage is enough, and five CTAs fit an SM in FP16, four in BF16.  The pass
+// is bound by its instructions and their latency (tensor pipe under 10%
+// busy), so resident warps count most: 256^3, round trip, 424 us with two
+// stages held to the end of a tile (four CTAs), 391 so in FP16, 558 -> 491 in
+// BF16; with two stages 412 and 532.
 constexpr int kTcsW = kTcStreamTile;     // transforms per tile
 constexpr int kTcsNT = kTcStreamThreads; // threads
 constexpr int kTcsG = kTcsNT / 128;      // UMMA groups of 128 rows
 static_assert(kTcsW * 16 == kTcsNT, "one contraction row per thread");
-constexpr int kTcsStages = 2;
 
 template <int FMT>
 struct TcsLayout {
@@ -570,9 +576,10 @@ struct TcsLayout {
   static constexpr int st_off = a_off + kTcsG * NT * kOpBytes;
   static constexpr int tmem_cols = 64 * kTcsG;           // groups x (leading, correction) x 32
   static_assert(tmem_cols == kTcStreamTmemCols, "tensor-memory columns");
+  static_assert(kTcsG * NT * kOpBytes >= kTcsW * kL * 8, "y1 fits the operand buffer");
 };
 
-__host__ __device__ inline int tcs_stage_bytes() { return (kTcsW * (kL + 1) * 8 + 127) / 128 * 128; }
+__host__ __device__ inline int tcs_stage_bytes() { return kTcsW * kL * 8; }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&d)[32]) {
   asm volatile(
@@ -588,38 +595,64 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&d)[32]) {
 
 // Power-of-two scale putting the largest component of 16 complex values
 // into [2^8, 2^9): returns the scale; *inv receives its inverse.
-__device__ __forceinline__ float tcs_scale(const float (&re)[16], const float (&im)[16], float* inv) {
+__device__ __forceinline__ float tcs_scale(const cpx (&u)[16], float* inv) {
   float mx = 0.f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) mx = fmaxf(mx, fmaxf(fabsf(re[i]), fabsf(im[i])));
+  for (int i = 0; i < 16; ++i) mx = fmaxf(mx, fmaxf(fabsf(u[i].x), fabsf(u[i].y)));
   const int ex = (__float_as_int(mx) >> 23) & 0xFF;
   const int s = min(max(135 - ex, -126), 126);
   *inv = pow2i(-s);
   return pow2i(s);
 }
 
-// Split row (re, im) * sc into NT terms and write them as row `row` of the
-// K-major A operands of group g (K: Re 0..15, Im 16..31).
+// The 16-bit term of a pair of values and its exact FP32 values.
 template <int FMT>
-__device__ __forceinline__ void tcs_write_a(unsigned char* aop, int g, int row, const float (&re)[16],
-                                            const float (&im)[16], float sc) {
+__device__ __forceinline__ uint32_t tcs_term(float a, float b, float& fa, float& fb) {
+  if constexpr (FMT == TC_F16) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    fa = f.x;
+    fb = f.y;
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    const uint32_t w = *reinterpret_cast<const uint32_t*>(&h);
+    fa = __uint_as_float(w << 16);
+    fb = __uint_as_float(w & 0xFFFF0000u);
+    return w;
+  }
+}
+
+// Split row u * sc into NT terms and write them as row `row` of the K-major
+// A operands of group g (K: Re 0..15, Im 16..31).  The scaling and the
+// remainders are packed over (re, im).
+template <int FMT>
+__device__ __forceinline__ void tcs_write_a(unsigned char* aop, int g, int row, const cpx (&u)[16], float sc) {
   constexpr int NT = TcsLayout<FMT>::NT;
 #pragma unroll
-  for (int kb = 0; kb < 4; ++kb) {
-    uint32_t w[NT][4];
+  for (int h = 0; h < 2; ++h) {  // K blocks 8h.. of Re and of Im
+    uint32_t wr[NT][4], wi[NT][4];
 #pragma unroll
-    for (int u = 0; u < 8; u += 2) {
-      uint32_t o[3];
-      const int k = kb * 8 + u;
-      const float a = k < 16 ? re[k] : im[k - 16], b = k + 1 < 16 ? re[k + 1] : im[k + 1 - 16];
-      split_pair<FMT, NT>(a * sc, b * sc, o);
+    for (int k = 0; k < 4; ++k) {
+      cpx a = cscale(u[8 * h + 2 * k], sc), b = cscale(u[8 * h + 2 * k + 1], sc);
 #pragma unroll
-      for (int z = 0; z < NT; ++z) w[z][u / 2] = o[z];
+      for (int z = 0; z < NT; ++z) {
+        cpx fa, fb;
+        wr[z][k] = tcs_term<FMT>(a.x, b.x, fa.x, fb.x);
+        wi[z][k] = tcs_term<FMT>(a.y, b.y, fa.y, fb.y);
+        if (z + 1 < NT) {
+          a = csub(a, fa);
+          b = csub(b, fb);
+        }
+      }
     }
 #pragma unroll
-    for (int z = 0; z < NT; ++z)
-      *reinterpret_cast<uint4*>(aop + (z * kTcsG + g) * kOpBytes + tc_operand_offset(row, kb * 8)) =
-          make_uint4(w[z][0], w[z][1], w[z][2], w[z][3]);
+    for (int z = 0; z < NT; ++z) {
+      unsigned char* o = aop + (z * kTcsG + g) * kOpBytes;
+      *reinterpret_cast<uint4*>(o + tc_operand_offset(row, 8 * h)) = make_uint4(wr[z][0], wr[z][1], wr[z][2], wr[z][3]);
+      *reinterpret_cast<uint4*>(o + tc_operand_offset(row, 16 + 8 * h)) =
+          make_uint4(wi[z][0], wi[z][1], wi[z][2], wi[z][3]);
+    }
   }
 }
 
@@ -656,22 +689,24 @@ __device__ __forceinline__ void tcs_issue_mma(uint32_t aop_a, uint32_t bop_a, ui
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mb) : "memory");
 }
 
-// This thread's row of both accumulators, summed: re[k], im[k], k = 0..15.
-__device__ __forceinline__ void tcs_read_d(uint32_t tmem, int warp, float (&re)[16], float (&im)[16]) {
+// This thread's row of both accumulators, summed: (re, im) of outputs 2k and
+// 2k + 1 as the pairs re[k], im[k], k = 0..7.
+__device__ __forceinline__ void tcs_read_d(uint32_t tmem, int warp, cpx (&re)[8], cpx (&im)[8]) {
   const uint32_t taddr = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(64 * (warp >> 2));
   uint32_t d[32], e[32];
   tmem_ld32(taddr, d);
   tmem_ld32(taddr + 32, e);
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  auto pair = [](const uint32_t* q) { return cmk(__uint_as_float(q[0]), __uint_as_float(q[1])); };
 #pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    re[k] = __uint_as_float(d[k]) + __uint_as_float(e[k]);
-    im[k] = __uint_as_float(d[16 + k]) + __uint_as_float(e[16 + k]);
+  for (int k = 0; k < 8; ++k) {
+    re[k] = cadd(pair(d + 2 * k), pair(e + 2 * k));
+    im[k] = cadd(pair(d + 16 + 2 * k), pair(e + 16 + 2 * k));
   }
 }
 
 template <int FMT, bool ROWS>
-__global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kernel(const AxisParams p, const TcParams q,
+__global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 5 : 4) tc_stream_kernel(const AxisParams p, const TcParams q,
                                                               const __grid_constant__ CUtensorMap tmap) {
   using Lay = TcsLayout<FMT>;
   constexpr int NT = Lay::NT;
@@ -683,6 +718,7 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
   unsigned char* bop = sm + Lay::b_off;
   cpx* tws = reinterpret_cast<cpx*>(sm + Lay::tw_off);
   unsigned char* aop = sm + Lay::a_off;
+  cpx* mid = reinterpret_cast<cpx*>(aop);  // y1, and outputs to be transposed, while no MMA reads the operands
   unsigned char* stages = sm + Lay::st_off;
   const int S = p.cpb;
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -746,6 +782,7 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
     const uint32_t dst = st0 + uint32_t(s) * uint32_t(sb);
     if (tma) {
       if (tid == 0) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(W * kL * 8) : "memory");
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -783,12 +820,13 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
   const bool rows_out = (p.flags & F_STAGE_ROWS) != 0;
   const bool twid = p.st_ns > 1;
   const long long first_limit = q.wait_polls > 0 ? q.wait_polls : kSpinLimit;
-  bool ok = true, pending = false, first = true;
+  bool ok = true, pending = false, first = true, refilled = false;
   uint32_t mph = 0;
   int it = 0;
   int64_t t = blockIdx.x;
   for (; t < ntiles; t += gridDim.x, ++it) {
     const int s = it % S;
+    refilled = false;
     if (!smbar_wait(bar0 + 8 * s, uint32_t(it / S) & 1u, kStreamSpinLimit)) atomicExch(bad, 1);
     __syncthreads();
     if (*bad) {
@@ -800,14 +838,14 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
     tile_pos(t, c0, b1, b2);
     const int64_t col = c0 + c;  // this thread's transform (b0 index)
     const bool active = col < p.d0;
-    float re[16], im[16], inv;
+    float inv;
+    cpx u[16];
 
     // ---- stage 1: row (c, n2 = d), inputs x[16 n1 + d]
 #pragma unroll
     for (int n1 = 0; n1 < 16; ++n1) {
-      const cpx u = tile[pos_in(c, 16 * n1 + d)];
-      re[n1] = u.x;
-      im[n1] = cj_in ? -u.y : u.y;
+      u[n1] = tile[pos_in(c, 16 * n1 + d)];
+      if (cj_in) u[n1].y = -u[n1].y;
     }
     if (twid) {
       // pre-twiddle of a later pass of a Stockham chain: element n = 16 n1 + d
@@ -829,19 +867,19 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
         if ((i & 3) == 1) w = cmul(w, d1);
         if ((i & 3) == 2) w = cmul(w, d2);
         if ((i & 3) == 3) w = cmul(w, d3);
-        const cpx x = cmul(cmk(re[i], im[i]), w);
-        re[i] = x.x;
-        im[i] = x.y;
+        u[i] = cmul(u[i], w);
       }
     }
-    float sc = tcs_scale(re, im, &inv);
-    tcs_write_a<FMT>(aop, g, row, re, im, sc);
+    float sc = tcs_scale(u, &inv);
+    tcs_write_a<FMT>(aop, g, row, u, sc);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     const bool withheld = first && q.withhold;
     if (tid == 0 && !withheld) tcs_issue_mma<FMT>(aop_a, bop_a, tmem, mma_bar);
     pending = !withheld;
+    issue(t + int64_t(S) * gridDim.x, s);  // every thread has read the stage: refill it
+    refilled = true;
     if (!smbar_wait(mma_bar, mph, first ? first_limit : kSpinLimit)) atomicExch(bad, 1);
     first = false;
     __syncthreads();
@@ -852,28 +890,30 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
     pending = false;
     mph ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    cpx re[8], im[8];
     tcs_read_d(tmem, warp, re, im);
-    // unscale and twiddle: y1[k1][n2] * w_256^(n2 k1), n2 = d; into the stage
+    // unscale and twiddle: y1[k1][n2] * w_256^(n2 k1), n2 = d; into the
+    // operand buffer, which the finished MMAs have left free
 #pragma unroll
-    for (int k1 = 0; k1 < 16; ++k1) {
-      const cpx w = tws[16 * k1 + d];
-      const cpx y = cmul(cmk(re[k1] * inv, im[k1] * inv), w);
-      const int idx = ROWS ? c * kL + 16 * k1 + (d ^ k1) : (16 * k1 + (d ^ (k1 & 1))) * W + c;
-      tile[idx] = y;
+    for (int k = 0; k < 8; ++k) {
+      const cpx rs = cscale(re[k], inv), is = cscale(im[k], inv);
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        const int k1 = 2 * k + o;
+        const cpx y = cmul(o ? cmk(rs.y, is.y) : cmk(rs.x, is.x), tws[16 * k1 + d]);
+        mid[ROWS ? c * kL + 16 * k1 + (d ^ k1) : (16 * k1 + (d ^ (k1 & 1))) * W + c] = y;
+      }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
 
     // ---- stage 2: row (c, k1 = d), inputs y1[16 d + n2], n2 = 0..15
 #pragma unroll
-    for (int n2 = 0; n2 < 16; ++n2) {
-      const int idx = ROWS ? c * kL + 16 * d + (n2 ^ d) : (16 * d + (n2 ^ (d & 1))) * W + c;
-      const cpx u = tile[idx];
-      re[n2] = u.x;
-      im[n2] = u.y;
-    }
-    sc = tcs_scale(re, im, &inv);
-    tcs_write_a<FMT>(aop, g, row, re, im, sc);
+    for (int n2 = 0; n2 < 16; ++n2)
+      u[n2] = mid[ROWS ? c * kL + 16 * d + (n2 ^ d) : (16 * d + (n2 ^ (d & 1))) * W + c];
+    sc = tcs_scale(u, &inv);
+    __syncthreads();  // every y1 has been read
+    tcs_write_a<FMT>(aop, g, row, u, sc);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -890,39 +930,42 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 4 : 3) tc_stream_kerne
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     tcs_read_d(tmem, warp, re, im);
     const float so = cj_out ? -inv : inv;
-    // outputs y[k1 + 16 k2], k1 = d
+    auto output = [&](int k2) {  // y[k1 + 16 k2], k1 = d
+      const cpx r = re[k2 / 2], i = im[k2 / 2];
+      return k2 & 1 ? cmk(r.y * inv, i.y * so) : cmk(r.x * inv, i.x * so);
+    };
     cpx* out = static_cast<cpx*>(p.out);
     const int64_t ob = b1 * p.os1 + b2 * p.os2;
     if (!rows_out) {
       if (active) {
-        cpx* o = out + ob + col * p.os0 + int64_t(d) * p.out_k;
+        Walk<cpx, false, 16> w(out + ob + col * p.os0 + int64_t(d) * p.out_k, p.out_k);
 #pragma unroll
-        for (int k2 = 0; k2 < 16; ++k2) o[int64_t(16 * k2) * p.out_k] = cmk(re[k2] * inv, im[k2] * so);
+        for (int k2 = 0; k2 < 16; ++k2, w.step()) *w.q = output(k2);
       }
     } else {
-      // contiguous outputs per transform: transpose through the stage
-      // (transform c at c*(256+1)), then store with k running fastest
+      // contiguous outputs per transform: transpose through the operand
+      // buffer (output k of transform c at c*256 + (k ^ 2c): a half warp's
+      // eight transforms and two outputs fall on distinct banks), then store
+      // with k running fastest
 #pragma unroll
-      for (int k2 = 0; k2 < 16; ++k2) tile[c * (kL + 1) + d + 16 * k2] = cmk(re[k2] * inv, im[k2] * so);
+      for (int k2 = 0; k2 < 16; ++k2) mid[c * kL + ((d + 16 * k2) ^ (2 * (c & 7)))] = output(k2);
       __syncthreads();
       const int nv = int(p.d0 - c0 < W ? p.d0 - c0 : W);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int e = tid + i * kTcsNT;
         const int cc = e / kL, k = e % kL;
-        if (cc < nv) out[ob + (c0 + cc) * p.os0 + int64_t(k) * p.out_k] = tile[cc * (kL + 1) + k];
+        if (cc < nv) out[ob + (c0 + cc) * p.os0 + int64_t(k) * p.out_k] = mid[cc * kL + (k ^ (2 * (cc & 7)))];
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();  // the stage and the accumulators are free
-    if (tma && tid == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    issue(t + int64_t(S) * gridDim.x, s);
+    __syncthreads();  // the operand buffer and the accumulators are free
   }
 
   if (!ok) {
     if (tid == 0 && q.status) atomicExch(q.status, 1);
     if (pending) mbar_wait(mma_bar, mph);
-    for (int k = 0; k < S; ++k, ++it, t += gridDim.x) {
+    for (int k = 0; k < S + (refilled ? 1 : 0); ++k, ++it, t += gridDim.x) {  // copies in flight
       if (t >= ntiles) break;
       smbar_wait(bar0 + 8 * (it % S), uint32_t(it / S) & 1u, kStreamSpinLimit);
     }
