@@ -313,6 +313,10 @@ struct minfft_aux {
   void* bufs[BUF_COUNT] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t buf_bytes[BUF_COUNT] = {0, 0, 0, 0, 0, 0};
   std::map<std::tuple<int, int, int>, Program> programs;  // (op, howmany, alias)
+  // the program of the last call (programs' nodes stay where they are until
+  // the map is cleared)
+  std::tuple<int, int, int> last_key{-1, 0, 0};
+  Program* last_program = nullptr;
   int precision = MINFFT_B200_PREC_FP32;  // arithmetic of the 256-point complex passes
   void* tc_mem = nullptr;                 // tensor-core B operands (both formats)
   int* dev_status = nullptr;              // set by kernels whose bounded device-side wait ran out
@@ -1963,8 +1967,12 @@ bool ensure_buffer(minfft_aux* a, int buf, size_t bytes) {
 
 Program* get_program(minfft_aux* a, int op, int howmany, bool alias) {
   auto key = std::make_tuple(op, howmany, alias ? 1 : 0);
+  if (a->last_program && a->last_key == key) return a->last_program;
   auto it = a->programs.find(key);
-  if (it != a->programs.end()) return &it->second;
+  if (it != a->programs.end()) {
+    a->last_key = key;
+    return a->last_program = &it->second;
+  }
   Program prog;
   if (!build_program(a, op, howmany, alias, &prog)) return nullptr;
   if (!a->host_only)
@@ -2501,6 +2509,7 @@ MB_EXPORT int minfft_b200_set_precision(minfft_aux* a, int mode) {
   if (a->precision != mode) {
     a->precision = mode;
     a->programs.clear();
+    a->last_program = nullptr;
   }
   return MINFFT_B200_OK;
 }
@@ -2941,6 +2950,7 @@ MB_EXPORT int minfft_b200_autotune(minfft_aux* a, int op, int howmany, int reps)
     for (auto& kv : best) g_tune[kv.first] = kv.second;
   }
   a->programs.clear();
+  a->last_program = nullptr;
   return rc;
 }
 
