@@ -197,9 +197,15 @@ __device__ __forceinline__ int64_t umod(int64_t a, int64_t b) {
 __device__ __forceinline__ int pad16(int p) { return p + (p >> 4); }
 __host__ __device__ constexpr int padded_len(int L) { return L + (L >> 4); }
 
+// Table reads.  A translation unit whose kernels keep their tables in shared
+// memory defines MB_TABLES_GENERIC: the read-only load is global-only.
 template <typename TT>
 __device__ __forceinline__ TT ldg(const TT* p) {
+#ifdef MB_TABLES_GENERIC
+  return *p;
+#else
   return __ldg(p);
+#endif
 }
 
 }  // namespace mb

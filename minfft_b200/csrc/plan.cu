@@ -39,6 +39,7 @@
 #include "pipe_pass.cuh"
 #include "stream_pass.cuh"
 #include "dct_split.h"
+#include "nd_pass.h"
 #include "line_kernels.h"
 #include "tc_pass.h"
 #include "minfft.h"
@@ -261,6 +262,9 @@ struct Launch {
   int dctq = -1;         // split-column DCT pass (dct_split.cu): mb::dctq_kernel's `which`, else -1
   mb::DctqParams dq{};   // its parameters (in, out, mid resolved at launch)
   int mid_buf = -1;      // its intermediate buffer
+  bool nd = false;       // whole small arrays in one launch (nd_pass.cu)
+  mb::NdParams ndp{};    // its parameters (in, out resolved at launch)
+  int64_t nd_in = 0, nd_out = 0;  // elements of all its arrays
   int64_t st_d2 = 1;     // streamed pass: outermost batch extent of its tensor copies
   bool tc = false;       // tensor-core split-precision pass (tc_pass.cu)
   mb::TcParams tcp{};    // its B operands and status word
@@ -269,8 +273,8 @@ struct Launch {
   TuneKey key{};         // axis kernels: autotuning key
   int L = 0;             // axis kernels: in-CTA DFT length
   int radix = 16;        // axis kernels: per-thread radix
-  AxisParams ap;
-  LineParams lp;
+  AxisParams ap{};
+  LineParams lp{};
   std::string label;  // kernel and shape, for launch-level timing
   double bytes = 0;   // algorithmic bytes: each input element read once, each output written once
 };
@@ -1524,6 +1528,117 @@ struct Planner {
     add_axis_kernel(mb::K_C2RQ, int(L), H * Nr, ap, mid, out_buf, false, true);
   }
 
+  // entries of the kind tables of host_table
+  static int table_entries(int kind, int64_t N) {
+    return int(kind == TB_RFT ? std::max<int64_t>(N / 4, 1) : kind == TB_T4POST ? N : std::max<int64_t>(N / 2, 1));
+  }
+
+  // A multi-dimensional transform of small arrays as one launch, a cluster of
+  // CTAs per array (nd_pass.cu), where its launches and not its work are the
+  // time: 2 to 4 axes of 2 .. 128 complex points each (256 reals), up to a
+  // CTA per SM in all.  Round trips, in us, as one launch per axis and so:
+  // DFT 64 x 64 f32 12.9 / 7.3, f64 13.1 / 8.1; 16^3 f32 18.4 / 11.1; real DFT
+  // 64 x 64 f64 13.0 / 10.5; DCT-2 + DCT-3 64 x 64 f32 12.8 / 10.5; DST-4 pair
+  // 64 x 64 f32 13.5 / 8.9.  Above 8192 complex points in single and 4096 in
+  // double one cluster takes too long (DFT 128 x 128 f64 12.8 / 13.2).  Types 2
+  // and 3 have the most code per step, and a step of a new length fetches its
+  // code anew: unequal axes only up to 512 points (64 x 128 f32 13.0 / 13.8,
+  // 16 x 32 f64 12.9 / 11.6).  A forced kernel form or radix keeps the axis
+  // passes.  steps: the transform's axis steps in order; mid_buf: the buffer
+  // between them.
+  bool plan_nd(const std::vector<AxisStep>& steps, int64_t howmany, int64_t in_elems, int64_t mid_elems,
+               int64_t out_elems, int mid_buf) {
+    static const bool on = [] {
+      const char* e = getenv("MINFFT_B200_ND");
+      return !(e && e[0] == '0');
+    }();
+    {
+      std::lock_guard<std::mutex> lk(g_tune_mu);
+      if (g_default_override.pipe >= 0 || g_default_override.cpb || g_default_override.radix != 16) return false;
+    }
+    if (!on || pipe_default() || howmany * mb::kNdCluster > sms || steps.size() < 2 ||
+        steps.size() > size_t(mb::kNdMaxAxes))
+      return false;
+    int64_t work = 0;  // complex points of the largest step
+    bool equal = true;
+    for (const AxisStep& s : steps) {
+      const int64_t L = s.combo == mb::K_CPLX ? s.N : s.N / 2;
+      if (s.N < 2 || ilog2(L) > mb::kNdMaxLog2L) return false;
+      work = std::max(work, s.outer / howmany * s.inner * L);
+      equal &= s.N == steps.front().N;
+    }
+    const int64_t most = sizeof(real) == 4 ? 8192 : 4096;
+    if (work > most + most / 16) return false;  // (a real DFT's spectrum holds one column more)
+    const int kind = steps.front().combo;
+    if ((kind == mb::K_DCT2 || kind == mb::K_DCT3) && !equal && work > 512) return false;
+    Launch ln;
+    ln.fn = mb::nd_kernel(steps.front().combo, steps.back().combo);
+    if (!ln.fn) return false;
+    mb::NdParams& d = ln.ndp;
+    d.naxes = (int)steps.size();
+    d.in_stride = in_elems;
+    d.mid_stride = mid_elems;
+    d.out_stride = out_elems;
+    for (size_t k = 0; k < steps.size(); ++k) {
+      const AxisStep& s = steps[k];
+      const int64_t L = s.combo == mb::K_CPLX ? s.N : s.N / 2;
+      AxisParams ap = base_params();
+      set_kind_tables(ap, s.combo, s.N);
+      mb::NdAxis& x = d.ax[k];
+      x.combo = s.combo;
+      x.log2L = ilog2(L);
+      x.nb = int(s.outer / howmany * s.inner);
+      x.inner = (int)s.inner;
+      x.in_row = (int)s.in_row;
+      x.out_row = (int)s.out_row;
+      x.flags = s.flags;
+      x.tw = tab(TB_TW, L);
+      x.t1 = ap.t1;
+      x.t2 = ap.t2;
+      x.n_tw = (int)L;
+      x.n_t1 = s.combo == mb::K_R2C ? table_entries(TB_RFT, s.N)
+               : (s.combo == mb::K_DCT2 || s.combo == mb::K_DCT3) ? table_entries(TB_T23, s.N)
+               : s.combo == mb::K_T4                              ? table_entries(TB_T4PRE, s.N)
+                                                                  : 0;
+      x.n_t2 = (s.combo == mb::K_C2R || s.combo == mb::K_DCT2 || s.combo == mb::K_DCT3) ? table_entries(TB_RFT, s.N)
+               : s.combo == mb::K_T4 ? table_entries(TB_T4POST, s.N)
+                                     : 0;
+      d.table_elems += x.n_tw + x.n_t1 + x.n_t2;
+    }
+    // CTAs of 64 threads while one round of 8 points per thread covers the array
+    ln.block = 64;
+    while (int(ln.block) < mb::kNdMaxThreads && int64_t(mb::kNdCluster) * ln.block * 8 < work) ln.block *= 2;
+    ln.smem = mb::nd_smem((int)ln.block, d.table_elems);
+    if (ln.smem > (size_t)dev_max_smem) return false;
+    if (!a->host_only && !ensure_smem_attr(ln.fn, ln.smem)) {
+      ok = false;
+      return true;
+    }
+    if (mid_buf != BUF_Y) need(mid_buf, size_t(mid_elems * howmany) * sizeof(cpx));
+    ln.nd = true;
+    ln.grid = unsigned(howmany * mb::kNdCluster);
+    ln.in_buf = BUF_X;
+    ln.mid_buf = mid_buf;
+    ln.out_buf = BUF_Y;
+    ln.in_c = complex_in(steps.front().combo);
+    ln.out_c = complex_out(steps.back().combo);
+    ln.vec_in = steps.front().combo == mb::K_R2C;
+    ln.vec_out = steps.back().combo == mb::K_C2R;
+    ln.nd_in = in_elems * howmany;
+    ln.nd_out = out_elems * howmany;
+    ln.combo = steps.front().combo;
+    ln.bytes = double(ln.nd_in) * (ln.in_c ? sizeof(cpx) : sizeof(real)) +
+               double(ln.nd_out) * (ln.out_c ? sizeof(cpx) : sizeof(real));
+    std::string shape;
+    for (const AxisStep& s : steps) shape += (shape.empty() ? "" : ",") + std::to_string(s.N);
+    char buf[160];
+    snprintf(buf, sizeof(buf), "nd_pass<%s,axes %s> batch=%lld", combo_name(steps.front().combo), shape.c_str(),
+             (long long)howmany);
+    ln.label = buf;
+    prog->launches.push_back(ln);
+    return true;
+  }
+
   void plan_axis(const AxisStep& s) {
     const size_t R_ = sizeof(real), C_ = sizeof(cpx);
     if (s.N == 1) {
@@ -1835,6 +1950,50 @@ bool build_program(minfft_aux* a, int op, int howmany, bool alias, Program* prog
     return cur;
   };
 
+  // Small multi-dimensional arrays in one launch.  (The real DFT and its
+  // inverse in place go through T1: every input row is read before the last
+  // step writes, but only within one array, and another array's input could
+  // lie under this one's larger output.)
+  if (nd > 2 && !(alias && howmany > 1 && (op == MINFFT_B200_REALDFT || op == MINFFT_B200_INVREALDFT))) {
+    const bool inverse = op == MINFFT_B200_INVDFT || op == MINFFT_B200_INVREALDFT;
+    const bool dft = op == MINFFT_B200_DFT || op == MINFFT_B200_INVDFT;
+    const bool rdft = op == MINFFT_B200_REALDFT || op == MINFFT_B200_INVREALDFT;
+    const int64_t N = D[nd - 1], K = N / 2 + 1;
+    std::vector<int64_t> H(D);  // extents of the steps along the outer axes
+    if (rdft) H[nd - 1] = K;
+    auto step = [&](int combo, size_t ax, int flags) {
+      AxisStep s{};
+      s.combo = combo;
+      s.N = D[ax];
+      s.outer = prod(H, 0, ax);
+      s.inner = prod(H, ax + 1, nd);
+      s.in_row = s.out_row = s.N * s.inner;
+      if (combo == mb::K_R2C) s.out_row = K;
+      if (combo == mb::K_C2R) s.in_row = K;
+      s.flags = flags;
+      return s;
+    };
+    int kind = mb::K_CPLX, fl = inverse ? (mb::F_CONJ_IN | mb::F_CONJ_OUT) : 0;
+    if (!dft && !rdft) {
+      kind = mb::K_T4;
+      if (op == MINFFT_B200_DCT2 || op == MINFFT_B200_DST2) kind = mb::K_DCT2;
+      if (op == MINFFT_B200_DCT3 || op == MINFFT_B200_DST3) kind = mb::K_DCT3;
+      if (op == MINFFT_B200_DST2 || op == MINFFT_B200_DST3 || op == MINFFT_B200_DST4) fl = mb::F_DST;
+    }
+    std::vector<AxisStep> steps;
+    for (size_t ax = nd - 1; ax >= 1; --ax)
+      steps.push_back(step(rdft && ax == nd - 1 ? (inverse ? mb::K_C2R : mb::K_R2C) : kind, ax,
+                           rdft && ax == nd - 1 ? 0 : fl));
+    if (op == MINFFT_B200_INVREALDFT) std::reverse(steps.begin(), steps.end());
+    const int64_t reals = prod(D, 1, nd), spec = prod(H, 1, nd);
+    // the steps between run in the output, or in T1: for the inverse real DFT,
+    // whose output cannot hold them, and the real DFT in place
+    const bool back = op == MINFFT_B200_INVREALDFT;
+    if (pl.plan_nd(steps, howmany, back ? spec : reals, rdft ? spec : reals, op == MINFFT_B200_REALDFT ? spec : reals,
+                   back || (alias && rdft) ? BUF_T1 : BUF_Y))
+      return pl.ok;
+  }
+
   switch (op) {
     case MINFFT_B200_DFT:
     case MINFFT_B200_INVDFT: {
@@ -2129,13 +2288,14 @@ bool launch_one(minfft_aux* a, const Launch& ln, void* const* bufs) {
     while (ch > 4 && (reinterpret_cast<uintptr_t>(ap.in) % ch) != 0) ch /= 2;
     ap.chunk = ch;
   }
-  if (ln.dctq >= 0) {
-    mb::DctqParams d = ln.dq;
+  if (ln.nd) {
+    mb::NdParams d = ln.ndp;
     d.in = bufs[ln.in_buf];
+    d.mid = bufs[ln.mid_buf];
     d.out = bufs[ln.out_buf];
-    d.mid = static_cast<cpx*>(bufs[ln.mid_buf]);
-    void* dargs[1] = {&d};
-    return enqueue(a, ln, dargs, ln.smem, "launch(dct split)");
+    d.flags = ap.flags & mb::F_VEC;
+    void* nargs[1] = {&d};
+    return enqueue(a, ln, nargs, ln.smem, "launch(nd)");
   }
   if (ln.dctq >= 0) {
     mb::DctqParams d = ln.dq;
@@ -2606,6 +2766,11 @@ void axis_batch_max(const AxisParams& ap, int64_t& oi, int64_t& oo) {
 
 Extent launch_extent(const Launch& ln) {
   Extent e{0, 0};
+  if (ln.nd) {  // whole arrays
+    e.in_max = ln.nd_in - 1;
+    e.out_max = ln.nd_out - 1;
+    return e;
+  }
   if (ln.dctq >= 0) {  // the whole real array and the whole block array
     const int64_t reals = ln.dq.H * ln.dq.Nr * ln.dq.N, blocks = ln.dq.H * (ln.dq.Nr / 2) * ln.dq.N;
     e.in_max = (ln.in_c ? blocks : reals) - 1;
@@ -2742,7 +2907,7 @@ MB_EXPORT int minfft_b200_plan_selfcheck_precision(int op, int d, const int* Ns,
            (long long)((e.out_max + 1) * oe), ln.out_buf, cap[ln.out_buf]);
     if (ln.block < 1 || ln.block > 1024 || ln.grid < 1) fail("launch %zu: bad shape %u x %u", i, ln.grid, ln.block);
     if (!ln.is_line && !ln.stream && ln.block > 512) fail("launch %zu: block %u above launch bounds", i, ln.block);
-    if (!ln.is_line && !ln.stream && !ln.tcs && ln.dctq < 0 &&
+    if (!ln.is_line && !ln.stream && !ln.tcs && !ln.nd && ln.dctq < 0 &&
         ln.block != unsigned(ln.ap.cpb * (ln.L / std::min(ln.radix, std::max(ln.L, 1)))))
       fail("launch %zu: block %u is not cpb x L/R", i, ln.block);
     if (ln.smem > size_t(di.max_smem)) fail("launch %zu: %zu bytes of shared memory", i, ln.smem);
@@ -2750,7 +2915,15 @@ MB_EXPORT int minfft_b200_plan_selfcheck_precision(int op, int d, const int* Ns,
                                                                  (ln.in_buf == BUF_Y && ln.out_buf == BUF_X)));
     if (alias_io && (ln.hbm_pass || (ln.is_line && ln.combo != mb::LK_UNIT)))
       fail("launch %zu (%s): runs in place but cannot", i, ln.label.c_str());
-    if (!ln.is_line && !ln.pipe && !ln.tc && !ln.stream && !ln.stream_rows && ln.dctq < 0 && ln.grid > 0 &&
+    if (ln.nd) {
+      const int64_t n = int64_t(ln.grid) / mb::kNdCluster;
+      const int64_t mid = ln.ndp.mid_stride * n * int64_t(ln.mid_buf == BUF_Y ? oe : sizeof(cpx));
+      if (ln.smem != mb::nd_smem((int)ln.block, ln.ndp.table_elems) || ln.grid % mb::kNdCluster ||
+          ln.block > unsigned(mb::kNdMaxThreads) || ln.block % 64 || size_t(mid) > cap[ln.mid_buf] ||
+          ln.ndp.in_stride * n != ln.nd_in || ln.ndp.out_stride * n != ln.nd_out)
+        fail("launch %zu (%s): shape, buffers or strides", i, ln.label.c_str());
+    }
+    if (!ln.is_line && !ln.pipe && !ln.tc && !ln.stream && !ln.stream_rows && !ln.nd && ln.dctq < 0 && ln.grid > 0 &&
         int64_t(ln.grid) * ln.ap.cpb < ln.ap.nbatch)
       fail("launch %zu: grid does not cover the batch", i);
     if (ln.stream_rows) {
@@ -2877,7 +3050,7 @@ MB_EXPORT int minfft_b200_autotune(minfft_aux* a, int op, int howmany, int reps)
   if (!p0) return g_err ? g_err : MINFFT_B200_ECUDA;
   std::vector<TuneKey> keys;
   for (const Launch& ln : p0->launches)
-    if (!ln.is_line && !ln.tc && ln.dctq < 0) keys.push_back(ln.key);
+    if (!ln.is_line && !ln.tc && !ln.nd && ln.dctq < 0) keys.push_back(ln.key);
   const size_t in_b = size_t(io_bytes(a, op, false)) * howmany, out_b = size_t(io_bytes(a, op, true)) * howmany;
   void *x = nullptr, *y = nullptr;
   if (!cuda_ok(cudaMalloc(&x, in_b), "cudaMalloc(autotune)")) return g_err;
