@@ -362,38 +362,25 @@ __device__ __forceinline__ bool rows_staged_in(const AxisParams& p) { return !p.
 __device__ __forceinline__ bool rows_staged_out(const AxisParams& p) { return !p.colmode && p.out_k == 1; }
 
 // ------------------------------------------------- root progressions
-// W^(g0 + r*D), r < R, for the root table pair (hi, lo) of W: each table
-// root is hi[e >> lobits] * lo[e & (2^lobits - 1)].  Three table roots per
-// thread (W^g0, W^D, W^4D); at(r) forms the rest as at most two products, as
-// the Stockham passes form theirs (apply_root_powers), just before use so
-// that only the seven factors stay live.  Every exponent g0 + r*D must lie
-// inside the tables; exponents are 32-bit (the planner keeps the tables
-// below 2^32 roots).
-template <int R>
+// The roots of a fused chain pass, W^(g0 + r*D) for a thread's elements r < R:
+// W^g0 from the table pair (hi, lo) of W -- hi[e >> lobits] * lo[e & (2^lobits
+// - 1)] -- and W^D.  The thread's elements are a whole Lt/R points apart
+// whatever the pass (TPT strides of Lt/L), so W^(r*D) does not depend on the
+// length: it is the 128th root of unity w_128^(r*K/R), a constant operand,
+// with K = 16, 32 or 64 for W of 8 Lt, 4 Lt (or w_16Lt^4) or 2 Lt.  (Formed
+// per thread from two more table roots, the steps took 40 of a thread's 700
+// instructions and its registers: the first pass of the DCT-4 of 2^24 points
+// in f32 went from 44 to 40 us.)  Exponents are 32-bit (the planner keeps
+// the tables below 2^32 roots).
+template <int R, int K>
 struct RootProgression {
-  cpx base, d1, d2, d3, d4, d8, d12;
+  cpx base;
   __device__ __forceinline__ RootProgression(const cpx* __restrict__ hi, const cpx* __restrict__ lo, int lobits,
-                                             uint32_t g0, uint32_t D) {
-    const uint32_t lomask = (1u << lobits) - 1u;
-    auto root = [&](uint32_t e) { return cmul(ldg(hi + (e >> lobits)), ldg(lo + (e & lomask))); };
-    base = root(g0);
-    d1 = R > 1 ? root(D) : czero();
-    d2 = cmul(d1, d1);
-    d3 = cmul(d2, d1);
-    d4 = R > 4 ? root(4 * D) : czero();
-    d8 = cmul(d4, d4);
-    d12 = cmul(d8, d4);
-  }
+                                             uint32_t g0)
+      : base(cmul(ldg(hi + (g0 >> lobits)), ldg(lo + (g0 & ((1u << lobits) - 1u))))) {}
   __device__ __forceinline__ cpx at(int r) const {
-    const int lo2 = r & 3, hi2 = r >> 2;
-    cpx t = base;
-    if (hi2 == 1) t = cmul(t, d4);
-    if (hi2 == 2) t = cmul(t, d8);
-    if (hi2 == 3) t = cmul(t, d12);
-    if (lo2 == 1) t = cmul(t, d1);
-    if (lo2 == 2) t = cmul(t, d2);
-    if (lo2 == 3) t = cmul(t, d3);
-    return t;
+    const int m = r * K / R;  // below 64
+    return m < 32 ? cmul(base, w128(m)) : cmul_negi(cmul(base, w128(m - 32)));
   }
 };
 
@@ -408,15 +395,16 @@ struct RootProgression {
 template <int L, int R>
 __device__ __forceinline__ void hbm_pretwiddle(cpx (&v)[R], const AxisParams& p, int64_t b0, int j) {
   constexpr int TPT = L / R;
-  const int64_t q = udiv(b0, p.st_div) & (p.st_ns - 1);
-  const int64_t lomask = (int64_t(1) << p.st_lobits) - 1;
-  auto root = [&](int64_t g) { return cmul(ldg(p.st_hi + (g >> p.st_lobits)), ldg(p.st_lo + (g & lomask))); };
+  // exponents stay below Lt <= 2^31: 32-bit
+  const uint32_t q = uint32_t(udiv(b0, p.st_div)) & uint32_t(p.st_ns - 1);
+  const uint32_t lomask = (1u << p.st_lobits) - 1u;
+  auto root = [&](uint32_t g) { return cmul(ldg(p.st_hi + (g >> p.st_lobits)), ldg(p.st_lo + (g & lomask))); };
   if constexpr (R < 4) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = cmul(v[r], root((q * (j + r * TPT)) << p.st_shift));
+    for (int r = 0; r < R; ++r) v[r] = cmul(v[r], root((q * uint32_t(j + r * TPT)) << p.st_shift));
   } else {
-    const int64_t gd = (q * TPT) << p.st_shift;
-    const cpx base = root((q * j) << p.st_shift);
+    const uint32_t gd = (q * uint32_t(TPT)) << p.st_shift;
+    const cpx base = root((q * uint32_t(j)) << p.st_shift);
     const cpx d1 = root(gd);
     const cpx d2 = cmul(d1, d1);
     const cpx d3 = cmul(d2, d1);
@@ -943,8 +931,7 @@ struct LoadT4Chain {
     }
     __syncthreads();
     // w_2N^g for g = g0 + r*TPT*in_n
-    const RootProgression<R> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(b1 * p.is1 + int64_t(x.j) * p.in_n),
-                                uint32_t(int64_t(TPT) * p.in_n));
+    const RootProgression<R, 32> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(b1 * p.is1 + int64_t(x.j) * p.in_n));
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = cmul(ew.at(r), cmk(a[r], get[r * TPT]));
   }
@@ -1095,7 +1082,7 @@ struct LoadDCT2Line {
 // the roots w_N^g.
 template <int L, int R>
 __device__ __forceinline__ void pack_tile(const Ctx& x, const Tile& t, const Mirror& mi, bool zero, cpx k0,
-                                          const RootProgression<R>& fw, cpx (&v)[R]) {
+                                          const RootProgression<R, 64>& fw, cpx (&v)[R]) {
   constexpr int TPT = L / R;
   scatter_mirror<L, R>(v, x, mi, t);
   __syncthreads();
@@ -1119,7 +1106,7 @@ struct LoadDCT3Line {
     const int64_t N = p.kn;
     const Mirror mi = mirror_spectrum<TPT>(p, x, ci.i);
     const bool zero = mi.turned;  // element 0 is point 0: x_0 and x_Lt
-    const int64_t g0 = ci.i + int64_t(x.j) * p.in_n, st = int64_t(TPT) * p.in_n;
+    const int64_t g0 = ci.i + int64_t(x.j) * p.in_n;
     const int64_t sa = dst ? -p.in_n : p.in_n;
     Walk<const real, false, TPT> wa(dst ? ci.in + (N - 1 - g0) : ci.in + g0, sa);
     Walk<const real, false, -TPT> wb(dst ? ci.in + (g0 - 1) : ci.in + (N - g0), sa);
@@ -1132,14 +1119,14 @@ struct LoadDCT3Line {
     const real r2 = real(1.414213562373095048801688724209698079);
     const cpx k0 = cmk(v[0].x + r2 * v[0].y, -(v[0].x - r2 * v[0].y));
     {
-      const RootProgression<R> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0), uint32_t(st));
+      const RootProgression<R, 16> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0));
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const cpx e = ew.at(r);
         v[r] = cmk(v[r].x * e.x - v[r].y * e.y, -(v[r].x * e.y) - v[r].y * e.x);
       }
     }
-    const RootProgression<R> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(4 * g0), uint32_t(4 * st));
+    const RootProgression<R, 64> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(4 * g0));
     pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
   }
 };
@@ -1157,7 +1144,7 @@ struct LoadC2RLine {
     const cpx* in = static_cast<const cpx*>(p.in) + line * p.k_in_line;
     const Mirror mi = mirror_spectrum<TPT>(p, x, i);
     const bool zero = mi.turned;
-    const int64_t g0 = i + int64_t(x.j) * p.in_n, st = int64_t(TPT) * p.in_n;
+    const int64_t g0 = i + int64_t(x.j) * p.in_n;
     Walk<const cpx, false, TPT> w(in + g0, p.in_n);
 #pragma unroll
     for (int r = 0; r < R; ++r, w.step()) v[r] = __ldcs(w.q);
@@ -1166,7 +1153,7 @@ struct LoadC2RLine {
       const cpx zl = in[p.kn / 2];
       k0 = cmk(v[0].x + zl.x, -(v[0].x - zl.x));
     }
-    const RootProgression<R> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0), uint32_t(st));
+    const RootProgression<R, 64> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0));
     pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
   }
 };
@@ -1211,6 +1198,19 @@ struct StoreCplx {
     __syncthreads();
     scatter_natural<L, R>(v, x.j, x.c, t);
     __syncthreads();
+    if ((blockDim.x & (L - 1)) == 0 && p.out_k == 1) {
+      // whole transforms per sweep of the CTA: a thread keeps its output k
+      const int k = threadIdx.x & (L - 1), step = int(blockDim.x) / L;
+      int c = threadIdx.x / L;
+      const cpx* q = t.s + t.idx(c, k);
+      cpx* o = out + k;
+      for (; c < to.nvalid; c += step, q += step * t.lp) {
+        cpx w = *q;
+        if (cj) w.y = -w.y;
+        o[to.out_off[c]] = w;
+      }
+      return;
+    }
     const int total = to.nvalid * L;
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
       const int c = e / L, k = e - c * L;
@@ -1537,8 +1537,7 @@ struct StoreT4Chain {
     real* sb = reinterpret_cast<real*>(t.s);
     const bool vec = (reinterpret_cast<uintptr_t>(out) % sizeof(cpx)) == 0;
     // g_2m = w_8N^(4m+1) for m = m0 + r*TPT*out_k
-    const RootProgression<R> gw(p.t1, p.t2, p.kbits, uint32_t(4 * (x.oout + int64_t(x.j) * p.out_k) + 1),
-                                uint32_t(4 * int64_t(TPT) * p.out_k));
+    const RootProgression<R, 32> gw(p.t1, p.t2, p.kbits, uint32_t(4 * (x.oout + int64_t(x.j) * p.out_k) + 1));
     __syncthreads();  // the last Stockham exchange has finished with the tile
     // a slot holds 2*lp >= 2L reals: the mirror's values below L, its own above
     real* own = sb + x.c * 2 * t.lp + x.j;
@@ -1576,8 +1575,8 @@ struct StoreR2CLine {
     constexpr int TPT = L / R;
     cpx* out = static_cast<cpx*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
     const Mirror mi = mirror_spectrum<TPT>(p, x, x.oout);
-    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
-    const RootProgression<R> fw(p.t1, p.t2, p.kbits, uint32_t(m0), uint32_t(st));
+    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k;
+    const RootProgression<R, 64> fw(p.t1, p.t2, p.kbits, uint32_t(m0));
     __syncthreads();  // the last Stockham exchange has finished with the tile
     scatter_mirror<L, R>(v, x, mi, t);
     __syncthreads();
@@ -1609,7 +1608,7 @@ struct StoreDCT2Line {
     const bool dst = (p.flags & F_DST) != 0;
     const int64_t N = p.kn;
     const Mirror mi = mirror_spectrum<TPT>(p, x, x.oout);
-    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k, st = int64_t(TPT) * p.out_k;
+    const int64_t m0 = x.oout + int64_t(x.j) * p.out_k;
     __syncthreads();  // the last Stockham exchange has finished with the tile
     scatter_mirror<L, R>(v, x, mi, t);
     __syncthreads();
@@ -1617,11 +1616,11 @@ struct StoreDCT2Line {
     const real y0 = 2 * (v[0].x + v[0].y), yl = r2 * (v[0].x - v[0].y);
     const cpx* zm = slot_at<TPT>(t, mi.slot, mi.jm);
     {
-      const RootProgression<R> fw(p.t1, p.t2, p.kbits, uint32_t(4 * m0), uint32_t(4 * st));
+      const RootProgression<R, 64> fw(p.t1, p.t2, p.kbits, uint32_t(4 * m0));
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = unpack_one2(v[r], zm[nat_off<TPT>(R - 1 - r)], fw.at(r));
     }
-    const RootProgression<R> ew(p.t1, p.t2, p.kbits, uint32_t(m0), uint32_t(st));
+    const RootProgression<R, 16> ew(p.t1, p.t2, p.kbits, uint32_t(m0));
     const int64_t sa = dst ? -p.out_k : p.out_k;
     Walk<real, false, TPT> wa(dst ? out + (N - 1 - m0) : out + m0, sa);
     Walk<real, false, -TPT> wb(dst ? out + (m0 - 1) : out + (N - m0), sa);
