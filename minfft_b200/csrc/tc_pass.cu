@@ -560,7 +560,8 @@ __global__ void __launch_bounds__(16 * TB, TB == 8 ? 4 : 2) tc256_kernel(const A
 // is bound by its instructions and their latency (tensor pipe under 10%
 // busy), so resident warps count most: 256^3, round trip, 424 us with two
 // stages held to the end of a tile (four CTAs), 391 so in FP16, 558 -> 491 in
-// BF16; with two stages 412 and 532.
+// BF16; with two stages 412 and 532.  Its prologue (operands, twiddles,
+// tensor memory) runs under the previous kernel's end: 391 -> 378.
 constexpr int kTcsW = kTcStreamTile;     // transforms per tile
 constexpr int kTcsNT = kTcStreamThreads; // threads
 constexpr int kTcsG = kTcsNT / 128;      // UMMA groups of 128 rows
@@ -735,8 +736,9 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 5 : 4) tc_stream_kerne
   const int64_t gpd = (p.d0 + W - 1) / W;
   const int64_t ntiles = p.ntiles;
 
-  pdl_wait();
-  pdl_release();
+  // Everything up to the first tile reads constant tables only and runs while
+  // the previous kernel drains.  (Its CTAs hold tensor memory until they end;
+  // the allocation waits for them at most.)
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      static_cast<uint32_t>(__cvta_generic_to_shared(tslot))),
@@ -814,7 +816,9 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 5 : 4) tc_stream_kerne
     }
   };
 
+  pdl_wait();
   for (int s = 0; s < S; ++s) issue(blockIdx.x + int64_t(s) * gridDim.x, s);
+  pdl_release();
 
   const bool cj_in = (p.flags & F_CONJ_IN) != 0, cj_out = (p.flags & F_CONJ_OUT) != 0;
   const bool rows_out = (p.flags & F_STAGE_ROWS) != 0;

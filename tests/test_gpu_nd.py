@@ -62,3 +62,31 @@ def test_batches_and_offsets(howmany, single):
 def test_which_shapes_take_one_launch(op, dims, single, one):
     _, rep, n = minfft_b200.engine(single).plan_selfcheck(op, dims)
     assert ("nd_pass" in rep and n == 1) == one, rep
+
+
+@pytest.mark.parametrize("single,dims,howmany", [(True, (64, 64, 64), 67), (False, (256, 8, 4096), 1)],
+                         ids=["f32-batch", "f64-3d"])
+def test_slabs_of_arrays_beyond_the_l2(single, dims, howmany):
+    """Complex arrays above 128 MiB run their inner axes slab by slab (the last
+    slab of the batch shorter than the others); the first, a middle and the
+    last array or plane against the oracle, in place too."""
+    eng = minfft_b200.engine(single)
+    _, _, n = eng.plan_selfcheck("dft", dims, howmany)
+    assert n > len(dims)
+    cdt = torch.complex64 if single else torch.complex128
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn((howmany,) + dims, dtype=cdt, device="cuda", generator=g)
+    y = torch.full_like(x, float("nan"))
+    plan = eng.plan("dft", dims)
+    plan.batch("dft", x.data_ptr(), y.data_ptr(), howmany)
+    torch.cuda.synchronize()
+    pick = (0, howmany // 2, howmany - 1) if howmany > 1 else (0,)
+    for i in pick:
+        ref = expected("dft", x[i].cpu().numpy(), dims)
+        assert rel_l2(y[i].cpu().numpy(), ref) <= tolerance(single, dims), i
+    plan.batch("invdft", y.data_ptr(), y.data_ptr(), howmany)
+    torch.cuda.synchronize()
+    plan.free()
+    scale = float(np.prod(dims))
+    err = (torch.linalg.vector_norm(y / scale - x) / torch.linalg.vector_norm(x)).item()
+    assert err <= 2 * tolerance(single, dims)
