@@ -150,7 +150,8 @@ __global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);  // one per stage
   volatile int* issued = reinterpret_cast<volatile int*>(smem + 128);  // last tile (by its ordinal) started into a stage
-  volatile int* bad = reinterpret_cast<volatile int*>(smem + 192);
+  volatile int* bad = reinterpret_cast<volatile int*>(smem + 192);  // a group gave up: the others stop waiting
+  volatile int* gbad = bad + 1;                                      // by group: its own exit
   unsigned char* stages = smem + kStreamHeader;
   const int S = p.cpb;  // stages
   const int G = blockDim.x / NT;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *bad = 0;
+    for (int i = 0; i < G; ++i) gbad[i] = 0;
   }
   __syncthreads();
   pdl_wait();
@@ -248,9 +250,9 @@ __global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 
   for (int k = g;; k += G) {
     const int64_t t = blockIdx.x + int64_t(k) * gridDim.x;
     if (t >= ntiles) break;
-    if (!arrived(k)) *bad = 1;
+    if (!arrived(k)) *bad = gbad[g] = 1;
     group_sync<NT>(g);
-    if (*bad) break;
+    if (gbad[g]) break;  // written by this group only, before its barrier: its threads agree
     cpx* tile = reinterpret_cast<cpx*>(stages + size_t(k % S) * p.stage_bytes);
     int64_t col0, b1, b2;
     tile_pos(t, col0, b1, b2);
