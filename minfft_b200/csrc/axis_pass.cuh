@@ -147,16 +147,21 @@ __device__ __forceinline__ void batch_offsets(const AxisParams& p, int64_t b, in
 // ------------------------------------------------------------ Stockham core
 // u[r] *= w^r for r = 1..RP-1 with w = tw[i1]: two table roots (w, w^4) per
 // sub-DFT, the other powers formed just before use as products of at most
-// four roundings, so only a handful of roots are live at a time.
-template <int RP>
+// four roundings, so only a handful of roots are live at a time.  The radix-8
+// kernels (kLoad) take w^2 and w^3 from the table too: they run where the
+// array is small and the loads hide, and 32- and 64-point lines then round
+// no more than radix 16 does (64 x 64 DCT-2 and -3 in single, error against
+// double: 3.8e-7 with products, 3.0e-7 with loads, 2.8e-7 at radix 16; the
+// time is the same).
+template <int RP, bool kLoad>
 __device__ __forceinline__ void apply_root_powers(cpx* u, const cpx* __restrict__ tw, int i1) {
   static_assert(RP <= 16, "radix up to 16");
   const cpx w1 = ldg(tw + i1);
   u[1] = cmul(u[1], w1);
   if constexpr (RP > 2) {
-    const cpx w2 = cmul(w1, w1);
+    const cpx w2 = kLoad ? ldg(tw + 2 * i1) : cmul(w1, w1);
     u[2] = cmul(u[2], w2);
-    const cpx w3 = cmul(w2, w1);
+    const cpx w3 = kLoad ? ldg(tw + 3 * i1) : cmul(w2, w1);
     u[3] = cmul(u[3], w3);
     if constexpr (RP > 4) {
       const cpx w4 = ldg(tw + 4 * i1);
@@ -192,7 +197,7 @@ __device__ __forceinline__ void pass_compute(cpx (&v)[R], int j, const cpx* __re
       const int jp = j + s * (L / R);
       const int q = jp & (NS - 1);
       constexpr int step = L / (NS * RP);
-      apply_root_powers<RP>(u, tw, q * step);
+      apply_root_powers<RP, R == 8>(u, tw, q * step);
     }
     fft_reg<RP>(u);
 #pragma unroll
