@@ -121,12 +121,13 @@ int minfft_b200_dft_noalloc(const void *x, void *y, int n, int inverse, void *st
  * a transform code (MINFFT_B200_*), its length n (1 .. 65536 for complex
  * transforms, 1 .. 131072 for the real ones) and device input and output
  * arrays (complex data aligned to its size).  Jobs are grouped by kind and
- * length into work items (up to 512*16/L short transforms per item; one item
- * per transform longer than 8192 complex points, which its CTA computes in
- * two passes through a private scratch slice) and handed out through an
- * atomic queue, largest items first.  The plan owns the root tables, the
- * queue and the scratch; execute only launches the captured graph on
- * `stream`.  Outputs of different jobs must not overlap their inputs. */
+ * length into work items (several transforms of up to 4096 complex points;
+ * one tile of 4096 points of a pass of a longer one) that persistent CTAs take
+ * from an atomic counter.  The plan owns the root tables, the counters and the
+ * scratch; execute only launches the captured graph on
+ * `stream`.  Outputs of different jobs must not overlap their inputs.  A
+ * device-side wait that ran out (see minfft_b200_device_status) makes the
+ * next execute of the batch return MINFFT_B200_ETIMEOUT. */
 typedef struct {
     int op;
     int n;

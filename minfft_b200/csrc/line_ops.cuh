@@ -1,12 +1,9 @@
 // Element-wise pre- and post-processing steps of real-data transforms whose
 // half-length complex DFT runs as several HBM passes, and the length-1 axis
 // steps, as device functions: Op::count(p) work items, Op::item(p, e) does
-// item e.  The steps the mixed-batch kernel runs as sweeps also come as
-// Op::load_at(p, it), which reads everything item it needs (data and roots)
-// into an Op::In, and Op::finish_at(p, it, in), which computes and stores:
-// a CTA that walks a line alone then issues the loads of several items
-// before any of their stores.  Used by the line kernels (line_kernels.cu)
-// and by the mixed-batch kernel (mixed.cu).
+// item e.  The paired steps split an item into load_at (everything it reads,
+// data and roots) and finish_at (computes and stores).  Used by the line
+// kernels (line_kernels.cu).
 //
 // Data layout: a batch of outer x inner lines along one axis; element n of
 // line (o, i) of the input sits at o*in_so + n*in_sn + i, of the output at
@@ -84,10 +81,6 @@ struct Op_dct2_pre {
   }
   static __device__ __forceinline__ ItemIdx index(const LineParams& p, int64_t e) {
     return split_item(e, p.inner, p.L);
-  }
-  static __device__ __forceinline__ In load(const LineParams& p, int64_t e) { return load_at(p, index(p, e)); }
-  static __device__ __forceinline__ void finish(const LineParams& p, int64_t e, const In& v) {
-    finish_at(p, index(p, e), v);
   }
   static __device__ __forceinline__ void item(const LineParams& p, int64_t e) {
     const ItemIdx it = index(p, e);
@@ -194,10 +187,6 @@ struct Op_c2r_pack {
   static __device__ __forceinline__ ItemIdx index(const LineParams& p, int64_t e) {
     return split_item(e, p.inner, p.L / 2 + 1);
   }
-  static __device__ __forceinline__ In load(const LineParams& p, int64_t e) { return load_at(p, index(p, e)); }
-  static __device__ __forceinline__ void finish(const LineParams& p, int64_t e, const In& v) {
-    finish_at(p, index(p, e), v);
-  }
   static __device__ __forceinline__ void item(const LineParams& p, int64_t e) {
     const ItemIdx it = index(p, e);
     finish_at(p, it, load_at(p, it));
@@ -243,10 +232,6 @@ struct Op_dct3_pack {
   static __device__ __forceinline__ ItemIdx index(const LineParams& p, int64_t e) {
     return split_item(e, p.inner, p.L / 2 + 1);
   }
-  static __device__ __forceinline__ In load(const LineParams& p, int64_t e) { return load_at(p, index(p, e)); }
-  static __device__ __forceinline__ void finish(const LineParams& p, int64_t e, const In& v) {
-    finish_at(p, index(p, e), v);
-  }
   static __device__ __forceinline__ void item(const LineParams& p, int64_t e) {
     const ItemIdx it = index(p, e);
     finish_at(p, it, load_at(p, it));
@@ -288,10 +273,6 @@ struct Op_r2c_unpack {
   }
   static __device__ __forceinline__ ItemIdx index(const LineParams& p, int64_t e) {
     return split_item(e, p.inner, p.L / 2 + 1);
-  }
-  static __device__ __forceinline__ In load(const LineParams& p, int64_t e) { return load_at(p, index(p, e)); }
-  static __device__ __forceinline__ void finish(const LineParams& p, int64_t e, const In& v) {
-    finish_at(p, index(p, e), v);
   }
   static __device__ __forceinline__ void item(const LineParams& p, int64_t e) {
     const ItemIdx it = index(p, e);
@@ -340,10 +321,6 @@ struct Op_dct2_post {
   static __device__ __forceinline__ ItemIdx index(const LineParams& p, int64_t e) {
     return split_item(e, p.inner, p.L / 2 + 1);
   }
-  static __device__ __forceinline__ In load(const LineParams& p, int64_t e) { return load_at(p, index(p, e)); }
-  static __device__ __forceinline__ void finish(const LineParams& p, int64_t e, const In& v) {
-    finish_at(p, index(p, e), v);
-  }
   static __device__ __forceinline__ void item(const LineParams& p, int64_t e) {
     const ItemIdx it = index(p, e);
     finish_at(p, it, load_at(p, it));
@@ -364,10 +341,6 @@ struct Op_dct3_post {
   }
   static __device__ __forceinline__ ItemIdx index(const LineParams& p, int64_t e) {
     return split_item(e, p.inner, p.L);
-  }
-  static __device__ __forceinline__ In load(const LineParams& p, int64_t e) { return load_at(p, index(p, e)); }
-  static __device__ __forceinline__ void finish(const LineParams& p, int64_t e, const In& v) {
-    finish_at(p, index(p, e), v);
   }
   static __device__ __forceinline__ void item(const LineParams& p, int64_t e) {
     const ItemIdx it = index(p, e);
