@@ -178,7 +178,7 @@ __device__ __noinline__ void run_small(const Params& mp, const Item& it, unsigne
   TileOffsets to{nullptr, nullptr, it.count};
   cpx v[R];
   LoadOp::template run<L, R>(p, x, t, v);
-  run_passes<L, R, 1>(v, j, c, t, p.tw);
+  run_passes<L, R, 1, KeepsTile<LoadOp>::value>(v, j, c, t, p.tw);
   StoreOp::template run<L, R>(p, x, t, to, v);
 }
 
@@ -309,7 +309,7 @@ __device__ __noinline__ void run_tile(const Params& mp, const Item& it, unsigned
   x.active = true;
   cpx v[R];
   Ld::template run<RP, R>(p, x, t, v);
-  run_passes<RP, R, 1>(v, x.j, x.c, t, p.tw);
+  run_passes<RP, R, 1, KeepsTile<Ld>::value>(v, x.j, x.c, t, p.tw);
   St::template run<RP, R>(p, x, t, to, v);
 }
 

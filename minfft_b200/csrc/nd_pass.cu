@@ -77,7 +77,7 @@ __device__ __noinline__ void nd_axis(const NdAxis& a, const cpx* tables, const v
     x.oout = b0 + b1 * a.out_row;
     cpx v[R];
     LoadOp::template run<L, R>(p, x, t, v);
-    run_passes<L, R, 1>(v, x.j, x.c, t, p.tw);
+    run_passes<L, R, 1, KeepsTile<LoadOp>::value>(v, x.j, x.c, t, p.tw);
     StoreOp::template run<L, R>(p, x, t, to, v);
     __syncthreads();  // the tile is free
   }
