@@ -420,9 +420,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) mixed_kernel(const __gri
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i), "l"(src + i) : "memory");
     }
   };
+  // A batch without long transforms has no waits, so any CTA may have any item:
+  // each starts with the one of its own index, and no CTA waits for a grid of
+  // atomics on the counter first (300 jobs of 2^4 .. 2^10 points in f32 14.3 us,
+  // 10.3 so; 11054 jobs 23.5 / 18.5; 4000 of 2^4 .. 2^11 in f64 24.4 / 18.9).
+  const unsigned dealt = mp.nbig ? 0u : gridDim.x;
   if (threadIdx.x == 0) {
-    fetch(int(atomicAdd(mp.counter, 1u)), 0);
-    ahead = atomicAdd(mp.counter, 1u);
+    fetch(int(mp.nbig ? atomicAdd(mp.counter, 1u) : blockIdx.x), 0);
+    ahead = dealt + atomicAdd(mp.counter, 1u);
   }
   for (int n = 0;; ++n) {
     if (threadIdx.x == 0) asm volatile("cp.async.wait_all;" ::: "memory");
@@ -431,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) mixed_kernel(const __gri
     const Item it = s_desc[n & 1];
     if (threadIdx.x == 0) {
       fetch(int(ahead), (n + 1) & 1);
-      ahead = atomicAdd(mp.counter, 1u);
+      ahead = dealt + atomicAdd(mp.counter, 1u);
     }
     bool ok = true;
     if (it.kind >= kFirst) {
