@@ -318,10 +318,10 @@ struct minfft_aux {
   void* bufs[BUF_COUNT] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t buf_bytes[BUF_COUNT] = {0, 0, 0, 0, 0, 0};
   std::map<std::tuple<int, int, int>, Program> programs;  // (op, howmany, alias)
-  // the program of the last call (programs' nodes stay where they are until
-  // the map is cleared)
-  std::tuple<int, int, int> last_key{-1, 0, 0};
-  Program* last_program = nullptr;
+  // the entry of the last call (the map's nodes stay where they are until it
+  // is cleared): one pointer to key and program together, so that a thread
+  // sharing the plan never takes another call's program for its own key
+  std::atomic<std::map<std::tuple<int, int, int>, Program>::value_type*> last{nullptr};
   int precision = MINFFT_B200_PREC_FP32;  // arithmetic of the 256-point complex passes
   void* tc_mem = nullptr;                 // tensor-core B operands (both formats)
   int* dev_status = nullptr;              // set by kernels whose bounded device-side wait ran out
@@ -2208,11 +2208,11 @@ bool ensure_buffer(minfft_aux* a, int buf, size_t bytes) {
 
 Program* get_program(minfft_aux* a, int op, int howmany, bool alias) {
   auto key = std::make_tuple(op, howmany, alias ? 1 : 0);
-  if (a->last_program && a->last_key == key) return a->last_program;
+  if (auto* last = a->last.load(std::memory_order_acquire); last && last->first == key) return &last->second;
   auto it = a->programs.find(key);
   if (it != a->programs.end()) {
-    a->last_key = key;
-    return a->last_program = &it->second;
+    a->last.store(&*it, std::memory_order_release);
+    return &it->second;
   }
   Program prog;
   if (!build_program(a, op, howmany, alias, &prog)) return nullptr;
@@ -2751,7 +2751,7 @@ MB_EXPORT int minfft_b200_set_precision(minfft_aux* a, int mode) {
   if (a->precision != mode) {
     a->precision = mode;
     a->programs.clear();
-    a->last_program = nullptr;
+    a->last.store(nullptr);
   }
   return MINFFT_B200_OK;
 }
@@ -3205,7 +3205,7 @@ MB_EXPORT int minfft_b200_autotune(minfft_aux* a, int op, int howmany, int reps)
     for (auto& kv : best) g_tune[kv.first] = kv.second;
   }
   a->programs.clear();
-  a->last_program = nullptr;
+  a->last.store(nullptr);
   return rc;
 }
 
