@@ -168,8 +168,8 @@ int minfft_b200_set_precision(minfft_aux *a, int mode);
 int minfft_b200_get_precision(const minfft_aux *a);
 /* Waits for plan `a`'s stream and reports whether one of its kernels gave up
  * on a bounded device-side wait (a tensor-core pass waiting for its matrix
- * operations) since the previous call: MINFFT_B200_ETIMEOUT, and that
- * launch's output is incomplete.  Clears the record.  minfft_b200_tc_status
+ * operations, a streamed pass waiting for a tile) since the previous call:
+ * MINFFT_B200_ETIMEOUT, and that launch's output is incomplete.  Clears the record.  minfft_b200_tc_status
  * is the same call. */
 int minfft_b200_device_status(const minfft_aux *a);
 int minfft_b200_tc_status(const minfft_aux *a);
@@ -228,6 +228,12 @@ long long minfft_b200_test_device_alloc_count(void);
  * minfft_b200_device_status (MINFFT_B200_ETIMEOUT).  polls = 0 restores
  * normal launches.  No fault is involved; meant for tests. */
 int minfft_b200_test_tc_withhold(long long polls);
+/* Stall injection for the streamed column pass (no counterpart in the
+ * reference).  With stall_us > 0, every such launch issued afterwards holds
+ * back the refill after each thread block's first tile for about that many
+ * microseconds; with polls > 0, its waits are limited to that many polls.
+ * Zeros restore normal launches.  No fault is involved; meant for tests. */
+int minfft_b200_test_stream_stall(long long stall_us, long long polls);
 
 #ifdef __cplusplus
 } /* extern "C" */

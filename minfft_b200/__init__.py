@@ -120,6 +120,8 @@ class Engine(MinfftLibrary):
         L.minfft_b200_test_device_alloc_count.restype = i64
         L.minfft_b200_test_tc_withhold.argtypes = [i64]
         L.minfft_b200_test_tc_withhold.restype = i32
+        L.minfft_b200_test_stream_stall.argtypes = [i64, i64]
+        L.minfft_b200_test_stream_stall.restype = i32
 
     # --------------------------------------------------------- errors
     def last_error(self) -> int:

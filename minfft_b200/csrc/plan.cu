@@ -90,6 +90,8 @@ std::atomic<long long> g_fail_at{0};
 // Test hook: > 0 makes tensor-core launches withhold their first commit and
 // give up after this many polls (see mb::TcParams).
 std::atomic<long long> g_tc_withhold{0};
+// Test hook of the streamed column pass (see mb::StreamTest).
+std::atomic<long long> g_stream_stall_us{0}, g_stream_polls{0};
 
 }  // namespace
 
@@ -2408,7 +2410,8 @@ bool launch_one(minfft_aux* a, const Launch& ln, void* const* bufs) {
       set_error(MINFFT_B200_EINVAL, "complex input not aligned to its size");
       return false;
     }
-    void* sargs[2] = {&ap, &map};
+    mb::StreamTest test{g_stream_stall_us.load(), g_stream_polls.load()};
+    void* sargs[3] = {&ap, &map, &test};
     return enqueue(a, ln, sargs, ln.smem, "launch(stream)");
   }
   if (ln.tc) {
@@ -3300,5 +3303,15 @@ MB_EXPORT int minfft_b200_test_tc_withhold(long long polls) {
     return MINFFT_B200_EINVAL;
   }
   g_tc_withhold.store(polls);
+  return MINFFT_B200_OK;
+}
+
+MB_EXPORT int minfft_b200_test_stream_stall(long long stall_us, long long polls) {
+  if (stall_us < 0 || polls < 0) {
+    set_error(MINFFT_B200_EINVAL, "stall and poll count must be >= 0");
+    return MINFFT_B200_EINVAL;
+  }
+  g_stream_stall_us.store(stall_us);
+  g_stream_polls.store(polls);
   return MINFFT_B200_OK;
 }

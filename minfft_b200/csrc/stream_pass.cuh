@@ -35,7 +35,11 @@
 // copy the tile with cp.async and the barrier counts their arrivals instead.
 //
 // Waits are bounded: a wait that runs out sets *status, the groups stop,
-// wait (bounded) for the copies in flight and return.
+// wait (bounded) for the copies in flight and return.  A group waiting for
+// issued[] waits for another group, which may itself be waiting for a slow
+// copy (managed memory coming from the host), so it has to outlast that wait:
+// 4 us between its polls, as long as a poll of an mbarrier that is not done
+// suspends the thread (measured), and twice as many polls.
 #pragma once
 
 #include <cuda.h>
@@ -45,6 +49,9 @@
 namespace mb {
 
 constexpr long long kStreamSpinLimit = 1LL << 22;
+// Polls of issued[] before a waiting group sleeps between them: about 100 us,
+// longer than a tile takes.
+constexpr int kIssuedSpins = 4096;
 
 __host__ __device__ constexpr int stream_cols(int L) {
   return L >= 512 ? int(128 / sizeof(cpx)) : int(256 / sizeof(cpx));
@@ -139,9 +146,16 @@ __host__ __device__ constexpr int stream_max_groups(int L, int R) {
   return nt < 32 ? 1 : (kStreamThreads / nt < 8 ? (kStreamThreads / nt < 1 ? 1 : kStreamThreads / nt) : 8);
 }
 
+// Test hook (zero in normal launches): stall_us > 0 makes group 0 hold back
+// the refill after its CTA's first tile for about that long; polls > 0 limits
+// the waits to that many polls.
+struct StreamTest {
+  long long stall_us, polls;
+};
+
 template <int L, int R>
 __global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 1)
-    stream_pass_kernel(const AxisParams p, const __grid_constant__ CUtensorMap tmap) {
+    stream_pass_kernel(const AxisParams p, const __grid_constant__ CUtensorMap tmap, const StreamTest q) {
   constexpr int W = stream_cols(L);
   constexpr int TPT = L / R;
   constexpr int NT = stream_group(L, R);
@@ -234,10 +248,12 @@ __global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 
   // completes.
   auto arrived = [&](int k) {
     const int s = k % S;
-    long long n = 0;
-    while (issued[s] != k)
-      if (++n > kStreamSpinLimit || *bad) return false;
-    return smbar_wait(mbar0 + 8 * s, uint32_t(k / S) & 1u, kStreamSpinLimit);
+    const long long limit = q.polls > 0 ? q.polls : kStreamSpinLimit;
+    for (long long n = 0; issued[s] != k; ++n) {
+      if (n > 2 * limit || *bad) return false;
+      if (n >= kIssuedSpins) __nanosleep(4000);
+    }
+    return smbar_wait(mbar0 + 8 * s, uint32_t(k / S) & 1u, limit);
   };
 
   // the first S tiles: group 0 starts them all
@@ -267,6 +283,8 @@ __global__ void __launch_bounds__(stream_group(L, R) * stream_max_groups(L, R), 
     }
     if (p.st_ns > 1) hbm_pretwiddle<L, R>(v, p, col, j);
     auto refill = [&] {
+      if (k == 0)
+        for (long long n = 0; n < q.stall_us; ++n) __nanosleep(1000);
       group_sync<NT>(g);
       issue(k + S);
     };
