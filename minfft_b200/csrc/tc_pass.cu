@@ -969,7 +969,11 @@ __global__ void __launch_bounds__(kTcsNT, FMT == TC_F16 ? 5 : 4) tc_stream_kerne
   if (!ok) {
     if (tid == 0 && q.status) atomicExch(q.status, 1);
     if (pending) mbar_wait(mma_bar, mph);
-    for (int k = 0; k < S + (refilled ? 1 : 0); ++k, ++it, t += gridDim.x) {  // copies in flight
+    if (refilled) {  // this tile's copy has been used and its stage's barrier is a phase on: the next one's is in flight
+      ++it;
+      t += gridDim.x;
+    }
+    for (int k = 0; k < S; ++k, ++it, t += gridDim.x) {  // copies in flight
       if (t >= ntiles) break;
       smbar_wait(bar0 + 8 * (it % S), uint32_t(it / S) & 1u, kStreamSpinLimit);
     }
