@@ -234,6 +234,11 @@ int minfft_b200_test_tc_withhold(long long polls);
  * microseconds; with polls > 0, its waits are limited to that many polls.
  * Zeros restore normal launches.  No fault is involved; meant for tests. */
 int minfft_b200_test_stream_stall(long long stall_us, long long polls);
+/* Timeout injection for mixed batches.  With polls > 0, every batch planned
+ * (or autotuned) afterwards leaves one finished tile of its first long
+ * transform uncounted and limits its waits to `polls` polls, so they run out;
+ * polls = 0 restores normal batches.  No fault is involved; meant for tests. */
+int minfft_b200_test_mixed_withhold(long long polls);
 
 #ifdef __cplusplus
 } /* extern "C" */

@@ -122,6 +122,8 @@ class Engine(MinfftLibrary):
         L.minfft_b200_test_tc_withhold.restype = i32
         L.minfft_b200_test_stream_stall.argtypes = [i64, i64]
         L.minfft_b200_test_stream_stall.restype = i32
+        L.minfft_b200_test_mixed_withhold.argtypes = [i64]
+        L.minfft_b200_test_mixed_withhold.restype = i32
 
     # --------------------------------------------------------- errors
     def last_error(self) -> int:

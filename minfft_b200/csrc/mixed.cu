@@ -28,11 +28,14 @@
 // slot is.  What an item waits for stands before it in the list, so it has
 // been taken by a running CTA, and first-pass tiles of the first users of a
 // slot wait for nothing: the waits end whatever the residency.  They are
-// bounded all the same; one that runs out sets *status and every CTA stops.
+// bounded all the same: a CTA whose wait runs out sets *status and stops.
+// The others go on until they wait for a tile that no longer comes, so the
+// launch ends after about twice the limit at most, with its output incomplete.
 #include <cuda_runtime.h>
 #include <stdio.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <deque>
@@ -67,9 +70,9 @@ constexpr int kBigMaxLog2L = 16;     // two passes through scratch up to 65536
 constexpr int kTilePoints = 16 * kThreads;  // points of a long item's tile
 constexpr int kOffsetsBytes = 1024;  // tile offsets of the long-item passes (<= 64 transforms)
 constexpr int kMinBlocks = sizeof(real) == 8 ? 2 : 4;  // CTAs per SM: 128 / 64 registers
-// Scratch of each long length: about 2.5 grids of tiles, small enough to stay
-// in the L2 beside the streams (20000 jobs in f32: 1056 us with 32 MiB, 1083
-// with 64, 1085 with 24).
+// Scratch of each long length: 1.7 grids of tiles (1024 in single on a grid of
+// 592 CTAs, 512 in double on 296), small enough to stay in the L2 beside the
+// streams (20000 jobs in f32: 1056 us with 32 MiB, 1083 with 64, 1085 with 24).
 constexpr size_t kSlotBytes = size_t(32) << 20;
 constexpr long long kWaitLimit = 1LL << 22;
 
@@ -105,6 +108,9 @@ struct Params {
   int nbig;           // long transforms
   unsigned* counter;  // the queue, then nbig counters of finished first-pass tiles and nbig of last-pass tiles
   int* status;        // host-mapped; set when a wait ran out
+  // Test hook (zero in normal batches): > 0 limits the waits to that many
+  // polls and leaves the first tile of the first long transform uncounted.
+  long long withhold;
   cpx* scratch;
   const cpx* tw[kSlots];    // w_L^m, by log2 L
   const cpx* rft[kSlots];   // real-DFT roots, by log2 N
@@ -228,9 +234,10 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 __device__ __forceinline__ bool tiles_done(const Params& mp, const unsigned* p, unsigned n) {
   bool ok = true;
   if (threadIdx.x == 0) {
+    const long long limit = mp.withhold > 0 ? mp.withhold : kWaitLimit;
     long long i = 0;
     while (ld_acquire(p) < n)
-      if (++i > kWaitLimit) {
+      if (++i > limit) {
         ok = false;
         *reinterpret_cast<volatile int*>(mp.status) = 1;
         break;
@@ -348,7 +355,7 @@ __device__ __forceinline__ bool run_long(const Params& mp, const Item& it, unsig
       run_first<128>(mp, it, smem);
     else
       run_first<256>(mp, it, smem);
-    tile_done(firsts + it.id);
+    if (!(mp.withhold > 0 && it.id == 0 && it.tile == 0)) tile_done(firsts + it.id);
   } else {
     if (!tiles_done(mp, firsts + it.id, tiles)) return false;
     switch (it.log2L - first_bits(it.log2L)) {
@@ -479,6 +486,10 @@ size_t kernel_smem() {
 using mb::cpx;
 using mb::real;
 using namespace mb::mixed;
+
+namespace {
+std::atomic<long long> g_withhold{0};  // test hook: batches planned from now on (Params::withhold)
+}
 
 struct minfft_b200_mixed {
   int device = 0;
@@ -687,6 +698,7 @@ bool build_items(minfft_b200_mixed* m) {
   m->params.items = static_cast<const Item*>(m->d_items);
   m->params.nitems = int(m->items.size());
   m->params.nbig = nbig;
+  m->params.withhold = g_withhold.load();
   m->params.counter = m->d_counter;
   // graph: reset the queue and the tile counters, run the persistent kernel
   release_graph(m);
@@ -890,4 +902,10 @@ MB_EXPORT int minfft_b200_mixed_autotune(minfft_b200_mixed* m, int reps) {
   m->split = best_split;
   m->grid = grid_for(best_per);
   return build_items(m) ? MINFFT_B200_OK : MINFFT_B200_ECUDA;
+}
+
+MB_EXPORT int minfft_b200_test_mixed_withhold(long long polls) {
+  if (polls < 0) return fail(MINFFT_B200_EINVAL, "poll count must be >= 0");
+  g_withhold.store(polls);
+  return MINFFT_B200_OK;
 }
