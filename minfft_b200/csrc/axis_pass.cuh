@@ -56,6 +56,47 @@ __device__ __forceinline__ cpx kind_base(const cpx* table, int j) {
   }
 }
 
+// The roots w^(j + i*(L/R)) of a kind table, i = 0 .. R/2: base times constant
+// w_128^(i*kStep), two roundings more than the table's entry unless j = 0.  At 16
+// and 32 points radix 16 has such threads for all or half of the roots, radix 8
+// for half as many, and a DCT-4 pair of 64 x 64 was less exact so (single 3.1e-7
+// for 2.6e-7, double 3.75e-16 for 3.67e-16).  There its kernels read each root
+// from the table, in single the other kinds' too, and at 128 points, where
+// radix 8 has a pass more (256 x 256: 3.7e-7 for 3.2e-7).  So 64 x 64 rounds to
+// 2.1e-7 and 3.4e-16 and 256 x 256 to 2.5e-7.  32768 DCT-4 of 64 points in double,
+// bound by L1 traffic, take 20.0 us a pair with table roots, 18.9 without, 28.1
+// at radix 16; in single 14.8, 14.6 and 43; with the tables in shared memory
+// (nd_pass.cu) reading is the faster way at every length (DCT-2 + DCT-3 of 64 x 64
+// in double 11.4 us, 12.4 without).
+#ifdef MB_TABLES_GENERIC
+constexpr bool kTablesNear = true;
+#else
+constexpr bool kTablesNear = false;
+#endif
+template <int L, int R, bool kT4>
+constexpr bool kTableRoots = R == 8 && L > R &&
+                             (kTablesNear || (kT4 && L == 32) || (sizeof(real) == 4 && (L == 32 || L == 128)));
+template <int L, int R, int kStep, bool kT4 = false>
+struct KindRoots {
+  const cpx* t;
+  cpx base;
+  __device__ __forceinline__ KindRoots(const cpx* table, int j) : t(table + j), base(czero()) {
+    if constexpr (!kTableRoots<L, R, kT4>) base = kind_base<L / R>(table, j);
+  }
+  __device__ __forceinline__ cpx operator()(int i) const {
+    if constexpr (kTableRoots<L, R, kT4>)
+      return ldg(t + i * (L / R));
+    else
+      return cmul(base, w128(i * kStep));
+  }
+};
+template <int L, int R>
+using RftRoots = KindRoots<L, R, 64 / R>;  // w_N^k, for 0 < k < L/2 only: i < R/2
+template <int L, int R>
+using T23Roots = KindRoots<L, R, 16 / R>;  // w_4N^k
+template <int L, int R>
+using T4Roots = KindRoots<L, R, 32 / R, true>;  // w_2N^k
+
 struct AxisParams {
   const void* in;
   void* out;
@@ -150,12 +191,13 @@ __device__ __forceinline__ void batch_offsets(const AxisParams& p, int64_t b, in
 // u[r] *= w^r for r = 1..RP-1 with w = tw[i1]: two table roots (w, w^4) per
 // sub-DFT, the other powers formed just before use as products of at most
 // four roundings, so only a handful of roots are live at a time.  The radix-8
-// kernels (kLoad) take w^2 and w^3 from the table too: they run where the
-// array is small and the loads hide, and 32- and 64-point lines then round
-// no more than radix 16 does (64 x 64 DCT-2 and -3 in single, error against
-// double: 3.8e-7 with products, 3.0e-7 with loads, 2.8e-7 at radix 16; the
-// time is the same).
-template <int RP, bool kLoad>
+// kernels (kLoad = 3) take w^2 and w^3 from the table too: they run where the
+// array is small and the loads hide, and 32- and 64-point DFTs then round no
+// more than radix 16 does (in the same time).  At 128 points radix 8 has three
+// passes to radix 16's two, and in single precision (kLoad = 7) takes every
+// power from the table (DCT-4 pair of 256 x 256: 3.7e-7 with products, 3.45e-7
+// with loads, 3.2e-7 at radix 16).
+template <int RP, int kLoad>
 __device__ __forceinline__ void apply_root_powers(cpx* u, const cpx* __restrict__ tw, int i1) {
   static_assert(RP <= 16, "radix up to 16");
   const cpx w1 = ldg(tw + i1);
@@ -168,9 +210,9 @@ __device__ __forceinline__ void apply_root_powers(cpx* u, const cpx* __restrict_
     if constexpr (RP > 4) {
       const cpx w4 = ldg(tw + 4 * i1);
       u[4] = cmul(u[4], w4);
-      u[5] = cmul(u[5], cmul(w4, w1));
-      u[6] = cmul(u[6], cmul(w4, w2));
-      u[7] = cmul(u[7], cmul(w4, w3));
+      u[5] = cmul(u[5], kLoad > 3 ? ldg(tw + 5 * i1) : cmul(w4, w1));
+      u[6] = cmul(u[6], kLoad > 3 ? ldg(tw + 6 * i1) : cmul(w4, w2));
+      u[7] = cmul(u[7], kLoad > 3 ? ldg(tw + 7 * i1) : cmul(w4, w3));
       if constexpr (RP > 8) {
         const cpx w8 = cmul(w4, w4);
         u[8] = cmul(u[8], w8);
@@ -199,7 +241,8 @@ __device__ __forceinline__ void pass_compute(cpx (&v)[R], int j, const cpx* __re
       const int jp = j + s * (L / R);
       const int q = jp & (NS - 1);
       constexpr int step = L / (NS * RP);
-      apply_root_powers<RP, R == 8>(u, tw, q * step);
+      constexpr int load = R != 8 ? 0 : (sizeof(real) == 4 && L == 128) ? 7 : 3;
+      apply_root_powers<RP, load>(u, tw, q * step);
     }
     fft_reg<RP>(u);
 #pragma unroll
@@ -549,14 +592,15 @@ struct LoadT4 {
       for (int r = 0; r < R; ++r) v[r] = czero();
       return;
     }
-    const cpx e = kind_base<TPT>(p.t1, x.j);  // w_2N^j; w_2N^(j + r*TPT) = e * w_4R^r
+    const T4Roots<L, R> e(p.t1, x.j);  // w_2N^(j + r*TPT)
     if (p.in_n == 1)
       rotate<true, L, R>(in, 1, x.j, e, dst, v);
     else
       rotate<false, L, R>(in, p.in_n, x.j, e, dst, v);
   }
   template <bool kUnit, int L, int R>
-  static __device__ __forceinline__ void rotate(const real* in, int64_t s, int j, cpx e, bool dst, cpx (&v)[R]) {
+  static __device__ __forceinline__ void rotate(const real* in, int64_t s, int j, const T4Roots<L, R>& e, bool dst,
+                                                cpx (&v)[R]) {
     constexpr int N = 2 * L, TPT = L / R;
     const real sg = dst ? real(-1) : real(1);
     Walk<const real, kUnit, 2 * TPT> lo(in + int64_t(2 * j) * s, s);
@@ -566,7 +610,7 @@ struct LoadT4 {
       // DST: -(a - ib) = -a + ib
       const real a = sg * *lo.q;
       const real b = *hi.q;
-      v[r] = cmul(cmul(e, w128(r * (32 / R))), cmk(a, b));
+      v[r] = cmul(e(r), cmk(a, b));
     }
   }
 };
@@ -720,7 +764,7 @@ struct LoadC2R {
   template <int L, int R>
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
     const cpx* in = static_cast<const cpx*>(p.in) + x.oin;
-    const cpx b2 = kind_base<L / R>(p.t2, x.j);
+    const RftRoots<L, R> rft(p.t2, x.j);
     const PairSlots<L, R> at(t, x.c, x.j);
     auto z = [&](int k) { return x.active ? in[k] : czero(); };
     pair_loop<L, R>(
@@ -735,7 +779,7 @@ struct LoadC2R {
           }
         },
         [&](int i, int k) {
-          const cpx za = z(k), zb = z(L - k), f = rft_root<R>(b2, i);
+          const cpx za = z(k), zb = z(L - k), f = rft(i);
           at.at(i) = pack_one(za, zb, f);
           at.mirror(i) = pack_mirror(za, zb, f);
         },
@@ -829,7 +873,8 @@ struct LoadDCT3 {
         // up front; every thread reads its pairs before any packed value
         // overwrites the row
         constexpr int TPT = L / R;
-        const cpx b1 = kind_base<TPT>(p.t1, x.j), b2 = kind_base<TPT>(p.t2, x.j);
+        const T23Roots<L, R> t23(p.t1, x.j);
+        const RftRoots<L, R> rft(p.t2, x.j);
         real* sr = tile_row(t, x.c);
         if (x.active) {
           if (p.colmode)
@@ -850,7 +895,7 @@ struct LoadDCT3 {
         cpx za[NP], zb[NP];
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-          const cpx rk = t23_root<R>(b1, i);  // w_4N^k
+          const cpx rk = t23(i);  // w_4N^k
           if (i == 0 && x.j == 0) {
             za[0] = cmk(*pa, real(0));
             zb[0] = cmk(r2 * *pc, real(0));
@@ -867,7 +912,7 @@ struct LoadDCT3 {
               at.at(i) = k == 0 ? cmk(za[0].x + zb[0].x, -(za[0].x - zb[0].x)) : cmk(2 * za[i].x, 2 * za[i].y);
             },
             [&](int i, int) {
-              const cpx f = rft_root<R>(b2, i);
+              const cpx f = rft(i);
               at.at(i) = pack_one(za[i], zb[i], f);
               at.mirror(i) = pack_mirror(za[i], zb[i], f);
             },
@@ -879,16 +924,17 @@ struct LoadDCT3 {
     }
     // the pairs (k, L-k) of pair_loop, read straight from global memory
     constexpr int TPT = L / R;
-    const cpx b1 = kind_base<TPT>(p.t1, x.j), b2 = kind_base<TPT>(p.t2, x.j);
+    const T23Roots<L, R> t23(p.t1, x.j);
+    const RftRoots<L, R> rft(p.t2, x.j);
     auto rd = [&](int m) { return in[int64_t(m) * p.in_n]; };
 #pragma unroll
     for (int i = 0; i <= R / 2; ++i) {
       const int k = x.j + i * TPT;
       if (i == R / 2 && x.j != 0) break;
-      const cpx rk = t23_root<R>(b1, i);  // w_4N^k
+      const cpx rk = t23(i);  // w_4N^k
       const cpx z0 = x.active ? zval_w(rd, k, L, dst, [&](int) { return rk; }) : czero();
       const cpx z1 = x.active ? zval_w(rd, L - k, L, dst, [&](int) { return t23_mirror(rk); }) : czero();
-      pack_into(t, x.c, k, L, z0, z1, rft_root<R>(b2, i));
+      pack_into(t, x.c, k, L, z0, z1, i < R / 2 ? rft(i) : czero());
     }
     __syncthreads();
     gather_natural<L, R>(v, x.j, x.c, t);
@@ -1244,7 +1290,7 @@ struct StoreR2C {
     __syncthreads();
     if (!x.active) return;
     cpx* out = static_cast<cpx*>(p.out) + x.oout;
-    const cpx b1 = kind_base<L / R>(p.t1, x.j);
+    const RftRoots<L, R> rft(p.t1, x.j);
     const PairSlots<L, R> at(t, x.c, x.j);
     pair_loop<L, R>(
         x,
@@ -1258,7 +1304,7 @@ struct StoreR2C {
           }
         },
         [&](int i, int k) {
-          const cpx za = at.at(i), zb = at.mirror(i), f = rft_root<R>(b1, i);
+          const cpx za = at.at(i), zb = at.mirror(i), f = rft(i);
           out[k] = cscale(unpack_one2(za, zb, f), real(0.5));
           out[L - k] = cscale(unpack_mirror2(za, zb, f), real(0.5));
         },
@@ -1313,7 +1359,8 @@ struct StoreDCT2 {
     const bool dst = (p.flags & F_DST) != 0;
     if (dst) out -= s;
     const real r2 = real(1.414213562373095048801688724209698079);
-    const cpx b1 = kind_base<TPT>(p.t1, x.j), b2 = kind_base<TPT>(p.t2, x.j);
+    const T23Roots<L, R> t23(p.t1, x.j);
+    const RftRoots<L, R> rft(p.t2, x.j);
     Walk<real, kUnit, TPT> lo(out + int64_t(x.j) * s, s), up(out + int64_t(L + x.j) * s, s);
     Walk<real, kUnit, -TPT> hi(out + int64_t(N - x.j) * s, s), dn(out + int64_t(L - x.j) * s, s);
     auto put = [&](real* a, real* b, cpx q) {  // y_n = Re, y_(N-n) = -Im
@@ -1335,7 +1382,7 @@ struct StoreDCT2 {
           }
         },
         [&](int i, int) {
-          const cpx za = at.at(i), zb = at.mirror(i), f = rft_root<R>(b2, i), e = t23_root<R>(b1, i);
+          const cpx za = at.at(i), zb = at.mirror(i), f = rft(i), e = t23(i);
           put(lo.q, hi.q, cmul(unpack_one2(za, zb, f), e));
           put(dn.q, up.q, cmul(unpack_mirror2(za, zb, f), t23_mirror(e)));
         },
@@ -1518,7 +1565,9 @@ struct StoreT4 {
     const cpx g = cscale(ldg(p.t2 + 2 * j), real(2));
 #pragma unroll
     for (int r = 0; r < R; ++r, lo.step(), hi.step()) {
-      const cpx A = cmul(cmul(g, w128(r * (32 / R))), v[r]);
+      const cpx gr = kTablesNear && R == 8 && L > R ? cscale(ldg(p.t2 + 2 * (j + r * TPT)), real(2))
+                                                    : cmul(g, w128(r * (32 / R)));
+      const cpx A = cmul(gr, v[r]);
       *lo.q = dst ? A.y : A.x;
       *hi.q = dst ? -A.x : -A.y;
     }
