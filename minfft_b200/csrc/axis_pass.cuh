@@ -63,7 +63,7 @@ __device__ __forceinline__ cpx kind_base(const cpx* table, int j) {
 // for 2.6e-7, double 3.75e-16 for 3.67e-16).  There its kernels read each root
 // from the table, in single the other kinds' too, and at 128 points, where
 // radix 8 has a pass more (256 x 256: 3.7e-7 for 3.2e-7).  So 64 x 64 rounds to
-// 2.1e-7 and 3.4e-16 and 256 x 256 to 2.5e-7.  32768 DCT-4 of 64 points in double,
+// 2.5e-7 and 3.4e-16 and 256 x 256 to 2.8e-7.  32768 DCT-4 of 64 points in double,
 // bound by L1 traffic, take 20.0 us a pair with table roots, 18.9 without, 28.1
 // at radix 16; in single 14.8, 14.6 and 43; with the tables in shared memory
 // (nd_pass.cu) reading is the faster way at every length (DCT-2 + DCT-3 of 64 x 64
@@ -436,6 +436,40 @@ struct RootProgression {
   __device__ __forceinline__ cpx at(int r) const {
     const int m = r * K / R;  // below 64
     return m < 32 ? cmul(base, w128(m)) : cmul_negi(cmul(base, w128(m - 32)));
+  }
+};
+
+// The same roots as constant + constant * (W^g0 - 1).  g0 lies within one step, so
+// |W^g0 - 1| < 0.2 (0.4 at radix 8), the product's roundings are a fraction of the
+// root's, and in single the constant brings along what its own rounding left
+// out: the root has one rounding (two in double), where the product form has
+// five, counting two tables, and a coarse entry times a fine one, as the
+// element-wise steps take, three.  hi and lo hold the roots minus one.
+// For the real and type-2/3 lines, which were up to 6% less exact with products
+// than with element-wise steps (DCT-2 + DCT-3 of 2^16 in single 3.41e-7 for 3.21e-7,
+// 3.15e-7 so; of 2^22 points 49.9 -> 50.1 us in single, 82.2 -> 82.8 in double), and
+// the mixed batch, whose type-4 jobs read tables of their own before (jobs of 2^16
+// points 2.19e-7 for 2.06e-7, 2.07e-7 so; 20000 jobs of all lengths 979 -> 1011 us).  Type-4 lines
+// gain on the element-wise step either way and keep the cheaper products (DCT-4 of
+// 2^24 points 171 us, 174 with steps).
+template <int R, int K>
+struct RootSteps {
+  cpx d;  // W^g0 - 1
+  __device__ __forceinline__ RootSteps(const cpx* __restrict__ hi, const cpx* __restrict__ lo, int lobits,
+                                       uint32_t g0) {
+    const cpx a = ldg(hi + (g0 >> lobits)), b = ldg(lo + (g0 & ((1u << lobits) - 1u)));
+    d = cadd(cadd(a, b), cmul(a, b));
+  }
+  __device__ __forceinline__ cpx at(int r) const {
+    const int m = r * K / R, n = m & 31;  // m below 64
+    const cpx c = w128(n);
+#if MINFFT_SINGLE  // with what the constant's rounding left out
+    const cpx e = cmk(roots128::kReR[n], roots128::kImR[n]);
+    const cpx w = cadd(c, cmk(e.x + c.x * d.x - c.y * d.y, e.y + c.x * d.y + c.y * d.x));
+#else  // (not as a fused multiply-add, which would round the larger sum twice)
+    const cpx t = cmul(c, d), w = cmk(__dadd_rn(c.x, t.x), __dadd_rn(c.y, t.y));
+#endif
+    return m < 32 ? w : cmul_negi(w);
   }
 };
 
@@ -954,7 +988,8 @@ struct LoadDCT3 {
 // (x[2g], x[2g+1]) as one vector, keeps x[2g] and hands x[2g+1] to its
 // mirror element's thread through the tile: every real is read once, in
 // whole sectors.
-struct LoadT4Chain {
+template <template <int, int> class Roots>
+struct LoadT4ChainBy {
   static constexpr bool kComplexIn = false;  // whether the raw input elements are complex
   static constexpr bool kStaged = false;
   template <int L, int R>
@@ -989,11 +1024,12 @@ struct LoadT4Chain {
     }
     __syncthreads();
     // w_2N^g for g = g0 + r*TPT*in_n
-    const RootProgression<R, 32> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(b1 * p.is1 + int64_t(x.j) * p.in_n));
+    const Roots<R, 32> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(b1 * p.is1 + int64_t(x.j) * p.in_n));
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = cmul(ew.at(r), cmk(a[r], get[r * TPT]));
   }
 };
+using LoadT4Chain = LoadT4ChainBy<RootProgression>;
 
 // ---- type-2, type-3 and real-DFT steps fused into the passes of a 1-D chain
 //
@@ -1140,7 +1176,7 @@ struct LoadDCT2Line {
 // the roots w_N^g.
 template <int L, int R>
 __device__ __forceinline__ void pack_tile(const Ctx& x, const Tile& t, const Mirror& mi, bool zero, cpx k0,
-                                          const RootProgression<R, 64>& fw, cpx (&v)[R]) {
+                                          const RootSteps<R, 64>& fw, cpx (&v)[R]) {
   constexpr int TPT = L / R;
   scatter_mirror<L, R>(v, x, mi, t);
   __syncthreads();
@@ -1177,14 +1213,14 @@ struct LoadDCT3Line {
     const real r2 = real(1.414213562373095048801688724209698079);
     const cpx k0 = cmk(v[0].x + r2 * v[0].y, -(v[0].x - r2 * v[0].y));
     {
-      const RootProgression<R, 16> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0));
+      const RootSteps<R, 16> ew(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0));
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const cpx e = ew.at(r);
         v[r] = cmk(v[r].x * e.x - v[r].y * e.y, -(v[r].x * e.y) - v[r].y * e.x);
       }
     }
-    const RootProgression<R, 64> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(4 * g0));
+    const RootSteps<R, 64> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(4 * g0));
     pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
   }
 };
@@ -1211,7 +1247,7 @@ struct LoadC2RLine {
       const cpx zl = in[p.kn / 2];
       k0 = cmk(v[0].x + zl.x, -(v[0].x - zl.x));
     }
-    const RootProgression<R, 64> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0));
+    const RootSteps<R, 64> fw(p.st_hi, p.st_lo, p.st_lobits, uint32_t(g0));
     pack_tile<L, R>(x, t, mi, zero, k0, fw, v);
   }
 };
@@ -1585,7 +1621,8 @@ struct StoreT4 {
 // y[N-1-2m'] of the mirror point m' = Lt-1-m (output L-1-k of the partner
 // sub-DFT), so each element hands that value to its mirror's thread through
 // the tile and writes the pair (y[2m], y[2m+1]) as one vector.
-struct StoreT4Chain {
+template <template <int, int> class Roots>
+struct StoreT4ChainBy {
   template <int L, int R>
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets&,
                                              cpx (&v)[R]) {
@@ -1598,7 +1635,7 @@ struct StoreT4Chain {
     real* sb = reinterpret_cast<real*>(t.s);
     const bool vec = (reinterpret_cast<uintptr_t>(out) % sizeof(cpx)) == 0;
     // g_2m = w_8N^(4m+1) for m = m0 + r*TPT*out_k
-    const RootProgression<R, 32> gw(p.t1, p.t2, p.kbits, uint32_t(4 * (x.oout + int64_t(x.j) * p.out_k) + 1));
+    const Roots<R, 32> gw(p.t1, p.t2, p.kbits, uint32_t(4 * (x.oout + int64_t(x.j) * p.out_k) + 1));
     __syncthreads();  // the last Stockham exchange has finished with the tile
     // a slot holds 2*lp >= 2L reals: the mirror's values below L, its own above
     real* own = sb + x.c * 2 * t.lp + x.j;
@@ -1624,6 +1661,7 @@ struct StoreT4Chain {
     }
   }
 };
+using StoreT4Chain = StoreT4ChainBy<RootProgression>;
 
 // Unpacking of the real DFT (reference minfft.c:547-578; StoreR2C) of output
 // point m: X_m, and at m = 0 also X_Lt.  Roots of N (t1, t2, kbits); the
@@ -1637,7 +1675,7 @@ struct StoreR2CLine {
     cpx* out = static_cast<cpx*>(p.out) + udiv(x.b, p.d0 * p.d1) * p.k_out_line;
     const Mirror mi = mirror_spectrum<TPT>(p, x, x.oout);
     const int64_t m0 = x.oout + int64_t(x.j) * p.out_k;
-    const RootProgression<R, 64> fw(p.t1, p.t2, p.kbits, uint32_t(m0));
+    const RootSteps<R, 64> fw(p.t1, p.t2, p.kbits, uint32_t(m0));
     __syncthreads();  // the last Stockham exchange has finished with the tile
     scatter_mirror<L, R>(v, x, mi, t);
     __syncthreads();
@@ -1677,11 +1715,11 @@ struct StoreDCT2Line {
     const real y0 = 2 * (v[0].x + v[0].y), yl = r2 * (v[0].x - v[0].y);
     const cpx* zm = slot_at<TPT>(t, mi.slot, mi.jm);
     {
-      const RootProgression<R, 64> fw(p.t1, p.t2, p.kbits, uint32_t(4 * m0));
+      const RootSteps<R, 64> fw(p.t1, p.t2, p.kbits, uint32_t(4 * m0));
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = unpack_one2(v[r], zm[nat_off<TPT>(R - 1 - r)], fw.at(r));
     }
-    const RootProgression<R, 16> ew(p.t1, p.t2, p.kbits, uint32_t(m0));
+    const RootSteps<R, 16> ew(p.t1, p.t2, p.kbits, uint32_t(m0));
     const int64_t sa = dst ? -p.out_k : p.out_k;
     Walk<real, false, TPT> wa(dst ? out + (N - 1 - m0) : out + m0, sa);
     Walk<real, false, -TPT> wb(dst ? out + (m0 - 1) : out + (N - m0), sa);
@@ -1744,8 +1782,14 @@ struct MirrorPairs {
   struct MirrorPairs<Op> {                     \
     static constexpr MirrorKind value = kind;  \
   }
-MB_MIRROR(LoadT4Chain, kReflected);
-MB_MIRROR(StoreT4Chain, kReflected);
+template <template <int, int> class Roots>
+struct MirrorPairs<LoadT4ChainBy<Roots>> {
+  static constexpr MirrorKind value = kReflected;
+};
+template <template <int, int> class Roots>
+struct MirrorPairs<StoreT4ChainBy<Roots>> {
+  static constexpr MirrorKind value = kReflected;
+};
 MB_MIRROR(LoadDCT2Line, kReflected);
 MB_MIRROR(StoreDCT3Line, kReflected);
 MB_MIRROR(LoadDCT3Line, kSpectrum);

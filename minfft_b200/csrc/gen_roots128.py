@@ -82,7 +82,7 @@ def fmt_float(v: float) -> str:
 
 def render() -> str:
     """Text of roots128.h."""
-    re_d, im_d, re_f, im_f = [], [], [], []
+    re_d, im_d, re_f, im_f, re_r, im_r = [], [], [], [], [], []
     for m in range(COUNT):
         a = 2 * PI * m / 128
         c, s = cos_sin(a)
@@ -90,13 +90,16 @@ def render() -> str:
         im_d.append(fmt_double(to_double(-s)))
         re_f.append(fmt_float(to_float(c)))
         im_f.append(fmt_float(to_float(-s)))
+        re_r.append(fmt_float(to_float(c - Decimal(to_float(c)))))
+        im_r.append(fmt_float(to_float(-s - Decimal(to_float(-s)))))
 
     def rows(vals):
         return ",\n".join("    " + ", ".join(vals[i:i + 4]) for i in range(0, len(vals), 4))
 
     out = f"""// Generated by gen_roots128.py -- do not edit.
 // w_128^m = exp(-2*pi*i*m/128) = (cos, -sin)(2*pi*m/128), m = 0..{COUNT - 1},
-// each part correctly rounded to double and to float.  Constant memory with
+// each part correctly rounded to double and to float, and what the rounding to
+// float left out (kReR, kImR), rounded to float itself.  Constant memory with
 // static initialisers (internal linkage: every translation unit that includes
 // this header holds its own copy, loaded with the module), so a loop index
 // known after unrolling becomes a constant-bank operand.
@@ -114,6 +117,10 @@ static __constant__ float kReF[kCount] = {{
 {rows(re_f)}}};
 static __constant__ float kImF[kCount] = {{
 {rows(im_f)}}};
+static __constant__ float kReR[kCount] = {{
+{rows(re_r)}}};
+static __constant__ float kImR[kCount] = {{
+{rows(im_r)}}};
 
 }}  // namespace roots128
 }}  // namespace mb

@@ -45,10 +45,11 @@ const void* stream_rows_kernel_fn(int combo, int log2L);
 
 // Root tables kept on the device by plans: w_N^m (m < N); the real-DFT
 // table w_N^k (k < N/4); the type-2/3 table w_4N^n (n < N/2); the type-4
-// tables w_2N^n (n < N/2) and w_8N^(2q+1) (q < N); and the coarse/fine pair
-// of a long length (w_N^(a << lobits), w_N^c), lobits = ceil(log2 N / 2).
+// tables w_2N^n (n < N/2) and w_8N^(2q+1) (q < N); the coarse/fine pair of a
+// long length (w_N^(a << lobits), w_N^c), lobits = ceil(log2 N / 2); and the
+// same pair minus one, rounded as such.
 namespace tables {
-enum TableKind : int { TB_TW = 0, TB_RFT, TB_T23, TB_T4PRE, TB_T4POST, TB_STHI, TB_STLO };
+enum TableKind : int { TB_TW = 0, TB_RFT, TB_T23, TB_T4PRE, TB_T4POST, TB_STHI, TB_STLO, TB_STHI1, TB_STLO1 };
 }
 
 // Radix actually used by a kernel of length L requested with radix R.

@@ -119,6 +119,8 @@ struct Params {
   const cpx* t4b[kSlots];   // type-4 post-rotation, by log2 N
   const cpx* sthi[kSlots];  // coarse roots of a long length, by log2 of it
   const cpx* stlo[kSlots];  // fine roots of a long length
+  const cpx* sthi1[kSlots];  // the same minus one
+  const cpx* stlo1[kSlots];
 };
 
 __host__ __device__ constexpr int small_radix(int L) { return L < 16 ? L : 16; }
@@ -290,16 +292,16 @@ __device__ __noinline__ void run_tile(const Params& mp, const Item& it, unsigned
     p.st_lobits = root_bits(lg);
     p.st_hi = mp.sthi[lg];
     p.st_lo = mp.stlo[lg];
-    p.t1 = mp.sthi[lr];
-    p.t2 = mp.stlo[lr];
+    p.t1 = mp.sthi1[lr];
+    p.t2 = mp.stlo1[lr];
     p.kbits = root_bits(lr);
   } else {
     p.in = it.in;
     p.out = mp.scratch + it.scratch;
     p.flags = (it.flags & (F_DST | F_CONJ_IN | F_VEC)) | F_STAGE_ROWS;
     p.st_lobits = root_bits(lr);
-    p.st_hi = mp.sthi[lr];
-    p.st_lo = mp.stlo[lr];
+    p.st_hi = mp.sthi1[lr];
+    p.st_lo = mp.stlo1[lr];
   }
   constexpr MirrorKind kMirror = MirrorPairs<Ld>::value != kNoMirror ? MirrorPairs<Ld>::value : MirrorPairs<St>::value;
   int64_t* offs = reinterpret_cast<int64_t*>(smem);
@@ -328,7 +330,7 @@ __device__ __forceinline__ void run_first(const Params& mp, const Item& it, unsi
     case K_C2R: run_tile<RP, false, LoadC2RLine, StoreCplx>(mp, it, smem); break;
     case K_DCT2: run_tile<RP, false, LoadDCT2Line, StoreCplx>(mp, it, smem); break;
     case K_DCT3: run_tile<RP, false, LoadDCT3Line, StoreCplx>(mp, it, smem); break;
-    default: run_tile<RP, false, LoadT4Chain, StoreCplx>(mp, it, smem); break;
+    default: run_tile<RP, false, LoadT4ChainBy<RootSteps>, StoreCplx>(mp, it, smem); break;
   }
 }
 
@@ -340,7 +342,7 @@ __device__ __forceinline__ void run_last(const Params& mp, const Item& it, unsig
     case K_C2R: run_tile<RP, true, LoadCplx, StoreRealPairs>(mp, it, smem); break;
     case K_DCT2: run_tile<RP, true, LoadCplx, StoreDCT2Line>(mp, it, smem); break;
     case K_DCT3: run_tile<RP, true, LoadCplx, StoreDCT3Line>(mp, it, smem); break;
-    default: run_tile<RP, true, LoadCplx, StoreT4Chain>(mp, it, smem); break;
+    default: run_tile<RP, true, LoadCplx, StoreT4ChainBy<RootSteps>>(mp, it, smem); break;
   }
 }
 
@@ -742,7 +744,7 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
   }
   m->count = count;
   m->jobs.resize(count);
-  std::vector<int> need_tw(kSlots, 0), need_st(kSlots, 0), nlong(kSlots, 0);
+  std::vector<int> need_tw(kSlots, 0), need_st(kSlots, 0), need_st1(kSlots, 0), nlong(kSlots, 0);
   std::vector<int> need_kind(kSlots * mb::K_COUNT, 0);
   for (int i = 0; i < count; ++i) {
     const minfft_b200_job& j = jobs[i];
@@ -778,10 +780,10 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
     if (lgL > kSmallMaxLog2L) {
       ++nlong[lgL];
       need_tw[first_bits(lgL)] = need_tw[lgL - first_bits(lgL)] = 1;
-      need_st[lgL] = 1;  // the last pass's pre-twiddle, then the fused steps' roots (run_tile)
-      if (combo == mb::K_R2C || combo == mb::K_C2R) need_st[lgn] = 1;
-      if (combo == mb::K_DCT2 || combo == mb::K_DCT3) need_st[lgn + 2] = 1;
-      if (combo == mb::K_T4) need_st[lgn + 1] = need_st[lgn + 3] = 1;
+      need_st[lgL] = 1;  // the last pass's pre-twiddle; need_st1: the fused steps' roots (run_tile)
+      if (combo == mb::K_R2C || combo == mb::K_C2R) need_st1[lgn] = 1;
+      if (combo == mb::K_DCT2 || combo == mb::K_DCT3) need_st1[lgn + 2] = 1;
+      if (combo == mb::K_T4) need_st1[lgn + 1] = need_st1[lgn + 3] = 1;
       continue;
     }
     need_tw[lgL] = 1;
@@ -800,6 +802,8 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
     if (good && need_st[lg]) {
       good = (P.sthi[lg] = upload(m, mb::tables::TB_STHI, L)) && (P.stlo[lg] = upload(m, mb::tables::TB_STLO, L));
     }
+    if (good && need_st1[lg])
+      good = (P.sthi1[lg] = upload(m, mb::tables::TB_STHI1, L)) && (P.stlo1[lg] = upload(m, mb::tables::TB_STLO1, L));
     for (int combo = 1; combo < mb::K_COUNT && good; ++combo) {
       if (!need_kind[combo * kSlots + lg]) continue;
       const int64_t N = L;

@@ -153,6 +153,17 @@ cpx root_w(int64_t m, int64_t N) {
   return r;
 }
 
+// w_N^m - 1: -2 sin^2(a/2) - i sin(a), a = 2 pi m/N
+cpx root_w_minus1(int64_t m, int64_t N) {
+  double c, s, ch, sh;
+  unit_root(-m, N, &c, &s);
+  unit_root(m, 2 * N, &ch, &sh);
+  cpx r;
+  r.x = (real)(-2 * sh * sh);
+  r.y = (real)s;
+  return r;
+}
+
 int ilog2(int64_t v) {
   int r = 0;
   while ((int64_t(1) << r) < v) ++r;
@@ -383,16 +394,19 @@ void host_table(int kind, int64_t N, std::vector<cpx>& h) {
       h.resize(N);
       for (int64_t q = 0; q < N; ++q) h[q] = root_w(2 * q + 1, 8 * N);
       break;
-    case TB_STHI: {  // w_N^(a << lobits)
+    case TB_STHI:    // w_N^(a << lobits)
+    case TB_STHI1: {  // the same minus one
       const int lb = (int)st_lobits_for(N);
       h.resize(std::max<int64_t>(N >> lb, 1));
-      for (int64_t q = 0; q < (int64_t)h.size(); ++q) h[q] = root_w(q << lb, N);
+      for (int64_t q = 0; q < (int64_t)h.size(); ++q)
+        h[q] = kind == TB_STHI ? root_w(q << lb, N) : root_w_minus1(q << lb, N);
       break;
     }
-    case TB_STLO: {  // w_N^c, c < 2^lobits
+    case TB_STLO:    // w_N^c, c < 2^lobits
+    case TB_STLO1: {  // the same minus one
       const int lb = (int)st_lobits_for(N);
       h.resize(int64_t(1) << lb);
-      for (int64_t q = 0; q < (int64_t)h.size(); ++q) h[q] = root_w(q, N);
+      for (int64_t q = 0; q < (int64_t)h.size(); ++q) h[q] = kind == TB_STLO ? root_w(q, N) : root_w_minus1(q, N);
       break;
     }
     default: break;
@@ -1920,7 +1934,8 @@ struct Planner {
       ap.tw = tab(TB_TW, Rp);
       int combo = mb::K_CPLX;
       // root table pairs of the fused steps: 2N and 8N (type 4), 4N (types 2
-      // and 3: w_4N^g, and w_N^g as its fourth power's entry), N (real DFT)
+      // and 3: w_4N^g, and w_N^g as its fourth power's entry), N (real DFT);
+      // all but type 4's minus one (RootSteps)
       auto roots_of = [&](int fused, bool in) -> int64_t {
         if (fused == mb::K_T4IN || fused == mb::K_T4OUT) return in ? 2 * s.N : 8 * s.N;
         return (fused == mb::K_C2RIN || fused == mb::K_R2COUT) ? s.N : 4 * s.N;
@@ -1930,8 +1945,8 @@ struct Planner {
         ap.flags |= (s.flags & mb::F_DST);
         if (combo != mb::K_DCT2IN) {
           const int64_t M = roots_of(combo, true);
-          ap.st_hi = tab(TB_STHI, M);  // coarse x fine
-          ap.st_lo = tab(TB_STLO, M);
+          ap.st_hi = tab(combo == mb::K_T4IN ? TB_STHI : TB_STHI1, M);  // coarse x fine
+          ap.st_lo = tab(combo == mb::K_T4IN ? TB_STLO : TB_STLO1, M);
           ap.st_lobits = (int)st_lobits_for(M);
         }
         ap.is2 = 0;
@@ -1943,8 +1958,8 @@ struct Planner {
         ap.flags |= (s.flags & mb::F_DST);
         if (combo != mb::K_DCT3OUT) {
           const int64_t M = roots_of(combo, false);
-          ap.t1 = tab(TB_STHI, M);  // coarse x fine
-          ap.t2 = tab(TB_STLO, M);
+          ap.t1 = tab(combo == mb::K_T4OUT ? TB_STHI : TB_STHI1, M);  // coarse x fine
+          ap.t2 = tab(combo == mb::K_T4OUT ? TB_STLO : TB_STLO1, M);
           ap.kbits = (int)st_lobits_for(M);
         }
         ap.os2 = 0;
