@@ -6,7 +6,9 @@
 // group of transforms whose DFT fits in one CTA (4096 points) is cut into
 // work items of up to `cpb` transforms (the items of a length-L group use
 // L/16 threads per transform, so a 256-thread CTA holds 256*16/L of them).
-// A longer transform (2^13 .. 2^16 complex points) is a Stockham chain of
+// Transforms of 8192 points, which take 512 threads, run in a kernel of their
+// own beside the persistent one, a CTA each (@).
+// A longer transform (2^14 .. 2^16 complex points) is a Stockham chain of
 // two passes through a scratch slot, and each pass is cut into tiles of 4096
 // points, one work item each, with the kind's pre- and post-processing fused
 // into the passes (the *Line and type-4 chain stages of axis_pass.cuh, which
@@ -66,6 +68,8 @@ namespace mixed {
 constexpr int kThreads = 256;
 constexpr int kSlots = 21;           // table slots by log2 length, 0 .. 20
 constexpr int kSmallMaxLog2L = 12;   // one-CTA DFTs up to 4096 points
+constexpr int kWideLog2L = 13;       // DFTs of a 512-thread CTA
+constexpr int kWideThreads = 512;
 constexpr int kBigMaxLog2L = 16;     // two passes through scratch up to 65536
 constexpr int kTilePoints = 16 * kThreads;  // points of a long item's tile
 constexpr int kOffsetsBytes = 1024;  // tile offsets of the long-item passes (<= 64 transforms)
@@ -104,7 +108,7 @@ struct __align__(16) Item {
 struct Params {
   const Job* jobs;  // in item order
   const Item* items;
-  int nitems;
+  int nitems;         // of the persistent kernel; the wide transforms' follow
   int nbig;           // long transforms
   unsigned* counter;  // the queue, then nbig counters of finished first-pass tiles and nbig of last-pass tiles
   int* status;        // host-mapped; set when a wait ran out
@@ -130,11 +134,11 @@ __host__ __device__ constexpr int first_bits(int lg) { return (lg + 1) / 2; }  /
 __host__ __device__ constexpr int root_bits(int lg) { return (lg + 1) / 2; }   // fine bits of a root pair
 
 // ---------------------------------------------------------------- device
-template <int L, class LoadOp, class StoreOp>
+template <int L, class LoadOp, class StoreOp, int T = kThreads>
 __device__ __noinline__ void run_small(const Params& mp, const Item& it, unsigned char* smem) {
   constexpr int R = small_radix(L);
   constexpr int TPT = L / R;
-  constexpr int CPB = kThreads / TPT;
+  constexpr int CPB = T / TPT;
   const int c = threadIdx.x / TPT, j = threadIdx.x % TPT;
   const bool active = c < it.count;
   Job job{};
@@ -189,42 +193,6 @@ __device__ __noinline__ void run_small(const Params& mp, const Item& it, unsigne
   run_passes<L, R, 1, KeepsTile<LoadOp>::value>(v, j, c, t, p.tw);
   StoreOp::template run<L, R>(p, x, t, to, v);
 }
-
-// Real rows read and written as complex pairs, by scalars where the row is
-// not aligned for pairs (the first pass of the real DFT, the last of its
-// inverse).
-struct LoadRealPairs {
-  template <int L, int R>
-  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
-    if (p.flags & F_VEC) {
-      LoadCplx::run<L, R>(p, x, t, v);
-      return;
-    }
-    const real* in = static_cast<const real*>(p.in);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const real* q = in + 2 * (x.oin + int64_t(x.j + r * (L / R)) * p.in_n);
-      v[r] = cmk(q[0], q[1]);
-    }
-  }
-};
-struct StoreRealPairs {
-  template <int L, int R>
-  static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, const TileOffsets& to,
-                                             cpx (&v)[R]) {
-    if (p.flags & F_VEC) {
-      StoreCplx::run<L, R>(p, x, t, to, v);
-      return;
-    }
-    real* out = static_cast<real*>(p.out);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      real* q = out + 2 * (x.oout + int64_t(x.j + r * (L / R)) * p.out_k);
-      q[0] = v[r].x;
-      q[1] = -v[r].y;
-    }
-  }
-};
 
 // Finished tiles of a long transform's pass, counted in global memory.
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -288,7 +256,7 @@ __device__ __noinline__ void run_tile(const Params& mp, const Item& it, unsigned
   if constexpr (kIsLast) {
     p.in = mp.scratch + it.scratch;
     p.out = it.out;
-    p.flags = (it.flags & (F_DST | F_CONJ_OUT | F_VEC)) | F_SRC_SMEM;  // scratch by plain loads: it stays in the L2
+    p.flags = (it.flags & (F_DST | F_CONJ_OUT)) | F_SRC_SMEM;  // scratch by plain loads: it stays in the L2
     p.st_lobits = root_bits(lg);
     p.st_hi = mp.sthi[lg];
     p.st_lo = mp.stlo[lg];
@@ -298,7 +266,7 @@ __device__ __noinline__ void run_tile(const Params& mp, const Item& it, unsigned
   } else {
     p.in = it.in;
     p.out = mp.scratch + it.scratch;
-    p.flags = (it.flags & (F_DST | F_CONJ_IN | F_VEC)) | F_STAGE_ROWS;
+    p.flags = (it.flags & (F_DST | F_CONJ_IN)) | F_STAGE_ROWS;
     p.st_lobits = root_bits(lr);
     p.st_hi = mp.sthi1[lr];
     p.st_lo = mp.stlo1[lr];
@@ -326,7 +294,7 @@ template <int RP>
 __device__ __forceinline__ void run_first(const Params& mp, const Item& it, unsigned char* smem) {
   switch (it.combo) {
     case K_CPLX: run_tile<RP, false, LoadCplx, StoreCplx>(mp, it, smem); break;
-    case K_R2C: run_tile<RP, false, LoadRealPairs, StoreCplx>(mp, it, smem); break;
+    case K_R2C: run_tile<RP, false, LoadCplx, StoreCplx>(mp, it, smem); break;
     case K_C2R: run_tile<RP, false, LoadC2RLine, StoreCplx>(mp, it, smem); break;
     case K_DCT2: run_tile<RP, false, LoadDCT2Line, StoreCplx>(mp, it, smem); break;
     case K_DCT3: run_tile<RP, false, LoadDCT3Line, StoreCplx>(mp, it, smem); break;
@@ -339,7 +307,7 @@ __device__ __forceinline__ void run_last(const Params& mp, const Item& it, unsig
   switch (it.combo) {
     case K_CPLX: run_tile<RP, true, LoadCplx, StoreCplx>(mp, it, smem); break;
     case K_R2C: run_tile<RP, true, LoadCplx, StoreR2CLine>(mp, it, smem); break;
-    case K_C2R: run_tile<RP, true, LoadCplx, StoreRealPairs>(mp, it, smem); break;
+    case K_C2R: run_tile<RP, true, LoadCplx, StoreCplx>(mp, it, smem); break;
     case K_DCT2: run_tile<RP, true, LoadCplx, StoreDCT2Line>(mp, it, smem); break;
     case K_DCT3: run_tile<RP, true, LoadCplx, StoreDCT3Line>(mp, it, smem); break;
     default: run_tile<RP, true, LoadCplx, StoreT4ChainBy<RootSteps>>(mp, it, smem); break;
@@ -360,11 +328,10 @@ __device__ __forceinline__ bool run_long(const Params& mp, const Item& it, unsig
     if (!(mp.withhold > 0 && it.id == 0 && it.tile == 0)) tile_done(firsts + it.id);
   } else {
     if (!tiles_done(mp, firsts + it.id, tiles)) return false;
-    switch (it.log2L - first_bits(it.log2L)) {
-      case 6: run_last<64>(mp, it, smem); break;
-      case 7: run_last<128>(mp, it, smem); break;
-      default: run_last<256>(mp, it, smem); break;
-    }
+    if (it.log2L - first_bits(it.log2L) == 7)
+      run_last<128>(mp, it, smem);
+    else
+      run_last<256>(mp, it, smem);
     tile_done(lasts + it.id);
   }
   return true;
@@ -466,7 +433,26 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) mixed_kernel(const __gri
   }
 }
 
-// shared memory of the kernel: offsets + the largest tile of any item
+// One transform of 8192 points per CTA.
+__global__ void __launch_bounds__(kWideThreads, kMinBlocks / 2) wide_kernel(const __grid_constant__ Params mp) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int L = 1 << kWideLog2L;
+  const Item it = mp.items[mp.nitems + blockIdx.x];
+  switch (it.combo) {
+    case K_CPLX: run_small<L, LoadCplx, StoreCplx, kWideThreads>(mp, it, smem); break;
+    case K_R2C: run_small<L, LoadR2C, StoreR2C, kWideThreads>(mp, it, smem); break;
+    case K_C2R: run_small<L, LoadC2R, StoreC2R, kWideThreads>(mp, it, smem); break;
+    case K_DCT2: run_small<L, LoadDCT2, StoreDCT2, kWideThreads>(mp, it, smem); break;
+    case K_DCT3: run_small<L, LoadDCT3, StoreDCT3, kWideThreads>(mp, it, smem); break;
+    default: run_small<L, LoadT4, StoreT4, kWideThreads>(mp, it, smem); break;
+  }
+}
+
+size_t wide_smem() {
+  return kOffsetsBytes + 16 * ((tile_pitch(1 << kWideLog2L, 16, 1, 0) * sizeof(cpx) + 15) / 16);
+}
+
+// shared memory of the persistent kernel: offsets + the largest tile of any item
 size_t kernel_smem() {
   size_t m = 0;
   for (int lg = 0; lg <= kSmallMaxLog2L; ++lg) {
@@ -474,7 +460,7 @@ size_t kernel_smem() {
     const int cpb = small_cpb(L);
     m = std::max(m, size_t(cpb) * tile_pitch(L, small_radix(L), cpb, 0) * sizeof(cpx));
   }
-  for (int rp : {64, 128, 256}) {  // long items' tiles
+  for (int rp : {128, 256}) {  // long items' tiles
     const int cpb = kThreads / (rp / 16);
     m = std::max(m, size_t(cpb) * tile_pitch(rp, 16, cpb, 1) * sizeof(cpx));
   }
@@ -497,7 +483,8 @@ struct minfft_b200_mixed {
   int device = 0;
   int count = 0;
   std::vector<Job> jobs;
-  std::vector<Item> items;
+  std::vector<Item> items;  // the persistent kernel's, then the wide transforms'
+  int nwide = 0;
   Params params;
   void* d_jobs = nullptr;
   void* d_items = nullptr;
@@ -579,6 +566,7 @@ void release_graph(minfft_b200_mixed* m) {
 // order them, upload, and capture counter reset + kernel in a graph.
 bool build_items(minfft_b200_mixed* m) {
   std::map<std::tuple<int, int, int, int>, std::vector<int>> groups;  // (long, combo, flags, log2L) -> jobs
+  std::vector<Item> wide;
   for (int i = 0; i < m->count; ++i) {
     const Job& j = m->jobs[i];
     const int combo = combo_of(j.op);
@@ -588,7 +576,7 @@ bool build_items(minfft_b200_mixed* m) {
       continue;
     }
     const int lgL = combo == mb::K_CPLX ? j.log2n : j.log2n - 1;
-    groups[std::make_tuple(lgL > kSmallMaxLog2L ? 1 : 0, combo, flags_of(j.op), lgL)].push_back(i);
+    groups[std::make_tuple(lgL > kWideLog2L ? 1 : 0, combo, flags_of(j.op), lgL)].push_back(i);
   }
   std::vector<std::pair<double, Item>> its;  // short items by cost
   std::vector<Item> longs;                   // one prototype per long transform
@@ -608,9 +596,6 @@ bool build_items(minfft_b200_mixed* m) {
         l.op = j.op;
         l.in = j.in;
         l.out = j.out;
-        // rows read or written as complex pairs: an unaligned one by scalars
-        const void* row = combo == mb::K_C2R ? j.out : j.in;
-        if (reinterpret_cast<uintptr_t>(row) % sizeof(cpx) == 0) l.flags |= mb::F_VEC;
         // the inverse real DFT's chain ends conjugated, as the complex inverse's does
         if (combo == mb::K_C2R) l.flags |= mb::F_CONJ_OUT;
         longs.push_back(l);
@@ -618,13 +603,17 @@ bool build_items(minfft_b200_mixed* m) {
       continue;
     }
     const int L = 1 << lgL;
-    const int per = combo < 0 ? kThreads : std::max(1, small_cpb(L) / m->split);
+    const int per = combo < 0 ? kThreads : lgL == kWideLog2L ? 1 : std::max(1, small_cpb(L) / m->split);
     for (size_t s = 0; s < js.size(); s += per) {
       it.kind = combo < 0 ? kUnit : kShort;
       it.count = int(std::min<size_t>(per, js.size() - s));
       it.first = int(order.size());
       it.op = m->jobs[js[s]].op;
       for (int k = 0; k < it.count; ++k) order.push_back(m->jobs[js[s + k]]);
+      if (lgL == kWideLog2L && combo >= 0) {
+        wide.push_back(it);
+        continue;
+      }
       its.push_back(std::make_pair(double(L) * std::max(1, lgL) * it.count, it));  // cost: points processed
     }
   }
@@ -677,7 +666,9 @@ bool build_items(minfft_b200_mixed* m) {
     }
   }
   while (nshort < its.size()) m->items.push_back(its[nshort++].second);
-  const int nbig = int(longs.size());
+  const int nbig = int(longs.size()), nitems = int(m->items.size());
+  m->items.insert(m->items.end(), wide.begin(), wide.end());
+  m->nwide = int(wide.size());
 
   if (m->d_jobs) cudaFree(m->d_jobs);
   if (m->d_items) cudaFree(m->d_items);
@@ -698,24 +689,39 @@ bool build_items(minfft_b200_mixed* m) {
     return false;
   m->params.jobs = static_cast<const Job*>(m->d_jobs);
   m->params.items = static_cast<const Item*>(m->d_items);
-  m->params.nitems = int(m->items.size());
+  m->params.nitems = nitems;
   m->params.nbig = nbig;
   m->params.withhold = g_withhold.load();
   m->params.counter = m->d_counter;
-  // graph: reset the queue and the tile counters, run the persistent kernel
+  // graph: reset the queue and the tile counters, run the persistent kernel;
+  // beside them the wide transforms' kernel, which starts first (the persistent
+  // CTAs take the SMs as its own leave them)
   release_graph(m);
-  cudaStream_t cs;
-  if (!ok(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
-  bool good = ok(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-  if (good) {
-    cudaMemsetAsync(m->d_counter, 0, m->counter_bytes, cs);
-    void* args[1] = {&m->params};
-    cudaLaunchKernel((const void*)mixed_kernel, dim3(m->grid), dim3(kThreads), args, m->smem, cs);
-    good = ok(cudaStreamEndCapture(cs, &m->graph), "cudaStreamEndCapture");
+  if (!ok(cudaGraphCreate(&m->graph, 0), "cudaGraphCreate")) return false;
+  void* args[1] = {&m->params};
+  auto kernel = [&](const void* fn, int grid, int threads, size_t smem, const cudaGraphNode_t* after) {
+    cudaKernelNodeParams k = {};
+    k.func = const_cast<void*>(fn);
+    k.gridDim = dim3(grid);
+    k.blockDim = dim3(threads);
+    k.sharedMemBytes = unsigned(smem);
+    k.kernelParams = args;
+    cudaGraphNode_t node;
+    return ok(cudaGraphAddKernelNode(&node, m->graph, after, after ? 1 : 0, &k), "cudaGraphAddKernelNode");
+  };
+  if (m->nwide && !kernel((const void*)wide_kernel, m->nwide, kWideThreads, wide_smem(), nullptr)) return false;
+  if (nitems) {
+    cudaMemsetParams z = {};
+    z.dst = m->d_counter;
+    z.elementSize = sizeof(unsigned);
+    z.width = m->counter_bytes / sizeof(unsigned);
+    z.height = 1;
+    cudaGraphNode_t node;
+    if (!ok(cudaGraphAddMemsetNode(&node, m->graph, nullptr, 0, &z), "cudaGraphAddMemsetNode") ||
+        !kernel((const void*)mixed_kernel, m->grid, kThreads, m->smem, &node))
+      return false;
   }
-  if (good) good = ok(cudaGraphInstantiate(&m->exec, m->graph, 0), "cudaGraphInstantiate");
-  cudaStreamDestroy(cs);
-  return good;
+  return ok(cudaGraphInstantiate(&m->exec, m->graph, 0), "cudaGraphInstantiate");
 }
 
 }  // namespace
@@ -777,7 +783,7 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
     }
     m->jobs[i] = Job{j.in, j.out, j.op, lgn};
     if (n == 1) continue;
-    if (lgL > kSmallMaxLog2L) {
+    if (lgL > kWideLog2L) {
       ++nlong[lgL];
       need_tw[first_bits(lgL)] = need_tw[lgL - first_bits(lgL)] = 1;
       need_st[lgL] = 1;  // the last pass's pre-twiddle; need_st1: the fused steps' roots (run_tile)
@@ -821,6 +827,9 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
   if (good)
     good = ok(cudaFuncSetAttribute((const void*)mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(m->smem)),
+              "cudaFuncSetAttribute") &&
+           ok(cudaFuncSetAttribute((const void*)wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(wide_smem())),
               "cudaFuncSetAttribute");
   int occ = 1;
   if (good)
@@ -830,7 +839,7 @@ MB_EXPORT minfft_b200_mixed* minfft_b200_mixed_plan(int count, const minfft_b200
   m->grid = sms * m->per_sm;
   // scratch slots of each long length, in kSlotBytes
   int64_t scratch = 0;
-  for (int lg = kSmallMaxLog2L + 1; lg <= kBigMaxLog2L; ++lg) {
+  for (int lg = kWideLog2L + 1; lg <= kBigMaxLog2L; ++lg) {
     const size_t bytes = (size_t(1) << lg) * sizeof(cpx);
     m->slots[lg] = int(std::min<size_t>(nlong[lg], kSlotBytes / bytes));
     m->slot_base[lg] = scratch;

@@ -89,3 +89,22 @@ def test_real_rows_not_aligned_for_pairs(single, n):
         assert (torch.linalg.vector_norm(y[i] - ref) / torch.linalg.vector_norm(ref)).item() <= tolerance(single, (n,))
         back = torch.linalg.vector_norm(z[i] / n - x[i]) / torch.linalg.vector_norm(x[i])
         assert back.item() <= 2 * tolerance(single, (n,))
+
+
+@precisions
+def test_transforms_of_8192_points_take_one_block_each(single):
+    """One item a transform, between shorter and longer jobs and alone; every kind."""
+    eng = minfft_b200.engine(single)
+    rng = np.random.default_rng(8)
+    wide = [(op, 1 << (13 if op in ("dft", "invdft") else 14)) for op in minfft_b200.OPS] * 3
+    for specs, items in ((wide, len(wide)), (wide + [("dct2", 64)] * 8 + [("dft", 1 << 15)], None)):
+        pool, jobs, host = make_batch(single, specs, rng)
+        h = eng.mixed_plan(jobs)
+        try:
+            assert items is None or eng.mixed_items(h) == items
+            eng.mixed_execute(h)
+            eng.mixed_execute(h)
+            torch.cuda.synchronize()
+            check_batch(single, pool, host)
+        finally:
+            eng.mixed_free(h)
