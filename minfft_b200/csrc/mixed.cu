@@ -397,13 +397,17 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) mixed_kernel(const __gri
     }
   };
   // A batch without long transforms has no waits, so any CTA may have any item:
-  // each starts with the one of its own index, and no CTA waits for a grid of
-  // atomics on the counter first (300 jobs of 2^4 .. 2^10 points in f32 14.3 us,
-  // 10.3 so; 11054 jobs 23.5 / 18.5; 4000 of 2^4 .. 2^11 in f64 24.4 / 18.9).
-  const unsigned dealt = mp.nbig ? 0u : gridDim.x;
+  // each starts with the one of its own index and goes on with the one a grid
+  // later, and only then turns to the counter, whose answer it asks for a whole
+  // item ahead.  (Thread 0 holds its CTA's first barrier up until the answer is
+  // there, behind a grid of atomics on one address: in single, 300 jobs of
+  // 2^4 .. 2^10 points take 14.3 us from the counter alone and 10.3 so, 5000 of 2^10
+  // 28.6 with one item dealt and 20.0 so, 9919 of 2^4 .. 2^12 41.5 and 35.2; 11054 of
+  // 2^4 .. 2^10 in double 30.6 and 27.1.)
+  const unsigned dealt = mp.nbig ? 0u : 2 * gridDim.x;
   if (threadIdx.x == 0) {
     fetch(int(mp.nbig ? atomicAdd(mp.counter, 1u) : blockIdx.x), 0);
-    ahead = dealt + atomicAdd(mp.counter, 1u);
+    ahead = mp.nbig ? atomicAdd(mp.counter, 1u) : gridDim.x + blockIdx.x;
   }
   for (int n = 0;; ++n) {
     if (threadIdx.x == 0) asm volatile("cp.async.wait_all;" ::: "memory");

@@ -108,3 +108,25 @@ def test_transforms_of_8192_points_take_one_block_each(single):
             check_batch(single, pool, host)
         finally:
             eng.mixed_free(h)
+
+
+@precisions
+def test_item_counts_around_one_and_two_grids(single):
+    """Without long transforms a block's first two items are dealt by index and the
+    rest come from the counter: one job an item, counts around the grid's size."""
+    eng = minfft_b200.engine(single)
+    cdt = torch.complex64 if single else torch.complex128
+    n, grid = 4096, torch.cuda.get_device_properties(0).multi_processor_count * (4 if single else 2)
+    x = torch.randn(2 * grid + 3, n, dtype=cdt, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    ref = torch.fft.fft(x.to(torch.complex128))
+    for count in (1, grid - 1, grid, grid + 1, 2 * grid, 2 * grid + 1, 2 * grid + 3):
+        y = torch.full_like(x[:count], float("nan"))
+        h = eng.mixed_plan([("dft", n, x[i].data_ptr(), y[i].data_ptr()) for i in range(count)])
+        try:
+            assert eng.mixed_items(h) == count
+            eng.mixed_execute(h)
+            torch.cuda.synchronize()
+        finally:
+            eng.mixed_free(h)
+        err = torch.linalg.vector_norm(y - ref[:count], dim=1) / torch.linalg.vector_norm(ref[:count], dim=1)
+        assert err.max().item() <= tolerance(single, (n,)), count
