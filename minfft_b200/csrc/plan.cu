@@ -542,12 +542,23 @@ struct Planner {
     if (r8 && mb::axis_kernel(combo, ilog2(L), 8)) *R = 8;
     const int tpt = L / std::min(*R, L);
     const int elem = (combo == mb::K_CPLX) ? int(sizeof(cpx)) : int(sizeof(real));
-    if (!col)
+    if (!col) {
       ap.cpb = std::max(1, 64 / tpt);
-    else if (few)
+      // Rows of a few bytes: CTAs of 64 of them start no faster than one in 1.2 ns
+      // (600000 real DFTs of 4 points in single 22.2 us a pair, 12.9 with 128 rows; of 2
+      // points 21.8, and 10.2 with 256; from 64 bytes on, and for the real kinds from 32
+      // on, more rows lose or gain nothing).  The real DFTs' and types 2 and 3's rows of
+      // 128 bytes take 256 from 24 MiB on (600000 real DFTs of 16 points in double 112
+      // us, 86 so; of 32 points in single 154 and 144; at 12 MiB 256 rows lose, 30.6
+      // against 36.7).
+      const int64_t row = L * int64_t(sizeof(cpx));
+      if (L <= 2 || (combo == mb::K_CPLX && row <= 32)) ap.cpb = L == 1 ? 256 : 128;
+      if (combo != mb::K_CPLX && combo != mb::K_T4 && row == 128 && nbatch * row >= (int64_t(24) << 20)) ap.cpb = 256;
+    } else if (few) {
       ap.cpb = std::max(32 / elem, 128 / tpt);
-    else if (sizeof(real) == 8)
+    } else if (sizeof(real) == 8) {
       ap.cpb = std::max(64 / elem, 128 / tpt);
+    }
     while (ap.cpb > 1 && !plain_fits(combo, L, ap.cpb, ap.flags, col ? 1 : 0, *R)) ap.cpb /= 2;
   }
 
