@@ -1010,6 +1010,15 @@ struct Planner {
       ok = false;
       return;
     }
+    // Columns of 2048 points and more, at most a CTA per SM: of these 512-thread
+    // CTAs two fit an SM, and since they come in while the previous kernel still
+    // holds some SMs (dependent launch), many SMs got two and others none.  More
+    // than half of an SM's shared memory spreads them out: DFT 4096 x 256 in
+    // single 43.5 us, 30.6 so; DCT-4 8192 x 256 72.1 and 48.1; DFT 2048 x 512 31.7 and
+    // 25.4.  Shorter columns would gain less than they lose by keeping the next
+    // column pass out (DCT-2 + DCT-3 of 128 x 128 x 64 29.0 and 36.5).
+    if (ap.colmode && L >= 2048 && ap.cpb * tpt >= 512 && (nbatch + ap.cpb - 1) / ap.cpb <= sms)
+      ln.smem = std::max(ln.smem, size_t(116) << 10);
     if (!a->host_only && !ensure_smem_attr(ln.fn, ln.smem)) {
       ok = false;
       return;
