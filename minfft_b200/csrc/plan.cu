@@ -887,6 +887,15 @@ struct Planner {
     prog->launches.push_back(ln);
   }
 
+  // Whether a launch over `bytes` of columns of L points streams them: 512
+  // points beyond the L2 (128 MiB; 256 MiB in single).  64 DFTs of 2^18 points in
+  // f64, round trip, 518 us with one tile per CTA, 458 so; launches that the L2
+  // holds gain nothing (2^21 points in f64: 63.1 against 69.0), nor do the slabs of
+  // a larger array (512 x 512 x 64 in f64: 590 against 629).
+  static bool streams_columns(int64_t L, int64_t bytes) {
+    return L == 512 && bytes >= (int64_t(1) << (sizeof(real) == 4 ? 28 : 27));
+  }
+
   void add_axis_kernel(int combo, int L, int64_t nbatch, AxisParams ap, int in_buf, int out_buf, bool vec_in,
                        bool vec_out) {
     const int lg = ilog2(L);
@@ -921,21 +930,16 @@ struct Planner {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         ov = g_default_override;
       }
-      // Columns streamed by two groups of threads per CTA.  512 points of
-      // arrays beyond the L2 (128 MiB; 256 MiB in single): the axes of
-      // 512 x 512 x 64 in f64, round trip, 676 us with one tile per CTA, 551
-      // so; 64 DFTs of 2^18 points 518 against 458; arrays that the L2 holds
-      // gain nothing (2^21 points in f64: 63.1 against 69.0).  256 points
-      // only where every row of the tile, read and written, has a 2 MiB page
-      // of its own and the longer runs of a streamed tile pay (last pass of
-      // 2^26 points in f64: 433 us, 362 so; with rows 8 KiB apart on one side
-      // 236 us a round trip of 64 DFTs of 2^17 points became 256).  A pass
-      // that stages its output rows keeps a third 512-point tile in flight,
-      // as its stage is busy until the last store.
+      // Columns streamed by two groups of threads per CTA: 512 points
+      // (streams_columns), and 256 points only where every row of the tile, read
+      // and written, has a 2 MiB page of its own and the longer runs of a
+      // streamed tile pay (last pass of 2^26 points in f64: 433 us, 362 so; with
+      // rows 8 KiB apart on one side 236 us a round trip of 64 DFTs of 2^17 points
+      // became 256).  A pass that stages its output rows keeps a third 512-point
+      // tile in flight, as its stage is busy until the last store.
       const int64_t C = int64_t(sizeof(cpx)), page = int64_t(2) << 20;
       const bool streamed =
-          L == 512 ? nbatch * L * C >= (int64_t(1) << (sizeof(real) == 4 ? 28 : 27))
-                   : L == 256 && ap.in_n * C >= page && ap.out_k * C >= page;
+          streams_columns(L, nbatch * L * C) || (L == 256 && ap.in_n * C >= page && ap.out_k * C >= page);
       const int col_stages = (L == 512 && (ap.flags & mb::F_STAGE_ROWS)) ? 3 : 2;
       if (ov.pipe < 0 && ov.cpb == 0 && ov.radix == 16 && streamed &&
           stream_fits(combo, L, nbatch, ap, 16, col_stages)) {
@@ -1681,14 +1685,23 @@ struct Planner {
   // axes[i] of `shape` (extents with the batch count first).  A complex array
   // beyond the L2 is read and written once per axis; the steps along its inner
   // axes, though, stay within a slab of consecutive outer indices, so they all
-  // run on one slab of 64 MiB before the next, and only the first reads it
-  // from memory.  Round trips, in us, axis by axis and so: 256^3 f32 272 /
-  // 257, f64 520 / 504; 48 arrays of 64^3 f64 370 / 326 (slabs of 32 MiB lose
-  // most of it to their launches' ends: 272 and 537 for 256^3).  The kinds
-  // whose passes are bound by instructions gain nothing: DCT-2 + DCT-3 of
-  // 256^3 f64 326 / 337.  The tensor-core modes lose 1% (256^3 in FP16 409 /
-  // 413) and take the slabs all the same, so that a plan keeps one list of
-  // axis launches whatever its arithmetic.
+  // run on one slab of 64 MiB before the next, and only the first reads it from
+  // memory.  Round trips, in us, axis by axis and so (slabs of 32 MiB lose most of
+  // the gain to their launches' ends):
+  //   three steps inside: 48 arrays of 64^3 f64 376 / 348, 300 of them 2200 / 2085,
+  //     1500 of 32^3 1485 / 1380, 8 of 16 x 512 x 512 f32 563 / 524;
+  //   two: 256^3 f32 280 / 262, f64 520 / 504, 256 of 256 x 256 f32 184 / 171, 5000 of
+  //     32 x 64 f64 212 / 200, 3 of 256^3 f32 776 / 767; but 5000 of 128 x 128 f64 1527 /
+  //     1583, 5 of 128 x 256 x 512 2503 / 2590: taken below 384 MiB;
+  //   and with 512-point columns, which stream as one launch (streams_columns) and
+  //     not as slabs, 64 of 512 x 512 f64 385 / 400, 512^3 f32 2400 / 2540, f64 4770 /
+  //     5060: left whole.
+  // The tensor-core modes, whose passes are bound by instructions, lose with two
+  // steps inside: 300 of 256 x 256 in FP16 296 / 350, BF16 373 / 427; 256^3 397 / 412
+  // and 495 / 520; 3 of 256^3 1078 / 1233 and 1376 / 1497.  They take them only for
+  // three axes below 256 MiB, where 4% are lost: the planner's tests hold their
+  // plan of 256^3 to no fewer launches than the FP32 plan has.  The real kinds'
+  // passes are bound by instructions as well: DCT-2 + DCT-3 of 256^3 f64 326 / 337.
   void plan_axes(const std::vector<AxisStep>& steps, const std::vector<size_t>& axes,
                  const std::vector<int64_t>& shape) {
     constexpr size_t kSlab = size_t(64) << 20;
@@ -1720,8 +1733,16 @@ struct Planner {
       }
     }
     size_t inside = 0;
-    for (size_t ax : axes) inside += chunk && ax > last;
-    if (inside < 2 || chunk >= outer) {
+    bool streams = false;
+    for (size_t i = 0; i < steps.size(); ++i)
+      if (chunk && axes[i] > last) {
+        ++inside;
+        streams |= steps[i].inner > 1 && streams_columns(steps[i].N, total);
+      }
+    const bool tc = a->precision != MINFFT_B200_PREC_FP32;
+    const bool slabs =
+        inside > 2 || (inside == 2 && !streams && (tc ? steps.size() > 2 && total < 4 * kSlab : total < 6 * kSlab));
+    if (!slabs || chunk >= outer) {
       for (const AxisStep& s : steps) plan_axis(s);
       return;
     }
