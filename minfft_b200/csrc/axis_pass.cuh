@@ -229,7 +229,7 @@ __device__ __forceinline__ void apply_root_powers(cpx* u, const cpx* __restrict_
   }
 }
 
-template <int L, int R, int RP, int NS>
+template <int L, int R, int RP, int NS, bool kScalar = false>
 __device__ __forceinline__ void pass_compute(cpx (&v)[R], int j, const cpx* __restrict__ tw) {
   constexpr int S = R / RP;  // sub-DFTs per thread in this pass
 #pragma unroll
@@ -244,7 +244,7 @@ __device__ __forceinline__ void pass_compute(cpx (&v)[R], int j, const cpx* __re
       constexpr int load = R != 8 ? 0 : (sizeof(real) == 4 && L == 128) ? 7 : 3;
       apply_root_powers<RP, load>(u, tw, q * step);
     }
-    fft_reg<RP>(u);
+    fft_reg<RP, kScalar>(u);
 #pragma unroll
     for (int r = 0; r < RP; ++r) v[s + r * S] = u[r];
   }
@@ -298,16 +298,16 @@ __device__ __forceinline__ void scatter_natural(const cpx (&v)[R], int j, int c,
 // the first exchange needs no barrier before its writes: a warp whose loads
 // have come goes on to them (round trips: 256^3 f32 258.0 us with the barrier,
 // 253.7 without; real DFT 2048 x 2048 f64 70.7 / 69.8).
-template <int L, int R, int NS, bool kFresh = false>
+template <int L, int R, int NS, bool kFresh = false, bool kScalar = false>
 __device__ __forceinline__ void run_passes(cpx (&v)[R], int j, int c, const Tile& t, const cpx* __restrict__ tw) {
   constexpr int RP = (L / NS >= R) ? R : (L / NS);
-  pass_compute<L, R, RP, NS>(v, j, tw);
+  pass_compute<L, R, RP, NS, kScalar>(v, j, tw);
   if constexpr (NS * RP < L) {
     if constexpr (!kFresh) __syncthreads();
     pass_scatter<L, R, RP, NS>(v, j, c, t);
     __syncthreads();
     gather_natural<L, R>(v, j, c, t);
-    run_passes<L, R, NS * RP>(v, j, c, t, tw);
+    run_passes<L, R, NS * RP, false, kScalar>(v, j, c, t, tw);
   }
 }
 
@@ -1826,11 +1826,18 @@ struct MinBlocks {
   static constexpr int value = sizeof(real) == 8 ? (R >= 16 ? 1 : 2) : (R >= 16 ? 2 : R == 8 ? 3 : 2);
 };
 
+// Complex columns of 4096 points in single, of which a CTA holds two: passes
+// whose sums are scalar instructions.  Packed sums, ahead everywhere else (8000
+// rows of 4096 points 198 us a pair, 213 scalar), cost them up to 5% on arrays
+// beyond the L2 -- column passes of the real DFT of 16384 x 2048 166 us scalar, 175
+// packed, of 4096 x 16384 368 and 387 -- in as many registers and without spills.
+struct LoadCplxScalar : LoadCplx {};
+
 // Load stages that take no shared memory at all: the exchange tile is as the
 // CTA's last barrier left it.
 template <class Op>
 struct KeepsTile {
-  static constexpr bool value = std::is_same<Op, LoadCplx>::value || std::is_same<Op, LoadR2C>::value ||
+  static constexpr bool value = std::is_base_of<LoadCplx, Op>::value || std::is_same<Op, LoadR2C>::value ||
                                 std::is_same<Op, LoadDCT2>::value || std::is_same<Op, LoadT4>::value;
 };
 
@@ -1876,7 +1883,7 @@ __global__ void __launch_bounds__(512, MinBlocks<R>::value) axis_pass_kernel(con
   pdl_wait();
   LoadOp::template run<L, R>(p, x, t, v);
   pdl_release();
-  run_passes<L, R, 1, KeepsTile<LoadOp>::value>(v, x.j, x.c, t, p.tw);
+  run_passes<L, R, 1, KeepsTile<LoadOp>::value, std::is_same<LoadOp, LoadCplxScalar>::value>(v, x.j, x.c, t, p.tw);
   StoreOp::template run<L, R>(p, x, t, to, v);
 }
 

@@ -132,25 +132,26 @@ __host__ __device__ constexpr int bitrev_c(int k, int n) {
   return r;
 }
 
-template <int H, int P, int K>
+// kScalar: sums and differences part by part in single precision too.
+template <int H, int P, int K, bool kScalar>
 __device__ __forceinline__ void bfly2(cpx* v) {
   cpx a = v[P], b = v[P + H];
-  v[P] = cadd(a, b);
+  v[P] = kScalar ? cmk(a.x + b.x, a.y + b.y) : cadd(a, b);
   if constexpr (4 * K == 2 * H)
     v[P + H] = cmk(a.y - b.y, b.x - a.x);  // times -i
   else
-    v[P + H] = twc<2 * H, K>(csub(a, b));
+    v[P + H] = twc<2 * H, K>(kScalar ? cmk(a.x - b.x, a.y - b.y) : csub(a, b));
 }
 
-template <int H, int... I>
+template <int H, bool kScalar, int... I>
 __device__ __forceinline__ void dif_stage(cpx* v, std::integer_sequence<int, I...>) {
-  (bfly2<H, (I / H) * 2 * H + (I % H), I % H>(v), ...);
+  (bfly2<H, (I / H) * 2 * H + (I % H), I % H, kScalar>(v), ...);
 }
 
-template <int N, int H>
+template <int N, int H, bool kScalar>
 __device__ __forceinline__ void dif_stages(cpx* v) {
-  dif_stage<H>(v, std::make_integer_sequence<int, N / 2>{});
-  if constexpr (H > 1) dif_stages<N, H / 2>(v);
+  dif_stage<H, kScalar>(v, std::make_integer_sequence<int, N / 2>{});
+  if constexpr (H > 1) dif_stages<N, H / 2, kScalar>(v);
 }
 
 template <int N, int... I>
@@ -159,10 +160,10 @@ __device__ __forceinline__ void bitrev_perm(cpx* v, std::integer_sequence<int, I
   ((v[I] = t[I]), ...);
 }
 
-template <int N>
+template <int N, bool kScalar = false>
 __device__ __forceinline__ void fft_reg(cpx* v) {
   if constexpr (N >= 2) {
-    dif_stages<N, N / 2>(v);
+    dif_stages<N, N / 2, kScalar>(v);
     bitrev_perm<N>(v, std::make_integer_sequence<int, N>{});
   }
 }

@@ -8,6 +8,7 @@
 namespace mb {
 
 const void* axis_kernel_cplx(int log2L, int radix16);
+const void* axis_kernel_cplx_columns(int log2L, int radix16);
 const void* axis_kernel_r2c(int log2L, int radix16);
 const void* axis_kernel_c2r(int log2L, int radix16);
 const void* axis_kernel_dct2(int log2L, int radix16);
@@ -56,9 +57,9 @@ int pipe_raw_elems(int combo, int L) {
   }
 }
 
-const void* axis_kernel(int combo, int log2L, int R) {
+const void* axis_kernel(int combo, int log2L, int R, bool columns) {
   switch (combo) {
-    case K_CPLX: return axis_kernel_cplx(log2L, R >= 16);
+    case K_CPLX: return columns ? axis_kernel_cplx_columns(log2L, R >= 16) : axis_kernel_cplx(log2L, R >= 16);
     case K_R2C: return axis_kernel_r2c(log2L, R >= 16);
     case K_C2R: return axis_kernel_c2r(log2L, R >= 16);
     case K_DCT2: return axis_kernel_dct2(log2L, R >= 16);

@@ -28,8 +28,9 @@ constexpr int kMaxLog2L = 13;  // largest in-CTA DFT: 8192 points
 
 // Returns the kernel function for combo, log2(L) and per-thread radix R (8 or
 // 16; lengths below 16 use R = L), or nullptr where the configuration does not
-// exist (more than 512 threads per transform).
-const void* axis_kernel(int combo, int log2L, int R = 16);
+// exist (more than 512 threads per transform).  columns: the pass runs over
+// strided columns (a form of its own for 4096 complex points in single).
+const void* axis_kernel(int combo, int log2L, int R = 16, bool columns = false);
 
 // The persistent, software-pipelined form of the same kernels (pipe_pass.cuh),
 // for log2(L) = 1 .. 13, or nullptr.

@@ -26,4 +26,10 @@ const void* axis_kernel_cplx(int log2L, int radix16) {
   return (log2L >= 0 && log2L <= 13) ? table[log2L][radix16 ? 1 : 0] : nullptr;
 }
 
+const void* axis_kernel_cplx_columns(int log2L, int radix16) {
+  if (sizeof(real) == 4 && log2L == 12 && radix16)
+    return (const void*)axis_pass_kernel<4096, 16, LoadCplxScalar, StoreCplx>;
+  return axis_kernel_cplx(log2L, radix16);
+}
+
 }  // namespace mb

@@ -997,7 +997,7 @@ struct Planner {
     Launch ln;
     ln.key = key;
     ln.radix = R;
-    ln.fn = mb::axis_kernel(combo, lg, R);
+    ln.fn = mb::axis_kernel(combo, lg, R, ap.colmode != 0);
     if (!ln.fn) {
       set_error(MINFFT_B200_EUNSUPPORTED, "no kernel for combo %d, L=%d", combo, L);
       ok = false;
