@@ -181,7 +181,9 @@ int minfft_b200_tc_status(const minfft_aux *a);
  * on `howmany` arrays of plan
  * `a`, using scratch buffers (`reps` timed runs each), and keep the fastest
  * in a process-wide table that every plan consults when it builds its launch
- * lists.  The table can be saved to and loaded from a text file. */
+ * lists.  The table can be saved to and loaded from a text file.  A transform
+ * of small arrays that runs in one launch has nothing to tune: the call then
+ * returns MINFFT_B200_OK and adds no entry. */
 int minfft_b200_autotune(minfft_aux *a, int op, int howmany, int reps);
 int minfft_b200_tune_save(const char *path);
 int minfft_b200_tune_load(const char *path);

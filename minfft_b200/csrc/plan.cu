@@ -1575,6 +1575,14 @@ struct Planner {
     return int(kind == TB_RFT ? std::max<int64_t>(N / 4, 1) : kind == TB_T4POST ? N : std::max<int64_t>(N / 2, 1));
   }
 
+  // Whether the tuning table holds an entry for the launch of an axis that takes
+  // one: it was measured for that launch, so the axes are then planned one by one.
+  static bool tuned(const AxisStep& s) {
+    const int L = int(s.combo == mb::K_CPLX ? s.N : s.N / 2);
+    TuneVal v;
+    return tune_lookup(TuneKey{s.combo, L, s.inner > 1 ? 1 : 0, 0, 0, s.outer * s.inner, s.inner, s.inner, s.inner}, &v);
+  }
+
   // A multi-dimensional transform of small arrays as one launch, a cluster of
   // CTAs per array (nd_pass.cu), where its launches and not its work are the
   // time: 2 to 4 axes of 2 .. 128 complex points each (256 reals), up to a
@@ -1585,8 +1593,8 @@ struct Planner {
   // double one cluster takes too long (DFT 128 x 128 f64 12.8 / 13.2).  Types 2
   // and 3 have the most code per step, and a step of a new length fetches its
   // code anew: unequal axes only up to 512 points (64 x 128 f32 13.0 / 13.8,
-  // 16 x 32 f64 12.9 / 11.6).  A forced kernel form or radix keeps the axis
-  // passes.  steps: the transform's axis steps in order; mid_buf: the buffer
+  // 16 x 32 f64 12.9 / 11.6).  A forced kernel form or radix and tuned axis
+  // launches keep the axis passes.  steps: the transform's axis steps in order; mid_buf: the buffer
   // between them.
   bool plan_nd(const std::vector<AxisStep>& steps, int64_t howmany, int64_t in_elems, int64_t mid_elems,
                int64_t out_elems, int mid_buf) {
@@ -1605,7 +1613,7 @@ struct Planner {
     bool equal = true;
     for (const AxisStep& s : steps) {
       const int64_t L = s.combo == mb::K_CPLX ? s.N : s.N / 2;
-      if (s.N < 2 || ilog2(L) > mb::kNdMaxLog2L) return false;
+      if (s.N < 2 || ilog2(L) > mb::kNdMaxLog2L || tuned(s)) return false;
       work = std::max(work, s.outer / howmany * s.inner * L);
       equal &= s.N == steps.front().N;
     }
@@ -1714,6 +1722,7 @@ struct Planner {
     for (const AxisStep& s : steps) {
       one_pass &= s.combo == mb::K_CPLX;
       total = std::max({total, bytes(s, false), bytes(s, true)});
+      one_pass &= !tuned(s);
       const int64_t L = s.combo == mb::K_CPLX ? s.N : s.N / 2;
       one_pass &= s.N >= 2 && ilog2(L) <= (s.inner > 1 ? kColCapLog2 : kRowCapLog2);
     }
