@@ -894,9 +894,6 @@ struct LoadDCT3 {
     const real b = dst ? rd(n - 1) : rd(N - n);
     return cconj(cmul(cmk(a, b), root(n)));
   }
-  static __device__ __forceinline__ cpx zval(const real* in, int64_t s, int n, int L, bool dst, const cpx* e) {
-    return zval_r([&](int i) { return in[int64_t(i) * s]; }, n, L, dst, e);
-  }
   template <int L, int R>
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile& t, cpx (&v)[R]) {
     const real* in = static_cast<const real*>(p.in) + x.oin;
@@ -1048,8 +1045,7 @@ using LoadT4Chain = LoadT4ChainBy<RootProgression>;
 //    L-n) and share a CTA's slots.
 // Bound by the same memory traffic as a plain pass: what they save is the
 // two passes over memory around the chain (dct2 + dct3 of 2^22 points in
-// f64: ten launches in 145 us before, six in 105 us now, 19 us for a plain
-// pass of 33.6 MB each way and 25 to 28 us for a fused one).
+// f64: ten launches in 148 us before, six in 83 us now).
 
 // Slot of the mirror sub-DFT, and the thread whose elements mirror this
 // thread's: element j + r*TPT pairs with element jm + (R-1-r)*TPT of that
@@ -1426,8 +1422,6 @@ struct StoreDCT2 {
   }
 };
 
-// Inverse real DFT output: the inverse half-length DFT (conjugate of the
-// forward result) read as interleaved reals (reference minfft.c:605,658).
 // Split column DFT of a 2-D real DFT with Nr = 4Q rows, forward half.  The
 // CTA holds the four rows j + Q*m (transform c = m: batch layout d0 = 4 with
 // is0 = Q rows, d1 = Q with is1 = one row, cpb = 4).  After their half-length
@@ -1492,6 +1486,8 @@ struct StoreR2CQ {
   }
 };
 
+// Inverse real DFT output: the inverse half-length DFT (conjugate of the
+// forward result) read as interleaved reals (reference minfft.c:605,658).
 struct StoreC2R {
   template <int L, int R>
   static __device__ __forceinline__ void run(const AxisParams& p, const Ctx& x, const Tile&, const TileOffsets&,

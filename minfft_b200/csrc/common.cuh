@@ -174,8 +174,9 @@ __device__ __forceinline__ void fft_reg(cpx* v) {
 // that predecessor grid has completed and its writes are visible (a no-op
 // for an ordinary launch); pdl_release() allows the next kernel to be
 // scheduled once every CTA of this grid has called it or exited.  Every
-// kernel the planner launches calls both: pdl_wait() before it touches global
-// memory, and pdl_release() only after that.  Released before the wait, a
+// kernel the planner launches calls both: pdl_wait() before it reads or writes
+// anything that a kernel writes (root tables and operands, which belong to the
+// plan and never change, may be read before), and pdl_release() only after that.  Released before the wait, a
 // grid still waiting for its predecessor would let its own successor in too:
 // with a queue of short kernels the SMs then fill with CTAs of several
 // waiting grids, and the one that may run is crowded onto what is left

@@ -14,7 +14,6 @@ constexpr int kNdMaxLog2L = 7;    // in-CTA DFTs of an axis: up to 128 points
 // One axis step, in execution order: nb transforms, transform b = b0 + inner*b1
 // starting at b0 + b1*in_row (out_row), elements inner apart.
 struct NdAxis {
-  int combo;  // K_CPLX, K_R2C, K_C2R, K_DCT2, K_DCT3, K_T4
   int log2L;
   int nb, inner, in_row, out_row;
   int flags;

@@ -1635,7 +1635,6 @@ struct Planner {
       AxisParams ap = base_params();
       set_kind_tables(ap, s.combo, s.N);
       mb::NdAxis& x = d.ax[k];
-      x.combo = s.combo;
       x.log2L = ilog2(L);
       x.nb = int(s.outer / howmany * s.inner);
       x.inner = (int)s.inner;
@@ -1689,7 +1688,7 @@ struct Planner {
     return true;
   }
 
-  // Plans the axis steps of a multi-dimensional transform, steps[i] along axis
+  // Plans the axis steps of a multi-dimensional complex DFT, steps[i] along axis
   // axes[i] of `shape` (extents with the batch count first).  A complex array
   // beyond the L2 is read and written once per axis; the steps along its inner
   // axes, though, stay within a slab of consecutive outer indices, so they all
@@ -1713,18 +1712,12 @@ struct Planner {
   void plan_axes(const std::vector<AxisStep>& steps, const std::vector<size_t>& axes,
                  const std::vector<int64_t>& shape) {
     constexpr size_t kSlab = size_t(64) << 20;
-    auto elem = [](bool c) { return c ? sizeof(cpx) : sizeof(real); };
-    auto bytes = [&](const AxisStep& s, bool out) {  // of the step's whole input / output
-      return size_t(s.outer) * size_t(out ? s.out_row : s.in_row) * elem(out ? complex_out(s.combo) : complex_in(s.combo));
-    };
+    auto bytes = [](const AxisStep& s) { return size_t(s.outer) * size_t(s.in_row) * sizeof(cpx); };  // in and out
     size_t total = 0;
     bool one_pass = true;
     for (const AxisStep& s : steps) {
-      one_pass &= s.combo == mb::K_CPLX;
-      total = std::max({total, bytes(s, false), bytes(s, true)});
-      one_pass &= !tuned(s);
-      const int64_t L = s.combo == mb::K_CPLX ? s.N : s.N / 2;
-      one_pass &= s.N >= 2 && ilog2(L) <= (s.inner > 1 ? kColCapLog2 : kRowCapLog2);
+      total = std::max(total, bytes(s));
+      one_pass &= !tuned(s) && s.N >= 2 && ilog2(s.N) <= (s.inner > 1 ? kColCapLog2 : kRowCapLog2);
     }
     // slabs of the indices of axes 0 .. a: the steps along the axes after a
     // stay inside; the smallest a whose slabs can be small enough
@@ -1766,8 +1759,7 @@ struct Planner {
         const int64_t n = std::min(chunk, outer - c);
         for (size_t k = i; k < e; ++k) {
           AxisStep s = steps[k];
-          s.in_off = bytes(s, false) / size_t(outer) * size_t(c);
-          s.out_off = bytes(s, true) / size_t(outer) * size_t(c);
+          s.in_off = s.out_off = bytes(s) / size_t(outer) * size_t(c);
           s.outer = s.outer / outer * n;
           plan_axis(s);
         }
@@ -1869,7 +1861,7 @@ struct Planner {
     // (LoadT4Chain, StoreT4Chain), the permutation, rotations and
     // de-interleave of types 2 and 3 and the real DFT's unpacking and packing
     // (the *Line ops).  Two passes over memory less: dct2 + dct3 of 2^22
-    // points in f64 144.9 -> 105.4 us.  In a tensor-core mode only an end
+    // points in f64 148 -> 83 us.  In a tensor-core mode only an end
     // pass on the CUDA cores fuses its step (128 to 1024 points for type 4, 16
     // to 1024 for the others): the 256-point tensor-core passes take plain
     // complex input and output.  The other step stays a separate
@@ -2222,8 +2214,6 @@ bool build_program(minfft_aux* a, int op, int howmany, bool alias, Program* prog
         break;
       }
       int cur = BUF_X;
-      std::vector<AxisStep> steps;
-      std::vector<size_t> axes;
       for (size_t ax = nd - 1; ax >= 1; --ax) {
         AxisStep s{};
         s.combo = combo;
@@ -2235,11 +2225,9 @@ bool build_program(minfft_aux* a, int op, int howmany, bool alias, Program* prog
         s.flags = fl;
         s.in_buf = cur;
         s.out_buf = BUF_Y;
-        steps.push_back(s);
-        axes.push_back(ax);
+        pl.plan_axis(s);
         if (!(s.N == 1 && combo == mb::K_DCT3 && cur == BUF_Y)) cur = BUF_Y;
       }
-      pl.plan_axes(steps, axes, D);
       if (cur != BUF_Y) pl.add_unit(mb::UNIT_SCALE_REAL, prod(D, 0, nd), 1, cur, BUF_Y);
       break;
     }
@@ -2313,7 +2301,7 @@ struct DeviceGuard {
 };
 
 // Programmatic dependent launch for the planner's kernels (every one of them
-// starts with pdl_release / pdl_wait): consecutive launches of a program
+// calls pdl_wait and later pdl_release): consecutive launches of a program
 // overlap the next kernel's scheduling with the previous one's drain.
 // MINFFT_B200_PDL=0 turns it off.
 bool pdl_enabled() {
