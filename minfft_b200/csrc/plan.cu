@@ -513,7 +513,11 @@ struct Planner {
   // kinds with a load or store stage of their own up to about 2048 points
   // per SM, where one wave of CTAs covers the batch and its latency is the
   // time (2048 DCT-2 + DCT-3 of 256 points in f64: 9.4 us a pair against
-  // 10.8; from 2^20 points on radix 16 is ahead, 20.7 against 23.3).
+  // 10.8; from 2^20 points on radix 16 is ahead, 20.7 against 23.3) and lines
+  // have at most 512 complex points: beyond, radix 8 takes four passes to radix
+  // 16's three (one real DFT of 8192 points in single 10.8 us a pair, 7.6 at
+  // radix 16; one DCT-2 + DCT-3 of 4096 in double 11.4 and 9.3; 290 DCT-4 of 2048
+  // 12.4 and 10.3).
   //
   // Row tiles are CTAs of about 64 threads, on which barriers and the wait
   // for the slowest load are short: 2048 DFTs of 1024 points in f64 take
@@ -538,7 +542,7 @@ struct Planner {
       while (ap.cpb > 1 && !plain_fits(combo, L, ap.cpb, ap.flags, col ? 1 : 0, *R)) ap.cpb /= 2;
       return;
     }
-    const bool r8 = L == 32 || L == 64 || (few && combo != mb::K_CPLX && L > 16);
+    const bool r8 = L == 32 || L == 64 || (few && combo != mb::K_CPLX && L > 16 && L <= 512);
     if (r8 && mb::axis_kernel(combo, ilog2(L), 8)) *R = 8;
     const int tpt = L / std::min(*R, L);
     const int elem = (combo == mb::K_CPLX) ? int(sizeof(cpx)) : int(sizeof(real));
