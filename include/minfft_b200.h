@@ -122,10 +122,10 @@ int minfft_b200_dft_noalloc(const void *x, void *y, int n, int inverse, void *st
  * transforms, 1 .. 131072 for the real ones) and device input and output
  * arrays (complex data aligned to its size).  Jobs are grouped by kind and
  * length into work items (several transforms of up to 4096 complex points;
- * one tile of 4096 points of a pass of a longer one) that persistent CTAs take
- * from an atomic counter.  The plan owns the root tables, the counters and the
- * scratch; execute only launches the captured graph on
- * `stream`.  Outputs of different jobs must not overlap their inputs.  A
+ * one tile of 4096 points of a pass of one longer than 8192) that persistent
+ * CTAs take from an atomic counter; transforms of 8192 points run beside them,
+ * a CTA each.  The plan owns the root tables, the counters and the scratch;
+ * execute only launches its graph on `stream`.  Outputs of different jobs must not overlap their inputs.  A
  * device-side wait that ran out (see minfft_b200_device_status) makes the
  * next execute of the batch return MINFFT_B200_ETIMEOUT. */
 typedef struct {
